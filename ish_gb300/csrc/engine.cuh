@@ -18,25 +18,23 @@ namespace ish {
 
 enum Mode : int { SG = 0, SW = 1 };
 
-// Sentinel used for "minus infinity" lanes; far below every value the safe
-// regime admits (|value| < 30000) and far from wrapping when a penalty is
-// added to it.
-constexpr int NEG_BIG = -20000;
-
 // Layouts of the wavefront profile in shared memory (for code c, thread t
 // and the thread's column j):
 //   PROF_S16:  16-bit scores, [c][t][j]; a record pair's word is assembled
 //              with one PRMT per column (large alphabets x long queries);
-//   PROF_PAIR: packed 32-bit words for every (code A, code B) pair,
-//              [cA][cB][t][j] (small alphabets);
-//   PROF_S32:  32-bit words with the score in the low half, [c][t][j]; the
-//              pair's word is one IMAD (the default).
+//   PROF_PAIR: 32-bit words for every (code A, code B) pair, [cA][cB][t][j]
+//              (small alphabets): packed halves for local alignment, the
+//              integer b * 65536 + a of the signed scores for semi-global;
+//   PROF_S32:  32-bit words, [c][t][j], the score in the low half (local) or
+//              as a signed integer (semi-global); the pair's word is one IMAD
+//              (the default).
 enum ProfLayout : int { PROF_S16 = 0, PROF_PAIR = 1, PROF_S32 = 2 };
 
 // Control word of the wavefront pipeline (one per row step).
 constexpr uint32_t CTL_NEW = 1u << 16;   // row 0 of a new record pair
 constexpr uint32_t CTL_IDLE = 1u << 17;  // no work in this slot
-constexpr int CTL_SEQ_SHIFT = 18;        // 5-bit pair sequence number
+constexpr uint32_t CTL_DONE = 1u << 18;  // thread 0: the work counter has run dry
+constexpr int CTL_SEQ_SHIFT = 19;        // 5-bit pair sequence number
 
 struct Decision {
   int32_t max_score;
@@ -71,18 +69,19 @@ struct WaveParams {
   uint32_t lane_mul;       // 65536: b * lane_mul + a packs two PROF_S32 words
   int open, ext, ends;
   int neg_limit;           // v_neg_limit of the reference (semi_global_aln/striped.mojo:329-334)
-  int hleft, fin;          // left boundary value and F entering the padding
+  int bias;                // semi-global: added to every H, E and F (see wave_params)
   int frame_mask;          // semi-global: R - 1, rows between frame resets (R * ext <= 2048)
   // packed 16-bit pairs of values used every row, precomputed on the host so
   // that the kernel reads them as operands instead of deriving them
   uint32_t pk_nopen;       // (-open, -open)
   uint32_t pk_next;        // (-ext, -ext)
-  uint32_t pk_eopen;       // (ext - open, ext - open): the framed E update
-  uint32_t pk_fsin;        // (fin + open, fin + open): F + open entering the padding
-  uint32_t pk_ext;         // (ext, ext) for semi-global, 0 for local: one row's frame step
-  uint32_t pk_drop;        // (-R * ext, -R * ext): a frame reset
+  uint32_t pk_eopen;       // (ext - open, ext - open): a gap opening in the frames
+  uint32_t pk_fsin;        // (open, open): local alignment, F + open entering the padding
+  uint32_t pk_left;        // semi-global: H entering the padding from the left at frame 0
+  uint32_t pk_left_ext;    // ... and its rise per row (0 with a fixed target start)
+  uint32_t pk_drop;        // -(R * ext) in both halves as one 32-bit integer: a frame reset
   uint32_t row_bytes;      // profile bytes between consecutive codes' rows ((G * kp) words)
-  const int16_t *hinit;    // H(-1, q) for q in [-d, Q), index q + d
+  const int16_t *hinit;    // H(-1, q) for q in [-d, Q), index c = q + d (semi-global: + c * ext, its frame)
   uint32_t first, count;   // sorted entries [first, first + count) are scored
   uint32_t pair_stride, pair_phase;  // of those, record pairs phase, phase + stride, ... (stride 0: every pair)
   uint32_t *counter;       // work counter (record pairs), zeroed before launch
@@ -136,6 +135,8 @@ inline uint32_t dup16_host(int v) {
 }
 __device__ __forceinline__ int lo16(uint32_t w) { return (int)(int16_t)(w & 0xffff); }
 __device__ __forceinline__ int hi16(uint32_t w) { return (int)(int16_t)(w >> 16); }
+__device__ __forceinline__ int ulo16(uint32_t w) { return (int)(w & 0xffffu); }
+__device__ __forceinline__ int uhi16(uint32_t w) { return (int)(w >> 16); }
 
 // Hit decision of the CPU matchers.  Float32 arithmetic with round-to-nearest,
 // exactly as Mojo's Float32 ops.

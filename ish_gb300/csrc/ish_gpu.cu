@@ -303,9 +303,9 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
   const int A = q.rows;
   const bool sg = q.algo == ISH_ALGO_SEMI_GLOBAL;
   const int ppad = (sg && !(q.ends & ISH_FREE_TARGET_START)) ? -(q.open + q.ext) : 0;
-  // semi-global scores carry +ext: with row frames rising by ext per row,
-  // H(i-1) in frame(i-1) plus P + ext lands in frame(i)
-  const int pext = sg ? q.ext : 0;
+  // semi-global scores carry +2 ext: with frames rising by ext per row and per
+  // column, H(i-1, j-1) plus P + 2 ext lands in the frame of (i, j)
+  const int pext = sg ? 2 * q.ext : 0;
   auto P = [&](int r, int col) -> int {
     if (col < 0) return ppad + pext;
     return q.M[(size_t)q.rep[r] * q.alphabet + q.q[col]] + pext;
@@ -319,7 +319,8 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
           for (int j = 0; j < K; ++j) {
             const int col = t * K + j - L.d;
             w[((size_t)(a * A + b) * G + t) * L.kp + j] =
-                ((uint32_t)P(a, col) & 0xffffu) | ((uint32_t)(P(b, col) & 0xffff) << 16);
+                sg ? ((uint32_t)P(b, col) << 16) + (uint32_t)P(a, col)
+                   : ((uint32_t)P(a, col) & 0xffffu) | ((uint32_t)P(b, col) << 16);
           }
     host.resize(w.size() * 4);
     memcpy(host.data(), w.data(), host.size());
@@ -327,7 +328,10 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
     std::vector<uint32_t> w((size_t)A * G * L.kp, 0u);
     for (int a = 0; a < A; ++a)
       for (int t = 0; t < G; ++t)
-        for (int j = 0; j < K; ++j) w[((size_t)a * G + t) * L.kp + j] = (uint32_t)P(a, t * K + j - L.d) & 0xffffu;
+        for (int j = 0; j < K; ++j) {
+          const uint32_t v = (uint32_t)P(a, t * K + j - L.d);
+          w[((size_t)a * G + t) * L.kp + j] = sg ? v : v & 0xffffu;
+        }
     host.resize(w.size() * 4);
     memcpy(host.data(), w.data(), host.size());
   } else {
@@ -350,6 +354,7 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
     const int col = c - L.d;
     int v = 0;
     if (sg && col >= 0 && !(q.ends & ISH_FREE_QUERY_START)) v = -q.open - q.ext * col;
+    if (sg) v += q.ext * c;  // column frame (c + 1) * ext, row frame -ext
     hin[c] = (int16_t)v;
   }
   CU(L.prof.ensure(L.prof_bytes));
@@ -716,15 +721,27 @@ void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDe
   p.ends = q.ends;
   p.neg_limit = q.neg_limit;
   const bool sg = mode == SG;
-  p.hleft = (sg && !(q.ends & ISH_FREE_TARGET_START)) ? NEG_BIG : 0;
-  p.fin = sg ? NEG_BIG : 0;
+  // Semi-global values are unsigned 16-bit: value + bias + row frame + column
+  // frame.  With a free target start H(i, j) >= -open - ext * j (a query gap
+  // from the left boundary), so with its column frame no H is below
+  // bias - open and no E or gap opening below bias - 2 open; a fixed one lowers
+  // the left boundary by open + ext per row.  `low` is that depth; the slack
+  // above it covers a score (an int8) added to the smallest value, the rows a
+  // pair is rounded up by and the floor that stands for minus infinity on the
+  // left (ext after its profile step).  At the top: H <= 30000, row frames
+  // < 2048 and column frames ext * G * K, where the regime keeps
+  // low + ext * (G * K + 3) <= 30000; the sum stays below 65,536.
+  const bool ts = q.ends & ISH_FREE_TARGET_START;
+  const int low = ts ? 2 * q.open : 3 * q.open + q.ext * (int)std::min<uint64_t>(rs.max_len, 32768);
+  p.bias = sg ? low + 8 * q.ext + 256 : 0;
   p.frame_mask = sg ? frame_rows(q.ext) - 1 : 0x3fffffff;
   p.pk_nopen = dup16_host(-q.open);
   p.pk_next = dup16_host(-q.ext);
   p.pk_eopen = dup16_host(q.ext - q.open);
-  p.pk_fsin = dup16_host(p.fin + q.open);
-  p.pk_ext = sg ? (uint32_t)q.ext * 0x10001u : 0u;
-  p.pk_drop = sg ? dup16_host(-(p.frame_mask + 1) * q.ext) : 0u;
+  p.pk_fsin = sg ? 0u : dup16_host(q.open);
+  p.pk_left = sg ? (ts ? (uint32_t)p.bias : (uint32_t)q.open) * 0x10001u : 0u;
+  p.pk_left_ext = sg && ts ? (uint32_t)q.ext * 0x10001u : 0u;
+  p.pk_drop = sg ? (uint32_t)(-(p.frame_mask + 1) * q.ext) * 0x10001u : 0u;
   p.row_bytes = (uint32_t)(L.G * L.kp * (L.layout == PROF_S16 ? 2 : 4));
   p.hinit = L.hinit.as<const int16_t>();
   p.error = error;

@@ -13,26 +13,34 @@
 // lanes" for short queries; G = 32 is a warp-wide anti-diagonal wavefront for
 // long queries.
 //
-// Per cell and record pair (two cells) the recurrence costs five DPX
-// instructions (four for semi-global, below), in two in-place passes over the
-// thread's columns:
+// Local alignment: five DPX instructions per cell and record pair (two cells),
+// in two in-place passes over the thread's columns:
 //   backward:  T = max(Hdiag + P, E);  u = T - open;  E = max(E - ext, u);  H := T
 //   forward:   H = max(Fs - open, T);  Fs = max(Fs - ext, T)
-// with Fs = F + open carried along the row (local alignment floors u at 0,
-// which keeps E, T and H non-negative).  E opens from T only, never from F: an
-// F-then-E gap pair always has an E-then-F twin of at least the same score,
-// which this recurrence keeps, so H is exactly the Gotoh H.  The serial
-// dependency along a row is the single Fs instruction per cell, and both passes
-// update H and E in place (no register rotation between rows).
+// with Fs = F + open carried along the row, and u floored at 0, which keeps E,
+// T and H non-negative.  E opens from T only, never from F: an F-then-E gap
+// pair always has an E-then-F twin of at least the same score, which this
+// recurrence keeps, so H is exactly the Gotoh H.
 //
-// Semi-global alignment needs only four: row r is held raised by a frame
-// f(r) = (r mod R) * ext, and the profile carries +ext, so H(r-1) + P lands in
-// f(r) and the E update E' = max(E - ext, T - open) becomes
-// E'(framed) = max(T(framed) + ext - open, E(framed)), one add-max.  Every R
-// rows (R * ext <= 2048, headroom the fast regime keeps above the largest
-// score) the carried row drops back to frame 0; scores leave the kernel with
-// their frame taken off.  Local alignment keeps five: its floor at 0 would
-// move with the frame.
+// Semi-global: three DPX instructions and a 32-bit add (two with the 32-bit
+// profile, whose pair word is assembled by the first):
+//   backward:  H[j] := H[j-1] + P[j]                (integer multiply-add pipe)
+//   forward:   H = max3(H, E, F);  E = max(H + c, E);  F = max(H + c, F)
+// The values are unsigned 16-bit, held raised by a bias and by frames that rise
+// by ext per row and per column: a gap extension then costs nothing, so both
+// gap updates are one add-max with the same c = ext - open, and the profile
+// carries +2 ext for the diagonal step.  Rows drop back to frame 0 every R rows
+// (R * ext <= 2048); the column frame runs over the whole padded query.  The
+// bias keeps every value of the low half non-negative, so that the sum
+// H + P, with P the pair's scores as ONE signed integer b * 65536 + a, never
+// borrows from the high half: the add can leave the DPX pipe (16 lanes per
+// clock and sub-partition), which bounds the row.  wave_params() in ish_gpu.cu
+// derives the bias and shows that every value fits 16 bits.
+// Measured on GB300 (row loops alone, 38 columns per thread): 9.3 clocks per
+// column and warp with the 32-bit profile, where the shared-memory loads bound
+// it (8.4), 8.0 with the pair profile, against 11.8 for four DPX per cell pair.
+// The 16-bit profile is joined by a PRMT per column, whose halves cannot be
+// added as one integer; it keeps T = max(Hdiag + P, E), H = max(T, F).
 //
 // End coordinates follow the reference exactly:
 //   semi-global, target end free: first row where H(i, Q-1) strictly beats the
@@ -72,12 +80,8 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   const unsigned FULL = 0xffffffffu;
   const uint32_t NOPEN = p.pk_nopen;
   const uint32_t NEXT = p.pk_next;
-  const uint32_t VFLOOR = (MODE == SW) ? 0u : 0x80008000u;
-  const uint32_t FS_IN = p.pk_fsin;  // F + open entering the padding
-  // semi-global row frames: row r is held raised by frame = (r mod R) * ext
-  const uint32_t EOPEN = p.pk_eopen;  // E' = max(T + ext - open, E)
-  const uint32_t NEGMIN = 0x80008000u;
-  const int f0 = (MODE == SG) ? p.ext : 0;  // row -1 sits in frame -ext
+  // semi-global: a gap opens from H at ext - open in the frames
+  const uint32_t EOPEN = p.pk_eopen;
   const bool te = (MODE == SG) && (p.ends & 8);
   const bool qe = (MODE == SG) && (p.ends & 2);
   // record pairs of the range: every pair_stride-th from pair_phase
@@ -87,13 +91,14 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   const int col0 = t * K - p.d;  // query column of register 0
   // parameters read every step, held in registers (the batched kernel's
   // parameters live in shared memory)
-  const int kp = p.kp, alpha = p.alphabet, fmask = p.frame_mask, ext = p.ext, hleft = p.hleft;
+  const int kp = p.kp, alpha = p.alphabet, fmask = p.frame_mask, ext = p.ext;
   const uint32_t remap_off = p.remap_off, lane_mul = p.lane_mul;
   // the frame of a row (always 0 for local alignment)
   auto frame_of = [&](int r) { return (MODE == SG) ? (r & fmask) * ext : 0; };
-  // +ext in both 16-bit halves: added to a boundary value hleft + frame
-  // (hleft 0 or NEG_BIG, frames <= 2048), the low half never carries
-  const uint32_t EXT2 = (MODE == SG) ? p.pk_ext : 0u;
+  // semi-global: H entering the padding from the left at row r is
+  // left0 + frame(r) / ext * left_ext (left_ext 0: a floor below every value)
+  const uint32_t LEFT0 = (MODE == SG) ? p.pk_left : 0u;
+  const uint32_t LEFT_EXT = (MODE == SG) ? p.pk_left_ext : 0u;
   // this thread's part of every profile row, and the bytes between the rows
   // of consecutive codes: a row's address is one multiply-add
   const unsigned char *prof_t = prof + (uint32_t)(t * kp) * (LAYOUT == PROF_S16 ? 2u : 4u);
@@ -113,48 +118,47 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
 #pragma unroll
   for (int k = 0; k < RPS; ++k) outH[k] = outF[k] = outB[k] = 0;
   uint32_t outC = CTL_IDLE;
-  int q4 = 0, lenA = 0, lenB = 0, lastA_row = -1, lastB_row = -1;  // q4: row of the step's first row
-  uint32_t pr = 0;
+  int q4 = 0, lenA = 0, lenB = 0;  // q4: row of the step's first row
   // this thread's record streams: 4 codes per 32-bit word, one word ahead
   const uint8_t *pa = nullptr, *pb = nullptr;
   uint32_t wA = 0, wB = 0, nA = 0, nB = 0;
   // tracking
-  uint32_t best = 0;         // SG: lane-wise running max of H(i, Q-1); SW: of this thread's cells
+  // SG: lane-wise running max of H(i, Q-1), at thread G-1 (the other threads
+  // hold the largest value, so that none of their rows count); SW: of this
+  // thread's cells
+  uint32_t best = 0;
   int rowA = -1, rowB = -1;  // first row of the lane's maximum
   uint32_t oR0 = 0, oR1 = 0, oR2 = 0, oR3 = 0;  // last-row partials for thread t+1
-  uint32_t iR0 = 0, iR1 = 0, iR2 = 0, iR3 = 0;  // ... and those of thread t-1
+  uint32_t iR0 = 0, iR1 = 0, iR2 = 0, iR3 = 0;  // ... and those of thread t-1, in the step after
   bool has_out = false;
-  // thread 0 of the group grabs record pairs: f_left steps of the current pair
-  // are still to start, f_ctl is the control word of the next step
-  bool f_done = false;
-  int f_left = 0;
-  uint32_t f_ctl = CTL_IDLE;
-  uint32_t f_seq = 31;
-  // the next row at which one of this thread's records ends (-3: none)
-  int ev_row = -3;
   const bool remap = remap_off != 0;
-  uint64_t steps = 0;
   constexpr int CHK = 8 / RPS;  // steps between termination checks
-  int chk = CHK;
+  uint32_t step = 0;
 
   // One row of the pair with record codes cA, cB: `diag` is H of the row above
-  // at column col0 - 1, `fs` is F + open entering column col0.  Updates H and
-  // E in place and returns F + open leaving the thread's last column.
+  // at column col0 - 1, `fs` is F (local alignment: F + open) entering column
+  // col0.  Updates H and E in place and returns F leaving the last column.
   auto row_step = [&](uint32_t cA, uint32_t cB, uint32_t diag, uint32_t fs) -> uint32_t {
     if (remap) {  // codes that score alike share a profile row
       cA = prof[remap_off + cA];
       cB = prof[remap_off + cB];
     }
     uint32_t P[K];
+    // semi-global: the profile word of column j plus H of the row above at
+    // column j - 1 (H still holds that row); local alignment adds it later
+    auto with_diag = [&](uint32_t w, int j) -> uint32_t {
+      if (MODE != SG) return w;
+      return w + (j == 0 ? diag : H[j > 0 ? j - 1 : 0]);
+    };
     if (LAYOUT == PROF_PAIR) {
       const uint4 *r4 = reinterpret_cast<const uint4 *>(prof_t + (cA * alpha + cB) * row_bytes);
 #pragma unroll
       for (int v = 0; v < (K + 3) / 4; ++v) {
         const uint4 w = r4[v];
-        if (4 * v + 0 < K) P[4 * v + 0] = w.x;
-        if (4 * v + 1 < K) P[4 * v + 1] = w.y;
-        if (4 * v + 2 < K) P[4 * v + 2] = w.z;
-        if (4 * v + 3 < K) P[4 * v + 3] = w.w;
+        if (4 * v + 0 < K) P[4 * v + 0] = with_diag(w.x, 4 * v + 0);
+        if (4 * v + 1 < K) P[4 * v + 1] = with_diag(w.y, 4 * v + 1);
+        if (4 * v + 2 < K) P[4 * v + 2] = with_diag(w.z, 4 * v + 2);
+        if (4 * v + 3 < K) P[4 * v + 3] = with_diag(w.w, 4 * v + 3);
       }
     } else if (LAYOUT == PROF_S32) {
       // 32-bit words holding the 16-bit score in the low half; the packed
@@ -167,10 +171,10 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
 #pragma unroll
       for (int v = 0; v < (K + 3) / 4; ++v) {
         const uint4 a = ra[v], b = rb[v];
-        if (4 * v + 0 < K) P[4 * v + 0] = b.x * mul + a.x;
-        if (4 * v + 1 < K) P[4 * v + 1] = b.y * mul + a.y;
-        if (4 * v + 2 < K) P[4 * v + 2] = b.z * mul + a.z;
-        if (4 * v + 3 < K) P[4 * v + 3] = b.w * mul + a.w;
+        if (4 * v + 0 < K) P[4 * v + 0] = b.x * mul + with_diag(a.x, 4 * v + 0);
+        if (4 * v + 1 < K) P[4 * v + 1] = b.y * mul + with_diag(a.y, 4 * v + 1);
+        if (4 * v + 2 < K) P[4 * v + 2] = b.z * mul + with_diag(a.z, 4 * v + 2);
+        if (4 * v + 3 < K) P[4 * v + 3] = b.w * mul + with_diag(a.w, 4 * v + 3);
       }
     } else {
       // 16-bit words (profiles too large for the 32-bit layout): one PRMT
@@ -188,23 +192,40 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         }
       }
     }
-    // backward pass (columns independent), then the F chain
+    if (MODE == SG && LAYOUT != PROF_S16) {
+      // the profile words hold H + P already (above)
 #pragma unroll
-    for (int j = K - 1; j >= 0; --j) {
-      const uint32_t T = __viaddmax_s16x2(j == 0 ? diag : H[j - 1], P[j], E[j]);
-      if (MODE == SG) {
-        E[j] = __viaddmax_s16x2(T, EOPEN, E[j]);  // in the row frames (see the header)
-      } else {
-        const uint32_t u = __viaddmax_s16x2(T, NOPEN, VFLOOR);
-        E[j] = __viaddmax_s16x2(E[j], NEXT, u);
+      for (int j = 0; j < K; ++j) {
+        const uint32_t h = __vimax3_u16x2(P[j], E[j], fs);
+        E[j] = __viaddmax_u16x2(h, EOPEN, E[j]);
+        fs = __viaddmax_u16x2(h, EOPEN, fs);
+        H[j] = h;
       }
-      H[j] = T;
-    }
+    } else if (MODE == SG) {
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      const uint32_t T = H[j];
-      H[j] = __viaddmax_s16x2(fs, NOPEN, T);
-      fs = __viaddmax_s16x2(fs, NEXT, T);
+      for (int j = K - 1; j >= 0; --j) H[j] = __viaddmax_u16x2(j == 0 ? diag : H[j - 1], P[j], E[j]);
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const uint32_t T = H[j];
+        H[j] = __vmaxu2(T, fs);
+        E[j] = __viaddmax_u16x2(T, EOPEN, E[j]);
+        fs = __viaddmax_u16x2(T, EOPEN, fs);
+      }
+    } else {
+      // backward pass (columns independent), then the F chain
+#pragma unroll
+      for (int j = K - 1; j >= 0; --j) {
+        const uint32_t T = __viaddmax_s16x2(j == 0 ? diag : H[j - 1], P[j], E[j]);
+        const uint32_t u = __viaddmax_s16x2(T, NOPEN, 0u);
+        E[j] = __viaddmax_s16x2(E[j], NEXT, u);
+        H[j] = T;
+      }
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        const uint32_t T = H[j];
+        H[j] = __viaddmax_s16x2(fs, NOPEN, T);
+        fs = __viaddmax_s16x2(fs, NEXT, T);
+      }
     }
     return fs;
   };
@@ -258,7 +279,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // (register K-1 of thread G-1); a strict improvement records the row, so
   // the FIRST row of the maximum wins.
   auto te_row = [&](int row) {
-    const uint32_t nb = __viaddmax_s16x2(best, 0u, __viaddmax_s16x2(H[K - 1], dup16(-frame_of(row)), NEGMIN));
+    const uint32_t nb = __viaddmax_u16x2(H[K - 1], dup16(-frame_of(row)), best);
     if (nb != best) {
       if (lo16(nb) != lo16(best)) rowA = row;
       if (hi16(nb) != hi16(best)) rowB = row;
@@ -275,24 +296,22 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // partial results left to right -- thread t-1's arrived as iR at the start
   // of this step, this thread's leave as oR at the next -- and thread G-1
   // writes the record's outputs.
-  auto on_event = [&](int row) {
-    const bool lastA = row == lastA_row, lastB = row == lastB_row;
-    {  // the other record's end, if it is still ahead
-      int nxt = lastA_row > row ? lastA_row : -3;
-      if (lastB_row > row && (nxt < 0 || lastB_row < nxt)) nxt = lastB_row;
-      ev_row = nxt;
-    }
+  auto on_event = [&](int row, uint32_t ctl) {
+    const bool lastA = row == lenA - 1, lastB = row == lenB - 1;
+    // the pair: its slot is rewritten only 32 pairs later
+    const uint32_t pr = slots[(ctl >> CTL_SEQ_SHIFT) & 31];
     if (MODE == SG) {
       uint32_t mx = 0, mq = 0;
       if (qe) {
-        int bA = -32768, bB = -32768, qA = 0x7fff, qB = 0x7fff;
+        int bA = 0, bB = 0, qA = 0x7fff, qB = 0x7fff;  // H + bias + row frame, above 0
         uint32_t row_h[K];  // staged as in the local-alignment scan
 #pragma unroll
         for (int j = 0; j < K; ++j) row_h[j] = H[j];
 #pragma unroll 1
         for (int j = 0; j < K; ++j) {
           if (col0 + j >= 0) {
-            const int a = lo16(row_h[j]), b = hi16(row_h[j]);
+            const int cf = (t * K + j + 1) * ext;
+            const int a = ulo16(row_h[j]) - cf, b = uhi16(row_h[j]) - cf;
             if (a > bA) {
               bA = a;
               qA = col0 + j;
@@ -304,12 +323,12 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
           }
         }
         if (t > 0) {  // columns to the left win ties
-          if (!(bA > lo16(iR0))) {
-            bA = lo16(iR0);
+          if (!(bA > ulo16(iR0))) {
+            bA = ulo16(iR0);
             qA = (int)(iR1 & 0xffffu);
           }
-          if (!(bB > hi16(iR0))) {
-            bB = hi16(iR0);
+          if (!(bB > uhi16(iR0))) {
+            bB = uhi16(iR0);
             qB = (int)(iR1 >> 16);
           }
         }
@@ -322,6 +341,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         }
       }
       if (t == G - 1) {
+        const int last_off = p.bias + G * K * ext;  // bias and column frame of the last column
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           if (!(x == 0 ? lastA : lastB)) continue;
@@ -329,13 +349,13 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
           const int T = x == 0 ? lenA : lenB;
           int score, er, eq = p.Q - 1;
           if (!te && !qe) {
-            score = (x == 0 ? lo16(H[K - 1]) : hi16(H[K - 1])) - frame_of(row);  // this row's H(i, Q-1)
+            score = (x == 0 ? ulo16(H[K - 1]) : uhi16(H[K - 1])) - frame_of(row) - last_off;  // this row's H(i, Q-1)
             er = T - 1;
           } else {
-            score = te ? (x == 0 ? lo16(best) : hi16(best)) : p.neg_limit;
+            score = te ? (x == 0 ? ulo16(best) : uhi16(best)) - last_off : p.neg_limit;
             er = x == 0 ? rowA : rowB;
             if (qe) {
-              const int s1 = (x == 0 ? lo16(mx) : hi16(mx)) - frame_of(row);
+              const int s1 = (x == 0 ? ulo16(mx) : uhi16(mx)) - frame_of(row) - p.bias;
               const int t1 = x == 0 ? (int)(mq & 0xffffu) : (int)(mq >> 16);
               if (s1 > score) {
                 score = s1;
@@ -408,7 +428,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       msgF[k] = __shfl_up_sync(FULL, outF[k], 1, G);
       msgB[k] = (MODE == SW) ? __shfl_up_sync(FULL, outB[k], 1, G) : 0u;
     }
-    uint32_t msgC = __shfl_up_sync(FULL, outC, 1, G);
+    uint32_t msgC = __shfl_up_sync(FULL, outC, 1, G);  // thread 0: its own last control word
     // partial results of records that ended in thread t-1's previous step
     if (__any_sync(FULL, has_out)) {
       iR0 = __shfl_up_sync(FULL, oR0, 1, G);
@@ -421,30 +441,27 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
     }
 
     if (t0) {
-      if (f_left <= 0 && !f_done) {
-        const uint32_t nt = atomicAdd(counter, 1u);
-        if (nt < npairs) {
-          const uint32_t np = nt * pstride + pphase;  // the pair's index in the range
-          f_seq = (f_seq + 1) & 31;
-          slots[f_seq] = np;
-          const uint32_t sA = p.first + 2 * np;
-          const int na = (int)p.rec.len[sA];
-          const int nb = (2 * np + 1 < p.count) ? (int)p.rec.len[sA + 1] : 0;
-          f_left = (max(max(na, nb), 1) + RPS - 1) / RPS;
-          f_ctl = CTL_NEW | (f_seq << CTL_SEQ_SHIFT);
-        } else {
-          f_done = true;
+      // thread 0 of the group goes on with its pair or takes the next one
+      msgC &= ~CTL_NEW;
+      if ((msgC & CTL_IDLE) || q4 + RPS >= max(lenA, lenB)) {
+        msgC |= CTL_IDLE;
+        if (!(msgC & CTL_DONE)) {
+          const uint32_t nt = atomicAdd(counter, 1u);
+          const uint32_t seq = ((msgC >> CTL_SEQ_SHIFT) + 1) & 31;
+          if (nt < npairs) {
+            slots[seq] = nt * pstride + pphase;  // the pair's index in the range
+            msgC = CTL_NEW | (seq << CTL_SEQ_SHIFT);
+          } else {
+            msgC = CTL_IDLE | CTL_DONE;
+          }
         }
       }
-      msgC = f_ctl;
-      f_ctl &= ~CTL_NEW;
-      if (--f_left <= 0) f_ctl = CTL_IDLE;
     }
 
     const bool busy = !(msgC & CTL_IDLE);
     if (busy) {
       if (msgC & CTL_NEW) {
-        pr = slots[(msgC >> CTL_SEQ_SHIFT) & 31];
+        const uint32_t pr = slots[(msgC >> CTL_SEQ_SHIFT) & 31];
         const uint32_t sA = p.first + 2 * pr;
         lenA = (int)p.rec.len[sA];
         pa = p.rec.codes + p.rec.off[sA];
@@ -455,22 +472,17 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
           lenB = 0;
           pb = pa;
         }
-        lastA_row = lenA - 1;
-        lastB_row = lenB > 0 ? lenB - 1 : -2;
-        // the earlier of the two records' last rows (either may be empty)
-        ev_row = lastA_row >= 0 ? lastA_row : -3;
-        if (lastB_row >= 0 && (ev_row < 0 || lastB_row < ev_row)) ev_row = lastB_row;
         nA = __ldg(reinterpret_cast<const uint32_t *>(pa));
         nB = lenB ? __ldg(reinterpret_cast<const uint32_t *>(pb)) : 0u;
         const int16_t *hi = p.hinit + t * K;
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-          const int h0 = hi[j];
-          H[j] = dup16(h0 - f0);
-          E[j] = (MODE == SW) ? 0u : dup16(h0 - p.open);
+          const int h0 = hi[j] + p.bias;
+          H[j] = (MODE == SW) ? 0u : dup16(h0);
+          E[j] = (MODE == SW) ? 0u : dup16(h0 + ext - p.open);  // row 0's frame is one ext above row -1's
         }
-        prevH = t0 ? dup16(p.hleft - f0) : dup16(p.hinit[t * K - 1] - f0);
-        best = (MODE == SW) ? 0u : dup16(p.neg_limit);
+        prevH = (MODE == SW || t0) ? 0u : dup16(p.hinit[t * K - 1] + p.bias);  // t0: set below
+        best = (MODE == SG && t != G - 1) ? 0xffffffffu : 0u;
         rowA = rowB = -1;
         q4 = 0;
       } else {
@@ -478,13 +490,14 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         if (MODE == SG) {
           if ((q4 & fmask) == 0) {
             // frame R*ext -> 0: lower what this step takes from the row above
+            // (values of row q4 - 1 in frame -ext: still non-negative halves)
             const uint32_t FRAME_DROP = p.pk_drop;
 #pragma unroll
             for (int j = 0; j < K; ++j) {
-              H[j] = __viaddmax_s16x2(H[j], FRAME_DROP, NEGMIN);
-              E[j] = __viaddmax_s16x2(E[j], FRAME_DROP, NEGMIN);
+              H[j] += FRAME_DROP;
+              E[j] += FRAME_DROP;
             }
-            prevH = __viaddmax_s16x2(prevH, FRAME_DROP, NEGMIN);
+            prevH += FRAME_DROP;  // (thread 0's is set below)
           }
         }
       }
@@ -507,20 +520,22 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         wA >>= 16;
         wB >>= 16;
       }
-      // thread 0: what enters the padding from the left, H = hleft in the
-      // row's frame and F = -infinity (semi-global) / 0 (local)
+      // thread 0: what enters the padding from the left, H at its boundary and
+      // F below every value (semi-global: 0; local: F + open = open)
       if (t0) {
-        const uint32_t hf = dup16(hleft + frame_of(q4));
+        const uint32_t hf = LEFT0 + (MODE == SG ? (uint32_t)(q4 & fmask) * LEFT_EXT : 0u);
+        if (MODE == SG) prevH = hf - LEFT_EXT;
 #pragma unroll
         for (int k = 0; k < RPS; ++k) {
-          msgH[k] = hf + (uint32_t)k * EXT2;
-          msgF[k] = FS_IN;
+          msgH[k] = hf + (uint32_t)k * LEFT_EXT;
+          msgF[k] = (MODE == SG) ? 0u : p.pk_fsin;
           msgB[k] = 0u;
         }
       }
     }
     // whether a record of the warp ends in this step's rows (warp-uniform)
-    const bool slow = __any_sync(FULL, busy && (unsigned)(ev_row - q4) < (unsigned)RPS);
+    const bool slow = __any_sync(FULL, busy && ((unsigned)(lenA - 1 - q4) < (unsigned)RPS ||
+                                                (unsigned)(lenB - 1 - q4) < (unsigned)RPS));
 
     if (busy) {
       if (!slow) {
@@ -539,14 +554,14 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
           // (frame(q4 + k) = frame(q4) + k * ext): m = max_k outH[k] - k * ext
           uint32_t m = outH[RPS - 1];
 #pragma unroll
-          for (int k = RPS - 2; k >= 0; --k) m = __viaddmax_s16x2(m, NEXT, outH[k]);
-          const uint32_t nb = __viaddmax_s16x2(m, dup16(-frame_of(q4)), best);
+          for (int k = RPS - 2; k >= 0; --k) m = __viaddmax_u16x2(m, NEXT, outH[k]);
+          const uint32_t nb = __viaddmax_u16x2(m, dup16(-frame_of(q4)), best);
           if (nb != best) {
             // the first row reaching the new maximum, per improved lane
             bool dA = lo16(nb) == lo16(best), dB = hi16(nb) == hi16(best);
 #pragma unroll
             for (int k = 0; k < RPS; ++k) {
-              const uint32_t u = __viaddmax_s16x2(outH[k], dup16(-frame_of(q4 + k)), NEGMIN);
+              const uint32_t u = __viaddmax_u16x2(outH[k], dup16(-frame_of(q4 + k)), 0u);
               if (!dA && lo16(u) == lo16(nb)) {
                 rowA = q4 + k;
                 dA = true;
@@ -584,25 +599,23 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
           outF[RPS - 1] = fs;
           if (MODE == SW) outB[RPS - 1] = sw_track(row, left);
           if (te) te_row(row);
-          if (row == ev_row) on_event(row);
+          if (row == lenA - 1 || row == lenB - 1) on_event(row, msgC);
         }
         prevH = d;
       }
       outC = msgC;
     } else {
-      outC = CTL_IDLE;
+      outC = msgC & (CTL_IDLE | CTL_DONE);
     }
 
     // Every step thread 0 starts reaches thread G-1 within G-1 steps, so the
     // group is done once thread 0 is and no step is in flight.  The step budget
     // (all rows of the range plus the pipeline depth) is a hard stop.
     // (checked every CHK steps; idle extra steps do nothing)
-    if (--chk == 0) {
-      chk = CHK;
-      steps += CHK * RPS;
-      const bool more = busy || (t0 && !f_done);
+    if ((++step & (CHK - 1)) == 0) {
+      const bool more = busy || (t0 && !(outC & CTL_DONE));
       if (!__any_sync(FULL, more)) break;
-      if (steps > p.max_steps) {
+      if (step / CHK > p.max_steps / (CHK * RPS)) {
         if (lane == 0) atomicOr(p.error, 2);
         break;
       }
