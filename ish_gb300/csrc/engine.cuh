@@ -33,8 +33,7 @@ enum ProfLayout : int { PROF_S16 = 0, PROF_PAIR = 1, PROF_S32 = 2 };
 // Control word of the wavefront pipeline (one per row step).
 constexpr uint32_t CTL_NEW = 1u << 16;   // row 0 of a new record pair
 constexpr uint32_t CTL_IDLE = 1u << 17;  // no work in this slot
-constexpr uint32_t CTL_DONE = 1u << 18;  // thread 0: the work counter has run dry
-constexpr int CTL_SEQ_SHIFT = 19;        // 5-bit pair sequence number
+constexpr int CTL_SEQ_SHIFT = 18;        // 5-bit pair sequence number
 
 struct Decision {
   int32_t max_score;
@@ -81,7 +80,6 @@ struct WaveParams {
   uint32_t pk_left_ext;    // ... and its rise per row (0 with a fixed target start)
   uint32_t pk_drop;        // -(R * ext) in both halves as one 32-bit integer: a frame reset
   uint32_t row_bytes;      // profile bytes between consecutive codes' rows ((G * kp) words)
-  const int16_t *hinit;    // H(-1, q) for q in [-d, Q), index c = q + d (semi-global: + c * ext, its frame)
   uint32_t first, count;   // sorted entries [first, first + count) are scored
   uint32_t pair_stride, pair_phase;  // of those, record pairs phase, phase + stride, ... (stride 0: every pair)
   uint32_t *counter;       // work counter (record pairs), zeroed before launch
@@ -107,7 +105,6 @@ struct BatchParams {
   uint32_t ntiles;
   uint32_t *tile_counter;     // one pair counter per tile, zeroed before launch
   uint32_t prof_area;         // shared-memory bytes reserved for the largest profile (16-byte multiple)
-  uint32_t slot_words;        // slot words per block: 32 per group at the class's smallest G
   uint64_t step_cap;          // nonzero: pipeline steps per warp and tile (ISH_OPT_STEP_BUDGET)
 };
 

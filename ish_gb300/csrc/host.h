@@ -54,7 +54,7 @@ struct WaveLayout {
   int G = 0, K = 0, d = 0, kp = 0, layout = 0;
   uint32_t prof_bytes = 0;  // profile rows, then (if remapped) the 256-byte code -> row table
   uint32_t remap_off = 0;   // byte offset of that table, 0: codes are rows
-  DevBuf prof, hinit;
+  DevBuf prof;
 };
 
 struct Query {

@@ -41,7 +41,6 @@ void release_query(Query &q) {
   q.plain_hinit.release();
   for (auto &l : q.layouts) {
     l.second.prof.release();
-    l.second.hinit.release();
   }
   q.layouts.clear();
   for (auto &kv : q.exact_prof) kv.second.release();
@@ -349,18 +348,8 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
     host.insert(host.end(), q.rowmap.begin(), q.rowmap.end());
     L.prof_bytes += 256;
   }
-  std::vector<int16_t> hin((size_t)G * K, 0);
-  for (int c = 0; c < G * K; ++c) {
-    const int col = c - L.d;
-    int v = 0;
-    if (sg && col >= 0 && !(q.ends & ISH_FREE_QUERY_START)) v = -q.open - q.ext * col;
-    if (sg) v += q.ext * c;  // column frame (c + 1) * ext, row frame -ext
-    hin[c] = (int16_t)v;
-  }
   CU(L.prof.ensure(L.prof_bytes));
-  CU(L.hinit.ensure(hin.size() * 2));
   CU(cudaMemcpy(L.prof.p, host.data(), L.prof_bytes, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(L.hinit.p, hin.data(), hin.size() * 2, cudaMemcpyHostToDevice));
   auto res = q.layouts.emplace(key, std::move(L));
   *out = &res.first->second;
   return ISH_OK;
@@ -743,7 +732,6 @@ void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDe
   p.pk_left_ext = sg && ts ? (uint32_t)q.ext * 0x10001u : 0u;
   p.pk_drop = sg ? (uint32_t)(-(p.frame_mask + 1) * q.ext) * 0x10001u : 0u;
   p.row_bytes = (uint32_t)(L.G * L.kp * (L.layout == PROF_S16 ? 2 : 4));
-  p.hinit = L.hinit.as<const int16_t>();
   p.error = error;
   p.rec = RecordsDev{rs.codes.as<const uint8_t>(), rs.off_s.as<const uint64_t>(), rs.len_s.as<const uint32_t>(),
                      rs.orig_s.as<const uint32_t>(), rs.n};
@@ -751,11 +739,11 @@ void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDe
   p.dec = Decision{q.max_score, q.thr};
 }
 
-// Shared memory of a wavefront block: the profile, 32 slot words per group,
+// Shared memory of a wavefront block: the profile, a slot word per thread,
 // and (local alignment) wave_save_words(K) save words per thread (see wave.cuh).
 size_t wave_smem(uint32_t prof_area, int threads, int G, int K, int mode) {
   const size_t save = mode == SW ? (size_t)threads * wave_save_words(K) * 4 : 0;
-  return prof_area + (size_t)(threads / G) * 32 * 4 + save;
+  return prof_area + (size_t)threads * 4 + save;
 }
 
 int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uint32_t count, OutDev out, int G, int K,

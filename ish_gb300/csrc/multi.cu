@@ -209,9 +209,8 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
     c.fn = batch_fn(c.K, c.mode, c.layout, lean);
     if (!c.fn) return fail(ctx, ISH_EOVERFLOW, "no batch kernel for K=%d", c.K);
     c.threads = wave_threads_lean(c.K, c.mode, lean);
-    const size_t slot_words = (size_t)(c.threads / c.Gmin) * 32;
     const size_t save = c.mode == SW ? (size_t)c.threads * wave_save_words(c.K) * 4 : 0;
-    c.smem = c.prof_area + slot_words * 4 + save;
+    c.smem = c.prof_area + (size_t)c.threads * 4 + save;
     CU(cudaFuncSetAttribute((const void *)c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
     int per_sm = 0;
     CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)c.fn, c.threads, c.smem));
@@ -289,7 +288,6 @@ int enqueue_plan(ish_ctx *ctx, MultiPlan &P, RecordSet &rs, cudaStream_t s) {
     b.ntiles = c.ntiles;
     b.tile_counter = P.counters.as<uint32_t>() + c.counter_base;
     b.prof_area = c.prof_area;
-    b.slot_words = (uint32_t)((c.threads / c.Gmin) * 32);
     b.step_cap = ctx->step_budget;
     if (c.ntiles) c.fn<<<c.grid, c.threads, c.smem, cs>>>(b);
     if (c.ntiles) ++P.kernels;

@@ -373,9 +373,8 @@ int step(Server &S, char *msg) {
         return ISH_EOVERFLOW;
       }
       const int threads = wave_threads_lean(C.K, C.mode, lean);
-      const size_t slot_words = (size_t)(threads / C.Gmin) * 32;
       const size_t save = C.mode == SW ? (size_t)threads * wave_save_words(C.K) * 4 : 0;
-      const size_t smem = C.prof_area + slot_words * 4 + save;
+      const size_t smem = C.prof_area + (size_t)threads * 4 + save;
       SCU(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       int per_sm = 0;
       SCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, threads, smem));
@@ -389,7 +388,6 @@ int step(Server &S, char *msg) {
       b.ntiles = C.count;
       b.tile_counter = S.step_counters.as<uint32_t>() + C.first;
       b.prof_area = C.prof_area;
-      b.slot_words = (uint32_t)slot_words;
       b.step_cap = S.ctx->step_budget;
       cudaStream_t cs = c == 0 ? s : S.side[c - 1];
       if (c > 0) SCU(cudaStreamWaitEvent(cs, S.fork, 0));

@@ -58,9 +58,9 @@ namespace ish {
 
 // Scores sorted entries [p.first, p.first + p.count) of the record set: the
 // groups of the calling block take record pairs from *counter until none are
-// left.  `prof` is the profile in shared memory; `slots_all` holds 32 words per
-// group (pair indices in flight), `save_all` wave_save_words(K) words per thread (local
-// alignment only).
+// left.  `prof` is the profile in shared memory; `slots_all` holds one word per
+// thread (a group's G pair indices in flight), `save_all` wave_save_words(K)
+// words per thread (local alignment only).
 template <int K, int MODE, int LAYOUT>
 __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned char *prof, uint32_t *slots_all,
                                           uint32_t *save_all, uint32_t *counter) {
@@ -71,7 +71,10 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   const int lane = tid & 31;
   const int t = lane & (G - 1);
   const bool t0 = t == 0;
-  uint32_t *slots = slots_all + (tid / G) * 32;
+  // pair indices in flight in the group, by sequence number modulo G: a pair
+  // is in at most G consecutive steps' threads, so thread 0 rewrites its slot
+  // only after thread G-1 has left it
+  uint32_t *slots = slots_all + (tid & ~(G - 1));
   // local alignment: per thread, the H row of the last improvement of each lane
   constexpr int KP8 = (K + 7) & ~7;
   uint16_t *saveA = reinterpret_cast<uint16_t *>(save_all + tid * wave_save_words(K));
@@ -82,6 +85,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   const uint32_t NEXT = p.pk_next;
   // semi-global: a gap opens from H at ext - open in the frames
   const uint32_t EOPEN = p.pk_eopen;
+  const uint32_t EOPEN_SUM = (uint32_t)(p.ext - p.open) * 0x10001u;  // ... as one integer for both halves
   const bool te = (MODE == SG) && (p.ends & 8);
   const bool qe = (MODE == SG) && (p.ends & 2);
   // record pairs of the range: every pair_stride-th from pair_phase
@@ -119,6 +123,9 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   for (int k = 0; k < RPS; ++k) outH[k] = outF[k] = outB[k] = 0;
   uint32_t outC = CTL_IDLE;
   int q4 = 0, lenA = 0, lenB = 0;  // q4: row of the step's first row
+  // the next q4 at which this thread has anything beside its rows to do, and
+  // (thread 0) the q4 at which its pair has no rows left
+  int wake = t0 ? RPS : 0x7fffffff, end_q = t0 ? RPS : -1;
   // this thread's record streams: 4 codes per 32-bit word, one word ahead
   const uint8_t *pa = nullptr, *pb = nullptr;
   uint32_t wA = 0, wB = 0, nA = 0, nB = 0;
@@ -129,10 +136,18 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   uint32_t best = 0;
   int rowA = -1, rowB = -1;  // first row of the lane's maximum
   uint32_t oR0 = 0, oR1 = 0, oR2 = 0, oR3 = 0;  // last-row partials for thread t+1
-  uint32_t iR0 = 0, iR1 = 0, iR2 = 0, iR3 = 0;  // ... and those of thread t-1, in the step after
-  bool has_out = false;
+  bool ended = false;  // a record of the warp ended in the last step
   const bool remap = remap_off != 0;
+  // whether the ends of records matter to this thread: with the query end
+  // fixed, only the last column (thread G-1) gives a semi-global result
+  const bool ends_here = MODE == SW || qe || t == G - 1;
+  // thread 0 of the group holds the next pair's number: it is taken CLAIM rows
+  // before the current pair ends, late enough that a group with a long pair
+  // leaves the next ones to the others, and early enough that neither the
+  // counter nor the new pair's lengths and codes are waited for
+  uint32_t f_next = t0 ? atomicAdd(counter, 1u) : 0u;
   constexpr int CHK = 8 / RPS;  // steps between termination checks
+  constexpr int CLAIM = 32, LOOK_META = 20, LOOK_CODES = 8;  // rows before a pair's end (see below)
   uint32_t step = 0;
 
   // One row of the pair with record codes cA, cB: `diag` is H of the row above
@@ -230,17 +245,19 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
     return fs;
   };
 
-  // Local alignment, after row `row`: only a row maximum above every cell so
+  // Local alignment, after row `row` (`live`: the halves of the lanes whose
+  // record holds that row): only a row maximum above every cell so
   // far in this thread AND in all columns to its left (`left`, their running
   // best up to this row, passed along the pipeline) can be the first row of
   // the record's maximum at its smallest column; anything else is dominated
   // (smaller, or equal in an earlier row or a smaller column), so only those
   // improvements are recorded.  Returns the running best passed on.
-  auto sw_track = [&](int row, uint32_t left) -> uint32_t {
+  auto sw_track = [&](int row, uint32_t left, uint32_t live) -> uint32_t {
     uint32_t cm = H[0];
 #pragma unroll
     for (int j = 1; j + 1 < K; j += 2) cm = __vimax3_s16x2(cm, H[j], H[j + 1]);
     if ((K & 1) == 0 && K > 1) cm = __viaddmax_s16x2(cm, 0u, H[K - 1]);
+    cm &= live;
     const uint32_t thr = __viaddmax_s16x2(best, 0u, left);
     const uint32_t nb = __viaddmax_s16x2(thr, 0u, cm);
     if (nb != thr) {
@@ -292,133 +309,125 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
     o = (a ? (v & 0xffffu) : (o & 0xffffu)) | (b ? (v & 0xffff0000u) : (o & 0xffff0000u));
   };
 
-  // The last row of one or both records of the pair (H holds it): fold the
-  // partial results left to right -- thread t-1's arrived as iR at the start
-  // of this step, this thread's leave as oR at the next -- and thread G-1
-  // writes the record's outputs.
-  auto on_event = [&](int row, uint32_t ctl) {
+  // Outputs of the pair's record x (0: A, 1: B), written by thread G-1.
+  auto put_out = [&](int x, uint32_t pr, int score, int eq, int er) {
+    const uint32_t orig = p.rec.orig[p.first + 2 * pr + x];
+    if (p.out.score) p.out.score[orig] = score;
+    if (p.out.qend) p.out.qend[orig] = eq;
+    if (p.out.tend) p.out.tend[orig] = er;
+    if (p.out.hit) p.out.hit[orig] = decide(MODE, score, eq, er, p.dec);
+  };
+  const int last_off = (MODE == SG) ? p.bias + G * K * ext : 0;  // bias and frame of the last column
+
+  // Semi-global with a free query end, at the last row of one or both records
+  // (H holds it): fold the maximum of the last row left to right -- thread
+  // t-1's partial arrived as iR at the start of this step, this thread's leaves
+  // as oR at the next.
+  auto qe_event = [&](int row, uint32_t ctl, uint32_t iR0, uint32_t iR1) {
     const bool lastA = row == lenA - 1, lastB = row == lenB - 1;
-    // the pair: its slot is rewritten only 32 pairs later
-    const uint32_t pr = slots[(ctl >> CTL_SEQ_SHIFT) & 31];
-    if (MODE == SG) {
-      uint32_t mx = 0, mq = 0;
-      if (qe) {
-        int bA = 0, bB = 0, qA = 0x7fff, qB = 0x7fff;  // H + bias + row frame, above 0
-        uint32_t row_h[K];  // staged as in the local-alignment scan
+    int bA = 0, bB = 0, qA = 0x7fff, qB = 0x7fff;  // H + bias + row frame, above 0
+    uint32_t row_h[K];  // staged: the loop indexes it
 #pragma unroll
-        for (int j = 0; j < K; ++j) row_h[j] = H[j];
+    for (int j = 0; j < K; ++j) row_h[j] = H[j];
 #pragma unroll 1
-        for (int j = 0; j < K; ++j) {
-          if (col0 + j >= 0) {
-            const int cf = (t * K + j + 1) * ext;
-            const int a = ulo16(row_h[j]) - cf, b = uhi16(row_h[j]) - cf;
-            if (a > bA) {
-              bA = a;
-              qA = col0 + j;
-            }
-            if (b > bB) {
-              bB = b;
-              qB = col0 + j;
-            }
-          }
+    for (int j = 0; j < K; ++j) {
+      if (col0 + j >= 0) {
+        const int cf = (t * K + j + 1) * ext;
+        const int a = ulo16(row_h[j]) - cf, b = uhi16(row_h[j]) - cf;
+        if (a > bA) {
+          bA = a;
+          qA = col0 + j;
         }
-        if (t > 0) {  // columns to the left win ties
-          if (!(bA > ulo16(iR0))) {
-            bA = ulo16(iR0);
-            qA = (int)(iR1 & 0xffffu);
-          }
-          if (!(bB > uhi16(iR0))) {
-            bB = uhi16(iR0);
-            qB = (int)(iR1 >> 16);
-          }
-        }
-        mx = (uint32_t)(bA & 0xffff) | ((uint32_t)bB << 16);
-        mq = (uint32_t)qA | ((uint32_t)qB << 16);
-        if (t < G - 1) {
-          put_lanes(oR0, mx, lastA, lastB);
-          put_lanes(oR1, mq, lastA, lastB);
-          has_out = true;
-        }
-      }
-      if (t == G - 1) {
-        const int last_off = p.bias + G * K * ext;  // bias and column frame of the last column
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (!(x == 0 ? lastA : lastB)) continue;
-          const uint32_t orig = p.rec.orig[p.first + 2 * pr + x];
-          const int T = x == 0 ? lenA : lenB;
-          int score, er, eq = p.Q - 1;
-          if (!te && !qe) {
-            score = (x == 0 ? ulo16(H[K - 1]) : uhi16(H[K - 1])) - frame_of(row) - last_off;  // this row's H(i, Q-1)
-            er = T - 1;
-          } else {
-            score = te ? (x == 0 ? ulo16(best) : uhi16(best)) - last_off : p.neg_limit;
-            er = x == 0 ? rowA : rowB;
-            if (qe) {
-              const int s1 = (x == 0 ? ulo16(mx) : uhi16(mx)) - frame_of(row) - p.bias;
-              const int t1 = x == 0 ? (int)(mq & 0xffffu) : (int)(mq >> 16);
-              if (s1 > score) {
-                score = s1;
-                er = T - 1;
-                eq = t1;
-              } else if (s1 == score && er == T - 1 && t1 < eq) {
-                eq = t1;
-              }
-            }
-          }
-          if (p.out.score) p.out.score[orig] = score;
-          if (p.out.qend) p.out.qend[orig] = eq;
-          if (p.out.tend) p.out.tend[orig] = er;
-          if (p.out.hit) p.out.hit[orig] = decide(SG, score, eq, er, p.dec);
-        }
-      }
-    } else {
-      int bA = lo16(best), bB = hi16(best), rA = rowA, rB = rowB, qA = 0x7fff, qB = 0x7fff;
-      // smallest column of this thread's maximum in its first row
-#pragma unroll 1
-      for (int j = K - 1; j >= 0; --j) {
-        if (bA > 0 && (int)(int16_t)saveA[j] == bA) qA = col0 + j;
-        if (bB > 0 && (int)(int16_t)saveB[j] == bB) qB = col0 + j;
-      }
-      if (t > 0) {
-        const int ia = lo16(iR0), ib = hi16(iR0), ira = (int)iR2, irb = (int)iR3;
-        const int iqa = (int)(int16_t)(iR1 & 0xffffu), iqb = (int)(int16_t)(iR1 >> 16);
-        if (ia > bA || (ia == bA && (ira < rA || (ira == rA && iqa < qA)))) {
-          bA = ia;
-          rA = ira;
-          qA = iqa;
-        }
-        if (ib > bB || (ib == bB && (irb < rB || (irb == rB && iqb < qB)))) {
-          bB = ib;
-          rB = irb;
-          qB = iqb;
-        }
-      }
-      if (t < G - 1) {
-        put_lanes(oR0, (uint32_t)(bA & 0xffff) | ((uint32_t)bB << 16), lastA, lastB);
-        put_lanes(oR1, (uint32_t)(qA & 0xffff) | ((uint32_t)qB << 16), lastA, lastB);
-        if (lastA) oR2 = (uint32_t)rA;
-        if (lastB) oR3 = (uint32_t)rB;
-        has_out = true;
-      } else {
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          if (!(x == 0 ? lastA : lastB)) continue;
-          const uint32_t orig = p.rec.orig[p.first + 2 * pr + x];
-          int score = x == 0 ? bA : bB, er = x == 0 ? rA : rB, eq = x == 0 ? qA : qB;
-          if (score == 0) {
-            er = -1;
-            eq = 0;
-          }
-          if (p.out.score) p.out.score[orig] = score;
-          if (p.out.qend) p.out.qend[orig] = eq;
-          if (p.out.tend) p.out.tend[orig] = er;
-          if (p.out.hit) p.out.hit[orig] = decide(SW, score, eq, er, p.dec);
+        if (b > bB) {
+          bB = b;
+          qB = col0 + j;
         }
       }
     }
+    if (t > 0) {  // columns to the left win ties
+      if (!(bA > ulo16(iR0))) {
+        bA = ulo16(iR0);
+        qA = (int)(iR1 & 0xffffu);
+      }
+      if (!(bB > uhi16(iR0))) {
+        bB = uhi16(iR0);
+        qB = (int)(iR1 >> 16);
+      }
+    }
+    if (t < G - 1) {
+      put_lanes(oR0, (uint32_t)(bA & 0xffff) | ((uint32_t)bB << 16), lastA, lastB);
+      put_lanes(oR1, (uint32_t)qA | ((uint32_t)qB << 16), lastA, lastB);
+      return;
+    }
+    const uint32_t pr = slots[(ctl >> CTL_SEQ_SHIFT) & (G - 1)];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      if (!(x == 0 ? lastA : lastB)) continue;
+      const int T = x == 0 ? lenA : lenB;
+      int score = te ? (x == 0 ? ulo16(best) : uhi16(best)) - last_off : p.neg_limit;
+      int er = x == 0 ? rowA : rowB, eq = p.Q - 1;
+      const int s1 = (x == 0 ? bA : bB) - frame_of(row) - p.bias, t1 = x == 0 ? qA : qB;
+      if (s1 > score) {
+        score = s1;
+        er = T - 1;
+        eq = t1;
+      } else if (s1 == score && er == T - 1 && t1 < eq) {
+        eq = t1;
+      }
+      put_out(x, pr, score, eq, er);
+    }
   };
 
+  // Local alignment, after the step in which one or both records end: fold the
+  // partial results left to right, as above.  Columns to the left win ties, so
+  // the saved row is searched for its column only where this thread's best
+  // beats the partial that came in.
+  auto sw_event = [&](uint32_t ctl, uint32_t iR0, uint32_t iR1, uint32_t iR2, uint32_t iR3) {
+    const bool lastA = (unsigned)(lenA - 1 - q4) < (unsigned)RPS, lastB = (unsigned)(lenB - 1 - q4) < (unsigned)RPS;
+    int bA = lo16(iR0), bB = hi16(iR0), rA = (int)iR2, rB = (int)iR3;
+    int qA = (int)(int16_t)(iR1 & 0xffffu), qB = (int)(int16_t)(iR1 >> 16);
+    if (t == 0) {
+      bA = bB = 0;
+      rA = rB = -1;
+      qA = qB = 0x7fff;
+    }
+    const int mA = lo16(best), mB = hi16(best);
+    const bool ownA = lastA && (mA > bA || (mA == bA && mA > 0 && rowA < rA));
+    const bool ownB = lastB && (mB > bB || (mB == bB && mB > 0 && rowB < rB));
+    if (ownA) {
+      bA = mA;
+      rA = rowA;
+    }
+    if (ownB) {
+      bB = mB;
+      rB = rowB;
+    }
+    if (ownA || ownB) {  // smallest column of this thread's maximum in its first row
+      const uint32_t *wa = reinterpret_cast<const uint32_t *>(saveA), *wb = reinterpret_cast<const uint32_t *>(saveB);
+#pragma unroll 1
+      for (int v = (K + 1) / 2 - 1; v >= 0; --v) {
+        const uint32_t a = wa[v], b = wb[v];
+        if (ownA && 2 * v + 1 < K && hi16(a) == bA) qA = col0 + 2 * v + 1;
+        if (ownA && lo16(a) == bA) qA = col0 + 2 * v;
+        if (ownB && 2 * v + 1 < K && hi16(b) == bB) qB = col0 + 2 * v + 1;
+        if (ownB && lo16(b) == bB) qB = col0 + 2 * v;
+      }
+    }
+    if (t < G - 1) {
+      put_lanes(oR0, (uint32_t)(bA & 0xffff) | ((uint32_t)bB << 16), lastA, lastB);
+      put_lanes(oR1, (uint32_t)(qA & 0xffff) | ((uint32_t)qB << 16), lastA, lastB);
+      if (lastA) oR2 = (uint32_t)rA;
+      if (lastB) oR3 = (uint32_t)rB;
+      return;
+    }
+    const uint32_t pr = slots[(ctl >> CTL_SEQ_SHIFT) & (G - 1)];
+    if (lastA) put_out(0, pr, bA, bA ? qA : 0, bA ? rA : -1);
+    if (lastB) put_out(1, pr, bB, bB ? qB : 0, bB ? rB : -1);
+  };
+
+  // Every thread of the warp computes every step: an idle one (no record pair
+  // in its pipeline slot) works on what its last pair left, whose lanes are
+  // final, and a new pair resets all of its state.
   while (true) {
     __syncwarp();
     uint32_t msgH[RPS], msgF[RPS], msgB[RPS];
@@ -428,40 +437,38 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       msgF[k] = __shfl_up_sync(FULL, outF[k], 1, G);
       msgB[k] = (MODE == SW) ? __shfl_up_sync(FULL, outB[k], 1, G) : 0u;
     }
-    uint32_t msgC = __shfl_up_sync(FULL, outC, 1, G);  // thread 0: its own last control word
+    uint32_t msgC = __shfl_up_sync(FULL, outC, 1, G);
+    if (t0) msgC &= ~CTL_NEW;  // its own last control word
     // partial results of records that ended in thread t-1's previous step
-    if (__any_sync(FULL, has_out)) {
+    uint32_t iR0 = 0, iR1 = 0, iR2 = 0, iR3 = 0;
+    if ((MODE == SW || qe) && ended) {
       iR0 = __shfl_up_sync(FULL, oR0, 1, G);
       iR1 = __shfl_up_sync(FULL, oR1, 1, G);
       if (MODE == SW) {
         iR2 = __shfl_up_sync(FULL, oR2, 1, G);
         iR3 = __shfl_up_sync(FULL, oR3, 1, G);
       }
-      has_out = false;
     }
-
-    if (t0) {
-      // thread 0 of the group goes on with its pair or takes the next one
-      msgC &= ~CTL_NEW;
-      if ((msgC & CTL_IDLE) || q4 + RPS >= max(lenA, lenB)) {
-        msgC |= CTL_IDLE;
-        if (!(msgC & CTL_DONE)) {
-          const uint32_t nt = atomicAdd(counter, 1u);
-          const uint32_t seq = ((msgC >> CTL_SEQ_SHIFT) + 1) & 31;
-          if (nt < npairs) {
-            slots[seq] = nt * pstride + pphase;  // the pair's index in the range
-            msgC = CTL_NEW | (seq << CTL_SEQ_SHIFT);
-          } else {
-            msgC = CTL_IDLE | CTL_DONE;
-          }
-        }
+    q4 += RPS;
+    // Everything beside the rows -- new pairs, frame resets, the look-ahead,
+    // record ends -- happens in steps that some thread of the warp waits for,
+    // so the others pay one comparison and one vote for all of it.
+    bool endA = false, endB = false, ends = false;
+    if (__any_sync(FULL, (msgC & CTL_NEW) || q4 == wake)) {
+      if (t0 && q4 == end_q) {  // thread 0 of the group takes the next pair
+        const uint32_t seq = (outC + (1u << CTL_SEQ_SHIFT)) & (31u << CTL_SEQ_SHIFT);
+        msgC = seq | (f_next < npairs ? CTL_NEW : CTL_IDLE);
       }
-    }
-
-    const bool busy = !(msgC & CTL_IDLE);
-    if (busy) {
-      if (msgC & CTL_NEW) {
-        const uint32_t pr = slots[(msgC >> CTL_SEQ_SHIFT) & 31];
+      const bool fresh = msgC & CTL_NEW;
+      if (fresh) q4 = 0;
+      const auto at = [&](int r) { return (unsigned)(max(lenA, lenB) - q4 - r) < (unsigned)RPS; };
+      if (fresh) {
+        uint32_t pr = f_next * pstride + pphase;  // the pair's index in the range
+        if (t0) {
+          slots[(msgC >> CTL_SEQ_SHIFT) & (G - 1)] = pr;
+        } else {
+          pr = slots[(msgC >> CTL_SEQ_SHIFT) & (G - 1)];
+        }
         const uint32_t sA = p.first + 2 * pr;
         lenA = (int)p.rec.len[sA];
         pa = p.rec.codes + p.rec.off[sA];
@@ -472,83 +479,155 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
           lenB = 0;
           pb = pa;
         }
+        if (t0) {
+          end_q = (max(max(lenA, lenB), 1) + RPS - 1) & ~(RPS - 1);
+          if (max(lenA, lenB) < CLAIM + RPS) f_next = atomicAdd(counter, 1u);
+        }
         nA = __ldg(reinterpret_cast<const uint32_t *>(pa));
         nB = lenB ? __ldg(reinterpret_cast<const uint32_t *>(pb)) : 0u;
-        const int16_t *hi = p.hinit + t * K;
+        // row -1: H(-1, c) is 0 in the padding and with a free query start,
+        // -open - ext * q else; with its frame c * ext (column frame less one
+        // row's) that is bias + c * ext, or one value for all of the query
+        const int h_query = p.bias + p.d * ext - p.open;
+        const bool qs = p.ends & 1;
 #pragma unroll
         for (int j = 0; j < K; ++j) {
-          const int h0 = hi[j] + p.bias;
-          H[j] = (MODE == SW) ? 0u : dup16(h0);
-          E[j] = (MODE == SW) ? 0u : dup16(h0 + ext - p.open);  // row 0's frame is one ext above row -1's
+          const int c = t * K + j;
+          const uint32_t h0 = (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
+          H[j] = (MODE == SW) ? 0u : h0;
+          E[j] = (MODE == SW) ? 0u : h0 + EOPEN_SUM;  // row 0's frame is one ext above row -1's
         }
-        prevH = (MODE == SW || t0) ? 0u : dup16(p.hinit[t * K - 1] + p.bias);  // t0: set below
+        {
+          const int c = t * K - 1;
+          prevH = (MODE == SW) ? 0u : (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
+        }
         best = (MODE == SG && t != G - 1) ? 0xffffffffu : 0u;
         rowA = rowB = -1;
-        q4 = 0;
       } else {
-        q4 += RPS;
-        if (MODE == SG) {
-          if ((q4 & fmask) == 0) {
-            // frame R*ext -> 0: lower what this step takes from the row above
-            // (values of row q4 - 1 in frame -ext: still non-negative halves)
-            const uint32_t FRAME_DROP = p.pk_drop;
+        if (MODE == SG && (q4 & fmask) == 0) {
+          // frame R*ext -> 0: lower what this step takes from the row above
+          // (values of row q4 - 1 in frame -ext: still non-negative halves)
+          const uint32_t FRAME_DROP = p.pk_drop;
 #pragma unroll
-            for (int j = 0; j < K; ++j) {
-              H[j] += FRAME_DROP;
-              E[j] += FRAME_DROP;
-            }
-            prevH += FRAME_DROP;  // (thread 0's is set below)
+          for (int j = 0; j < K; ++j) {
+            H[j] += FRAME_DROP;
+            E[j] += FRAME_DROP;
+          }
+          prevH += FRAME_DROP;  // (thread 0's is set below)
+        }
+        // thread 0: the next pair is claimed, and what it needs first is
+        // fetched into L1
+        if (t0 && at(CLAIM)) f_next = atomicAdd(counter, 1u);
+        if (t0 && (at(LOOK_META) || at(LOOK_CODES)) && f_next < npairs) {
+          const uint32_t sA = p.first + 2 * (f_next * pstride + pphase);
+          if (at(LOOK_META)) {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p.rec.len + sA));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p.rec.off + sA));
+          } else {
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(p.rec.codes + p.rec.off[sA]));
+            if (sA + 1 < p.first + p.count)
+              asm volatile("prefetch.global.L1 [%0];" ::"l"(p.rec.codes + p.rec.off[sA + 1]));
           }
         }
       }
-      // ---- record codes of this step ----
-      // Codes were checked against the alphabet when the set was loaded and
-      // every record slot is zero-padded to 16 bytes.  Past a record's end the
-      // last word repeats: those rows only feed a lane whose result is final.
-      if (RPS == 4 || (q4 & 3) == 0) {
-        wA = nA;
-        wB = nB;
-        if (q4 + 4 < lenA) nA = __ldg(reinterpret_cast<const uint32_t *>(pa + q4 + 4));
-        if (q4 + 4 < lenB) nB = __ldg(reinterpret_cast<const uint32_t *>(pb + q4 + 4));
-        // long records: the codes 256 rows ahead are pulled into L1, so the
-        // group's loads hit L1 even when few warps are left to hide latency
-        if ((q4 & 127) == 0) {
-          if (q4 + 256 < lenA) asm volatile("prefetch.global.L1 [%0];" ::"l"(pa + q4 + 256));
-          if (q4 + 256 < lenB) asm volatile("prefetch.global.L1 [%0];" ::"l"(pb + q4 + 256));
-        }
-      } else {
-        wA >>= 16;
-        wB >>= 16;
+      // long records: the codes 256 rows ahead are pulled into L1, so the
+      // group's loads hit L1 even when few warps are left to hide latency
+      if (t0 && (q4 & 127) == 0) {
+        if (q4 + 256 < lenA) asm volatile("prefetch.global.L1 [%0];" ::"l"(pa + q4 + 256));
+        if (q4 + 256 < lenB) asm volatile("prefetch.global.L1 [%0];" ::"l"(pb + q4 + 256));
       }
-      // thread 0: what enters the padding from the left, H at its boundary and
-      // F below every value (semi-global: 0; local: F + open = open)
+      // whether a record of the warp ends in this step's rows (warp-uniform)
+      endA = ends_here && (unsigned)(lenA - 1 - q4) < (unsigned)RPS;
+      endB = ends_here && (unsigned)(lenB - 1 - q4) < (unsigned)RPS;
+      ends = __any_sync(FULL, endA || endB);
+      // the next step to wait for
+      wake = 0x7fffffff;
+      const auto wait_for = [&](int q) {
+        if (q > q4) wake = min(wake, q);
+      };
+      if (MODE == SG) wait_for((q4 | fmask) + 1);
+      if (ends_here) {
+        wait_for((lenA - 1) & ~(RPS - 1));
+        wait_for((lenB - 1) & ~(RPS - 1));
+      }
       if (t0) {
-        const uint32_t hf = LEFT0 + (MODE == SG ? (uint32_t)(q4 & fmask) * LEFT_EXT : 0u);
-        if (MODE == SG) prevH = hf - LEFT_EXT;
-#pragma unroll
-        for (int k = 0; k < RPS; ++k) {
-          msgH[k] = hf + (uint32_t)k * LEFT_EXT;
-          msgF[k] = (MODE == SG) ? 0u : p.pk_fsin;
-          msgB[k] = 0u;
-        }
+        const int rows = max(lenA, lenB);
+        wait_for(end_q);
+        wait_for((rows - CLAIM) & ~(RPS - 1));
+        wait_for((rows - LOOK_META) & ~(RPS - 1));
+        wait_for((rows - LOOK_CODES) & ~(RPS - 1));
+        if ((q4 | 127) + 256 < rows) wait_for((q4 | 127) + 1);
       }
     }
-    // whether a record of the warp ends in this step's rows (warp-uniform)
-    const bool slow = __any_sync(FULL, busy && ((unsigned)(lenA - 1 - q4) < (unsigned)RPS ||
-                                                (unsigned)(lenB - 1 - q4) < (unsigned)RPS));
-
-    if (busy) {
-      if (!slow) {
-        // ---- the step's rows, no record ending ----
+    ended = ends;
+    outC = msgC;
+    // ---- record codes of this step ----
+    // Codes were checked against the alphabet when the set was loaded and
+    // every record slot is zero-padded to 16 bytes.  Past a record's end the
+    // last word repeats: those rows only feed a lane whose result is final.
+    if (RPS == 4 || (q4 & 3) == 0) {
+      wA = nA;
+      wB = nB;
+      if (q4 + 4 < lenA) nA = __ldg(reinterpret_cast<const uint32_t *>(pa + q4 + 4));
+      if (q4 + 4 < lenB) nB = __ldg(reinterpret_cast<const uint32_t *>(pb + q4 + 4));
+    } else {
+      wA >>= 16;
+      wB >>= 16;
+    }
+    // thread 0: what enters the padding from the left, H at its boundary and
+    // F below every value (semi-global: 0; local: F + open = open)
+    if (t0) {
+      const uint32_t hf = LEFT0 + (MODE == SG ? (uint32_t)(q4 & fmask) * LEFT_EXT : 0u);
+      if (MODE == SG) prevH = hf - LEFT_EXT;
 #pragma unroll
-        for (int k = 0; k < RPS; ++k) {
-          const uint32_t fs = row_step(__byte_perm(wA, 0u, 0x4440 + k), __byte_perm(wB, 0u, 0x4440 + k),
-                                       k == 0 ? prevH : msgH[k - 1], msgF[k]);
-          outH[k] = H[K - 1];
-          outF[k] = fs;
-          if (MODE == SW) outB[k] = sw_track(q4 + k, msgB[k]);
+      for (int k = 0; k < RPS; ++k) {
+        msgH[k] = hf + (uint32_t)k * LEFT_EXT;
+        msgF[k] = (MODE == SG) ? 0u : p.pk_fsin;
+        msgB[k] = 0u;
+      }
+    }
+    if (MODE == SG && qe && ends) {
+      // ---- free query end, a record of the warp ends: one row at a time, with
+      // the last row's maximum taken after it ----
+      uint32_t d = prevH, sA = wA, sB = wB;
+#pragma unroll 1
+      for (int k = 0; k < RPS; ++k) {
+        const int row = q4 + k;
+        const uint32_t fs = row_step(sA & 0xffu, sB & 0xffu, d, msgF[0]);
+        sA >>= 8;
+        sB >>= 8;
+        d = msgH[0];
+#pragma unroll
+        for (int j = 0; j + 1 < RPS; ++j) {
+          msgH[j] = msgH[j + 1];
+          msgF[j] = msgF[j + 1];
+          outH[j] = outH[j + 1];
+          outF[j] = outF[j + 1];
         }
-        prevH = msgH[RPS - 1];
+        outH[RPS - 1] = H[K - 1];
+        outF[RPS - 1] = fs;
+        if (te) te_row(row);
+        if (row == lenA - 1 || row == lenB - 1) qe_event(row, msgC, iR0, iR1);
+      }
+      prevH = d;
+    } else {
+      // ---- the step's rows ----
+#pragma unroll
+      for (int k = 0; k < RPS; ++k) {
+        const uint32_t fs = row_step(__byte_perm(wA, 0u, 0x4440 + k), __byte_perm(wB, 0u, 0x4440 + k),
+                                     k == 0 ? prevH : msgH[k - 1], msgF[k]);
+        outH[k] = H[K - 1];
+        outF[k] = fs;
+        if (MODE == SW) {
+          uint32_t live = 0xffffffffu;  // a record that ended in this step has no further rows
+          if (k > 0 && ends) live = (q4 + k == lenA ? 0u : 0xffffu) | (q4 + k == lenB ? 0u : 0xffff0000u);
+          outB[k] = sw_track(q4 + k, msgB[k], live);
+        }
+      }
+      prevH = msgH[RPS - 1];
+      if (MODE == SW) {
+        if (endA || endB) sw_event(msgC, iR0, iR1, iR2, iR3);
+      } else if (!ends) {
         if (te) {
           // the largest H(., Q-1) of the step's rows without their frames
           // (frame(q4 + k) = frame(q4) + k * ext): m = max_k outH[k] - k * ext
@@ -574,47 +653,40 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
             best = nb;
           }
         }
-      } else {
-        // ---- a record of the warp ends in these rows: one row at a time,
-        // with the end-of-record work after its last row ----
-        uint32_t d = prevH, sA = wA, sB = wB;
-#pragma unroll 1
-        for (int k = 0; k < RPS; ++k) {
-          const int row = q4 + k;
-          const uint32_t fs = row_step(sA & 0xffu, sB & 0xffu, d, msgF[0]);
-          sA >>= 8;
-          sB >>= 8;
-          d = msgH[0];
-          const uint32_t left = msgB[0];
+      } else if (t == G - 1) {
+        // a record of the warp ends: row by row, this thread's records up to
+        // their last row, then their outputs
+        int sA = 0, sB = 0;
 #pragma unroll
-          for (int j = 0; j + 1 < RPS; ++j) {
-            msgH[j] = msgH[j + 1];
-            msgF[j] = msgF[j + 1];
-            msgB[j] = msgB[j + 1];
-            outH[j] = outH[j + 1];
-            outF[j] = outF[j + 1];
-            outB[j] = outB[j + 1];
+        for (int k = 0; k < RPS; ++k) {
+          const uint32_t u = __viaddmax_u16x2(outH[k], dup16(-frame_of(q4 + k)), 0u);
+          const bool inA = q4 + k < lenA, inB = q4 + k < lenB;
+          if (inA) sA = ulo16(u);
+          if (inB) sB = uhi16(u);
+          if (te && inA && ulo16(u) > ulo16(best)) {
+            best = (best & 0xffff0000u) | (u & 0xffffu);
+            rowA = q4 + k;
           }
-          outH[RPS - 1] = H[K - 1];
-          outF[RPS - 1] = fs;
-          if (MODE == SW) outB[RPS - 1] = sw_track(row, left);
-          if (te) te_row(row);
-          if (row == lenA - 1 || row == lenB - 1) on_event(row, msgC);
+          if (te && inB && uhi16(u) > uhi16(best)) {
+            best = (best & 0xffffu) | (u & 0xffff0000u);
+            rowB = q4 + k;
+          }
         }
-        prevH = d;
+        if (endA || endB) {
+          const uint32_t pr = slots[(msgC >> CTL_SEQ_SHIFT) & (G - 1)];
+          if (endA) put_out(0, pr, (te ? ulo16(best) : sA) - last_off, p.Q - 1, te ? rowA : lenA - 1);
+          if (endB) put_out(1, pr, (te ? uhi16(best) : sB) - last_off, p.Q - 1, te ? rowB : lenB - 1);
+        }
       }
-      outC = msgC;
-    } else {
-      outC = msgC & (CTL_IDLE | CTL_DONE);
     }
 
-    // Every step thread 0 starts reaches thread G-1 within G-1 steps, so the
-    // group is done once thread 0 is and no step is in flight.  The step budget
+    // Every step thread 0 starts reaches thread G-1 within G-1 steps, and thread
+    // 0 idles only when no pair is left, so the group is done once all of its
+    // threads idle.  The step budget
     // (all rows of the range plus the pipeline depth) is a hard stop.
     // (checked every CHK steps; idle extra steps do nothing)
     if ((++step & (CHK - 1)) == 0) {
-      const bool more = busy || (t0 && !(outC & CTL_DONE));
-      if (!__any_sync(FULL, more)) break;
+      if (!__any_sync(FULL, !(outC & CTL_IDLE))) break;
       if (step / CHK > p.max_steps / (CHK * RPS)) {
         if (lane == 0) atomicOr(p.error, 2);
         break;
@@ -636,7 +708,7 @@ __device__ __forceinline__ void wave_rows_smem_params(const WaveParams &p, const
   wave_rows<K, MODE, LAYOUT>(sp, prof, slots_all, save_all, p.counter);
 }
 
-// Shared memory of a block: the profile, then 32 slot words per group, then
+// Shared memory of a block: the profile, then a slot word per thread, then
 // (local alignment) wave_save_words(K) save words per thread.
 template <int K, int MODE, int LAYOUT, int LEAN = 0>
 __global__ void __launch_bounds__(wave_threads_lean(K, MODE, LEAN), wave_blocks_lean(K, MODE, LEAN))
@@ -649,7 +721,7 @@ __global__ void __launch_bounds__(wave_threads_lean(K, MODE, LEAN), wave_blocks_
     for (uint32_t i = threadIdx.x; i < nvec; i += blockDim.x) dst[i] = src[i];
   }
   uint32_t *slots_all = reinterpret_cast<uint32_t *>(smem_raw + ((p.prof_bytes + 15u) & ~15u));
-  uint32_t *save_all = slots_all + (blockDim.x / p.G) * 32;
+  uint32_t *save_all = slots_all + blockDim.x;
   if constexpr (WAVE_PARAMS_SMEM(K, MODE, LEAN)) {
     wave_rows_smem_params<K, MODE, LAYOUT>(p, smem_raw, slots_all, save_all);
   } else {
@@ -673,7 +745,7 @@ __global__ void __launch_bounds__(wave_threads_lean(K, MODE, LEAN), wave_blocks_
   __shared__ WaveParams sp;
   __shared__ int s_skip;
   uint32_t *slots_all = reinterpret_cast<uint32_t *>(smem_raw + b.prof_area);
-  uint32_t *save_all = slots_all + b.slot_words;
+  uint32_t *save_all = slots_all + blockDim.x;
   const uint32_t start = (uint32_t)(((uint64_t)blockIdx.x * b.ntiles) / gridDim.x);
   for (uint32_t it = 0; it < b.ntiles; ++it) {
     uint32_t tile = start + it;
