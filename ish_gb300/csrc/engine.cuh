@@ -68,14 +68,12 @@ struct WaveParams {
   uint32_t lane_mul;       // 65536: b * lane_mul + a packs two PROF_S32 words
   int open, ext, ends;
   int neg_limit;           // v_neg_limit of the reference (semi_global_aln/striped.mojo:329-334)
-  int bias;                // semi-global: added to every H, E and F (see wave_params)
+  int bias;                // added to every H, E and F (see wave_params)
   int frame_mask;          // semi-global: R - 1, rows between frame resets (R * ext <= 2048)
   // packed 16-bit pairs of values used every row, precomputed on the host so
   // that the kernel reads them as operands instead of deriving them
-  uint32_t pk_nopen;       // (-open, -open)
   uint32_t pk_next;        // (-ext, -ext)
   uint32_t pk_eopen;       // (ext - open, ext - open): a gap opening in the frames
-  uint32_t pk_fsin;        // (open, open): local alignment, F + open entering the padding
   uint32_t pk_left;        // semi-global: H entering the padding from the left at frame 0
   uint32_t pk_left_ext;    // ... and its rise per row (0 with a fixed target start)
   uint32_t pk_drop;        // -(R * ext) in both halves as one 32-bit integer: a frame reset

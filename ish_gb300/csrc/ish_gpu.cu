@@ -722,12 +722,11 @@ void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDe
   // low + ext * (G * K + 3) <= 30000; the sum stays below 65,536.
   const bool ts = q.ends & ISH_FREE_TARGET_START;
   const int low = ts ? 2 * q.open : 3 * q.open + q.ext * (int)std::min<uint64_t>(rs.max_len, 32768);
-  p.bias = sg ? low + 8 * q.ext + 256 : 0;
+  // (local alignment: H >= 0, E, F and openings >= -open, H <= 30000)
+  p.bias = sg ? low + 8 * q.ext + 256 : q.open + 256;
   p.frame_mask = sg ? frame_rows(q.ext) - 1 : 0x3fffffff;
-  p.pk_nopen = dup16_host(-q.open);
   p.pk_next = dup16_host(-q.ext);
   p.pk_eopen = dup16_host(q.ext - q.open);
-  p.pk_fsin = sg ? 0u : dup16_host(q.open);
   p.pk_left = sg ? (ts ? (uint32_t)p.bias : (uint32_t)q.open) * 0x10001u : 0u;
   p.pk_left_ext = sg && ts ? (uint32_t)q.ext * 0x10001u : 0u;
   p.pk_drop = sg ? (uint32_t)(-(p.frame_mask + 1) * q.ext) * 0x10001u : 0u;

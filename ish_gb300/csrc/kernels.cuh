@@ -57,14 +57,14 @@ __global__ void k_gather_hits(const uint32_t *idx, const uint32_t *count, const 
 // multiple of the rows per step (the rows past both records' ends feed nothing).
 // Semi-global row frames reset only at step boundaries, so the fast regime
 // keeps R >= WAVE_RPS_SG rows per frame period (gap_extend <= 512 at 4).
-// Chosen per mode from measurements (protein, K = 38): semi-global 4, local 2
-// (local alignment's per-row maximum and dominance state make four rows per
-// step cost more registers than they save).
+// Four for local alignment too: its carried dominance bar is one word per step,
+// so four rows cost no more registers than two (protein, 8 threads x 38
+// columns: 5,573 GCUPS against 5,302 with two).
 #ifndef WAVE_RPS_SG
 #define WAVE_RPS_SG 4
 #endif
 #ifndef WAVE_RPS_SW
-#define WAVE_RPS_SW 2
+#define WAVE_RPS_SW 4
 #endif
 
 // Wavefront kernels are instantiated for K = 2, 4, ..., WAVE_KMAX columns per

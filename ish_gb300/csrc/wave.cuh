@@ -13,29 +13,32 @@
 // lanes" for short queries; G = 32 is a warp-wide anti-diagonal wavefront for
 // long queries.
 //
-// Local alignment: five DPX instructions per cell and record pair (two cells),
-// in two in-place passes over the thread's columns:
-//   backward:  T = max(Hdiag + P, E);  u = T - open;  E = max(E - ext, u);  H := T
-//   forward:   H = max(Fs - open, T);  Fs = max(Fs - ext, T)
-// with Fs = F + open carried along the row, and u floored at 0, which keeps E,
-// T and H non-negative.  E opens from T only, never from F: an F-then-E gap
-// pair always has an E-then-F twin of at least the same score, which this
-// recurrence keeps, so H is exactly the Gotoh H.
+// The packed values are unsigned 16-bit, raised by a bias, and a row is one
+// pass over the thread's columns that updates H and E in place.  E and F open
+// from H.  The DPX add-max and three-input maximum share one pipe (16 lanes per
+// clock and sub-partition), which bounds the row, so whatever can be a plain
+// 32-bit add of both halves -- the bias keeps the low half from borrowing from
+// the high one -- runs beside it on the integer multiply-add pipe.
 //
-// Semi-global: three DPX instructions and a 32-bit add (two with the 32-bit
-// profile, whose pair word is assembled by the first):
-//   backward:  H[j] := H[j-1] + P[j]                (integer multiply-add pipe)
-//   forward:   H = max3(H, E, F);  E = max(H + c, E);  F = max(H + c, F)
-// The values are unsigned 16-bit, held raised by a bias and by frames that rise
-// by ext per row and per column: a gap extension then costs nothing, so both
-// gap updates are one add-max with the same c = ext - open, and the profile
-// carries +2 ext for the diagonal step.  Rows drop back to frame 0 every R rows
-// (R * ext <= 2048); the column frame runs over the whole padded query.  The
-// bias keeps every value of the low half non-negative, so that the sum
-// H + P, with P the pair's scores as ONE signed integer b * 65536 + a, never
-// borrows from the high half: the add can leave the DPX pipe (16 lanes per
-// clock and sub-partition), which bounds the row.  wave_params() in ish_gpu.cu
-// derives the bias and shows that every value fits 16 bits.
+// Local alignment, four DPX instructions and two adds per cell and record pair
+// (two cells), the first of which assembles the pair's profile word P:
+//   T = max(Hdiag + P, floor);  H = max3(T, E, F);  u = H - open
+//   E = max(E - ext, u);  F = max(F - ext, u)
+// with the floor at score 0 and half a three-input maximum per column for the
+// row's best.  (The five-instruction form that floors H - open instead, and one
+// in which max3(Hdiag + P, E, floor) leaves the F chain one instruction long,
+// measured 5 % and 3 % slower at 38 columns.)
+//
+// Semi-global, three DPX instructions and an add (two with the 32-bit profile):
+//   T = Hdiag + P;  H = max3(T, E, F);  E = max(H + c, E);  F = max(H + c, F)
+// The values are also raised by frames that rise by ext per row and per column:
+// a gap extension then costs nothing, so both gap updates are one add-max with
+// the same c = ext - open, and the profile carries +2 ext for the diagonal
+// step.  Rows drop back to frame 0 every R rows
+// (R * ext <= 2048); the column frame runs over the whole padded query.  P is
+// the pair's scores as ONE signed integer b * 65536 + a.  wave_params() in
+// ish_gpu.cu derives the bias and shows that every value fits 16 bits.
+// (Local alignment cannot use frames: its floor would move with them.)
 // Measured on GB300 (row loops alone, 38 columns per thread): 9.3 clocks per
 // column and warp with the 32-bit profile, where the shared-memory loads bound
 // it (8.4), 8.0 with the pair profile, against 11.8 for four DPX per cell pair.
@@ -81,7 +84,8 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   uint16_t *saveB = saveA + KP8;
 
   const unsigned FULL = 0xffffffffu;
-  const uint32_t NOPEN = p.pk_nopen;
+  // local: score 0, and -open in both halves as one integer
+  const uint32_t FLOOR = (uint32_t)p.bias * 0x10001u, NOPEN_SUM = (uint32_t)(-p.open) * 0x10001u;
   const uint32_t NEXT = p.pk_next;
   // semi-global: a gap opens from H at ext - open in the frames
   const uint32_t EOPEN = p.pk_eopen;
@@ -115,12 +119,12 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
     E[j] = 0;
   }
   uint32_t prevH = 0;  // H(row above the step's first row, column col0 - 1)
-  // per row of the step, passed to thread t+1: H of the last column, F + open
-  // leaving it, and (local alignment) the running best of this thread's and
-  // all earlier columns
-  uint32_t outH[RPS], outF[RPS], outB[RPS];
+  // passed to thread t+1: per row of the step, H of the last column and F
+  // leaving it; local alignment: the best of this thread's and all earlier
+  // columns up to the step's last row, which the next thread uses a step later
+  uint32_t outH[RPS], outF[RPS], outB = 0, left_best = 0;
 #pragma unroll
-  for (int k = 0; k < RPS; ++k) outH[k] = outF[k] = outB[k] = 0;
+  for (int k = 0; k < RPS; ++k) outH[k] = outF[k] = 0;
   uint32_t outC = CTL_IDLE;
   int q4 = 0, lenA = 0, lenB = 0;  // q4: row of the step's first row
   // the next q4 at which this thread has anything beside its rows to do, and
@@ -135,7 +139,12 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // thread's cells
   uint32_t best = 0;
   int rowA = -1, rowB = -1;  // first row of the lane's maximum
-  uint32_t oR0 = 0, oR1 = 0, oR2 = 0, oR3 = 0;  // last-row partials for thread t+1
+  // last-row partials for thread t+1: semi-global in registers, local alignment
+  // in the padding behind the thread's saved row: scores and columns of A and B
+  // (16 bits each), then their rows
+  uint32_t oR0 = 0, oR1 = 0;
+  constexpr int save_stride = wave_save_words(K) / 4;
+  uint4 *partial = reinterpret_cast<uint4 *>(save_all + tid * wave_save_words(K) + KP8);
   bool ended = false;  // a record of the warp ended in the last step
   const bool remap = remap_off != 0;
   // whether the ends of records matter to this thread: with the query end
@@ -151,45 +160,63 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   uint32_t step = 0;
 
   // One row of the pair with record codes cA, cB: `diag` is H of the row above
-  // at column col0 - 1, `fs` is F (local alignment: F + open) entering column
-  // col0.  Updates H and E in place and returns F leaving the last column.
+  // at column col0 - 1, `fs` is F entering column col0.  Updates H and E in
+  // place, column by column from the left (each profile word is used as it
+  // arrives, which keeps few of them in registers), and returns F leaving the
+  // last column.
   auto row_step = [&](uint32_t cA, uint32_t cB, uint32_t diag, uint32_t fs) -> uint32_t {
     if (remap) {  // codes that score alike share a profile row
       cA = prof[remap_off + cA];
       cB = prof[remap_off + cB];
     }
-    uint32_t P[K];
-    // semi-global: the profile word of column j plus H of the row above at
-    // column j - 1 (H still holds that row); local alignment adds it later
-    auto with_diag = [&](uint32_t w, int j) -> uint32_t {
-      if (MODE != SG) return w;
-      return w + (j == 0 ? diag : H[j > 0 ? j - 1 : 0]);
+    // one column: `dp` is the pair's scores, semi-global (but for PROF_S16)
+    // with H of the row above one column to the left added
+    auto cell = [&](int j, uint32_t dp) {
+      uint32_t &h = H[j], &e = E[j];
+      if (MODE == SG && LAYOUT != PROF_S16) {
+        diag = h;
+        h = __vimax3_u16x2(dp, e, fs);
+        e = __viaddmax_u16x2(h, EOPEN, e);
+        fs = __viaddmax_u16x2(h, EOPEN, fs);
+      } else if (MODE == SG) {
+        const uint32_t T = __viaddmax_u16x2(diag, dp, e);
+        diag = h;
+        h = __vmaxu2(T, fs);
+        e = __viaddmax_u16x2(T, EOPEN, e);
+        fs = __viaddmax_u16x2(T, EOPEN, fs);
+      } else {
+        const uint32_t T = __viaddmax_u16x2(diag, dp, FLOOR);
+        diag = h;
+        h = __vimax3_u16x2(T, e, fs);
+        const uint32_t u = h + NOPEN_SUM;
+        e = __viaddmax_u16x2(e, NEXT, u);
+        fs = __viaddmax_u16x2(fs, NEXT, u);
+      }
     };
     if (LAYOUT == PROF_PAIR) {
       const uint4 *r4 = reinterpret_cast<const uint4 *>(prof_t + (cA * alpha + cB) * row_bytes);
 #pragma unroll
       for (int v = 0; v < (K + 3) / 4; ++v) {
         const uint4 w = r4[v];
-        if (4 * v + 0 < K) P[4 * v + 0] = with_diag(w.x, 4 * v + 0);
-        if (4 * v + 1 < K) P[4 * v + 1] = with_diag(w.y, 4 * v + 1);
-        if (4 * v + 2 < K) P[4 * v + 2] = with_diag(w.z, 4 * v + 2);
-        if (4 * v + 3 < K) P[4 * v + 3] = with_diag(w.w, 4 * v + 3);
+        const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (4 * v + m < K) cell(4 * v + m, MODE == SG ? ww[m] + diag : ww[m]);
       }
     } else if (LAYOUT == PROF_S32) {
-      // 32-bit words holding the 16-bit score in the low half; the packed
-      // pair is b * 65536 + a, one integer multiply-add (the multiplier is a
-      // runtime value, so this stays an IMAD on the FMA pipe, which the DPX
-      // recurrence on the ALU pipe leaves idle)
+      // a 32-bit word per code; the packed pair is b * 65536 + a, one integer
+      // multiply-add (the multiplier is a runtime value, so this stays an IMAD
+      // on the FMA pipe, which the DPX recurrence on the ALU pipe leaves idle)
       const uint4 *ra = reinterpret_cast<const uint4 *>(prof_t + cA * row_bytes);
       const uint4 *rb = reinterpret_cast<const uint4 *>(prof_t + cB * row_bytes);
       const uint32_t mul = lane_mul;
 #pragma unroll
       for (int v = 0; v < (K + 3) / 4; ++v) {
         const uint4 a = ra[v], b = rb[v];
-        if (4 * v + 0 < K) P[4 * v + 0] = b.x * mul + with_diag(a.x, 4 * v + 0);
-        if (4 * v + 1 < K) P[4 * v + 1] = b.y * mul + with_diag(a.y, 4 * v + 1);
-        if (4 * v + 2 < K) P[4 * v + 2] = b.z * mul + with_diag(a.z, 4 * v + 2);
-        if (4 * v + 3 < K) P[4 * v + 3] = b.w * mul + with_diag(a.w, 4 * v + 3);
+        const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int m = 0; m < 4; ++m)
+          if (4 * v + m < K) cell(4 * v + m, MODE == SG ? aw[m] + (bw[m] * mul + diag) : bw[m] * mul + aw[m]);
       }
     } else {
       // 16-bit words (profiles too large for the 32-bit layout): one PRMT
@@ -202,68 +229,32 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-          if (8 * v + 2 * m < K) P[8 * v + 2 * m] = __byte_perm(aw[m], bw[m], 0x5410);
-          if (8 * v + 2 * m + 1 < K) P[8 * v + 2 * m + 1] = __byte_perm(aw[m], bw[m], 0x7632);
+          if (8 * v + 2 * m < K) cell(8 * v + 2 * m, __byte_perm(aw[m], bw[m], 0x5410));
+          if (8 * v + 2 * m + 1 < K) cell(8 * v + 2 * m + 1, __byte_perm(aw[m], bw[m], 0x7632));
         }
-      }
-    }
-    if (MODE == SG && LAYOUT != PROF_S16) {
-      // the profile words hold H + P already (above)
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const uint32_t h = __vimax3_u16x2(P[j], E[j], fs);
-        E[j] = __viaddmax_u16x2(h, EOPEN, E[j]);
-        fs = __viaddmax_u16x2(h, EOPEN, fs);
-        H[j] = h;
-      }
-    } else if (MODE == SG) {
-#pragma unroll
-      for (int j = K - 1; j >= 0; --j) H[j] = __viaddmax_u16x2(j == 0 ? diag : H[j - 1], P[j], E[j]);
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const uint32_t T = H[j];
-        H[j] = __vmaxu2(T, fs);
-        E[j] = __viaddmax_u16x2(T, EOPEN, E[j]);
-        fs = __viaddmax_u16x2(T, EOPEN, fs);
-      }
-    } else {
-      // backward pass (columns independent), then the F chain
-#pragma unroll
-      for (int j = K - 1; j >= 0; --j) {
-        const uint32_t T = __viaddmax_s16x2(j == 0 ? diag : H[j - 1], P[j], E[j]);
-        const uint32_t u = __viaddmax_s16x2(T, NOPEN, 0u);
-        E[j] = __viaddmax_s16x2(E[j], NEXT, u);
-        H[j] = T;
-      }
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const uint32_t T = H[j];
-        H[j] = __viaddmax_s16x2(fs, NOPEN, T);
-        fs = __viaddmax_s16x2(fs, NEXT, T);
       }
     }
     return fs;
   };
 
   // Local alignment, after row `row` (`live`: the halves of the lanes whose
-  // record holds that row): only a row maximum above every cell so
-  // far in this thread AND in all columns to its left (`left`, their running
-  // best up to this row, passed along the pipeline) can be the first row of
-  // the record's maximum at its smallest column; anything else is dominated
-  // (smaller, or equal in an earlier row or a smaller column), so only those
-  // improvements are recorded.  Returns the running best passed on.
-  auto sw_track = [&](int row, uint32_t left, uint32_t live) -> uint32_t {
+  // record holds that row): a row maximum that does not beat every cell so far
+  // in this thread AND in the columns to its left can never be the first row of
+  // the record's maximum at its smallest column (it is smaller, or equal in a
+  // later row or a larger column), so only the others are recorded.  `thr` is
+  // that bar: this thread's rows up to the last, the left columns' rows up to
+  // the last step (a later row of theirs may tie without winning).
+  auto sw_track = [&](int row, uint32_t &thr, uint32_t live) {
     uint32_t cm = H[0];
 #pragma unroll
-    for (int j = 1; j + 1 < K; j += 2) cm = __vimax3_s16x2(cm, H[j], H[j + 1]);
-    if ((K & 1) == 0 && K > 1) cm = __viaddmax_s16x2(cm, 0u, H[K - 1]);
+    for (int j = 1; j + 1 < K; j += 2) cm = __vimax3_u16x2(cm, H[j], H[j + 1]);
+    if ((K & 1) == 0 && K > 1) cm = __vmaxu2(cm, H[K - 1]);
     cm &= live;
-    const uint32_t thr = __viaddmax_s16x2(best, 0u, left);
-    const uint32_t nb = __viaddmax_s16x2(thr, 0u, cm);
+    const uint32_t nb = __vmaxu2(thr, cm);
     if (nb != thr) {
       // keep this row (shared-memory stores only); the column of the maximum
       // is looked up once, at the record's last row
-      const bool upA = lo16(cm) > lo16(thr), upB = hi16(cm) > hi16(thr);
+      const bool upA = ulo16(cm) > ulo16(thr), upB = uhi16(cm) > uhi16(thr);
       // the improving lane's halves of the row: one PRMT per two columns
 #define ISH_H(j) ((j) < K ? H[(j) < K ? (j) : 0] : 0u)
       if (upA) {
@@ -288,8 +279,8 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       if (upA) rowA = row;
       if (upB) rowB = row;
       best = ((upA ? cm : best) & 0xffffu) | ((upB ? cm : best) & 0xffff0000u);
+      thr = nb;
     }
-    return nb;
   };
 
   // Semi-global, target end free, one row: the running max of column Q-1
@@ -391,7 +382,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       rA = rB = -1;
       qA = qB = 0x7fff;
     }
-    const int mA = lo16(best), mB = hi16(best);
+    const int mA = ulo16(best) - p.bias, mB = uhi16(best) - p.bias;
     const bool ownA = lastA && (mA > bA || (mA == bA && mA > 0 && rowA < rA));
     const bool ownB = lastB && (mB > bB || (mB == bB && mB > 0 && rowB < rB));
     if (ownA) {
@@ -403,21 +394,30 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       rB = rowB;
     }
     if (ownA || ownB) {  // smallest column of this thread's maximum in its first row
+      const int sA = bA + p.bias, sB = bB + p.bias;
       const uint32_t *wa = reinterpret_cast<const uint32_t *>(saveA), *wb = reinterpret_cast<const uint32_t *>(saveB);
 #pragma unroll 1
       for (int v = (K + 1) / 2 - 1; v >= 0; --v) {
         const uint32_t a = wa[v], b = wb[v];
-        if (ownA && 2 * v + 1 < K && hi16(a) == bA) qA = col0 + 2 * v + 1;
-        if (ownA && lo16(a) == bA) qA = col0 + 2 * v;
-        if (ownB && 2 * v + 1 < K && hi16(b) == bB) qB = col0 + 2 * v + 1;
-        if (ownB && lo16(b) == bB) qB = col0 + 2 * v;
+        if (ownA && 2 * v + 1 < K && uhi16(a) == sA) qA = col0 + 2 * v + 1;
+        if (ownA && ulo16(a) == sA) qA = col0 + 2 * v;
+        if (ownB && 2 * v + 1 < K && uhi16(b) == sB) qB = col0 + 2 * v + 1;
+        if (ownB && ulo16(b) == sB) qB = col0 + 2 * v;
       }
     }
     if (t < G - 1) {
-      put_lanes(oR0, (uint32_t)(bA & 0xffff) | ((uint32_t)bB << 16), lastA, lastB);
-      put_lanes(oR1, (uint32_t)(qA & 0xffff) | ((uint32_t)qB << 16), lastA, lastB);
-      if (lastA) oR2 = (uint32_t)rA;
-      if (lastB) oR3 = (uint32_t)rB;
+      uint16_t *h = reinterpret_cast<uint16_t *>(partial);
+      int *r = reinterpret_cast<int *>(partial);
+      if (lastA) {
+        h[0] = (uint16_t)bA;
+        h[2] = (uint16_t)qA;
+        r[2] = rA;
+      }
+      if (lastB) {
+        h[1] = (uint16_t)bB;
+        h[3] = (uint16_t)qB;
+        r[3] = rB;
+      }
       return;
     }
     const uint32_t pr = slots[(ctl >> CTL_SEQ_SHIFT) & (G - 1)];
@@ -430,24 +430,31 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // final, and a new pair resets all of its state.
   while (true) {
     __syncwarp();
-    uint32_t msgH[RPS], msgF[RPS], msgB[RPS];
+    uint32_t msgH[RPS], msgF[RPS], msgB = 0;
 #pragma unroll
     for (int k = 0; k < RPS; ++k) {
       msgH[k] = __shfl_up_sync(FULL, outH[k], 1, G);
       msgF[k] = __shfl_up_sync(FULL, outF[k], 1, G);
-      msgB[k] = (MODE == SW) ? __shfl_up_sync(FULL, outB[k], 1, G) : 0u;
     }
+    if (MODE == SW) msgB = __shfl_up_sync(FULL, outB, 1, G);
     uint32_t msgC = __shfl_up_sync(FULL, outC, 1, G);
     if (t0) msgC &= ~CTL_NEW;  // its own last control word
     // partial results of records that ended in thread t-1's previous step
     uint32_t iR0 = 0, iR1 = 0, iR2 = 0, iR3 = 0;
-    if ((MODE == SW || qe) && ended) {
+    if (MODE == SW) {
+      if (ended) {
+        if (t > 0) {
+          const uint4 v = *(partial - save_stride);
+          iR0 = v.x;
+          iR1 = v.y;
+          iR2 = v.z;
+          iR3 = v.w;
+        }
+        __syncwarp();  // read before this step's ends rewrite them
+      }
+    } else if (qe && ended) {
       iR0 = __shfl_up_sync(FULL, oR0, 1, G);
       iR1 = __shfl_up_sync(FULL, oR1, 1, G);
-      if (MODE == SW) {
-        iR2 = __shfl_up_sync(FULL, oR2, 1, G);
-        iR3 = __shfl_up_sync(FULL, oR3, 1, G);
-      }
     }
     q4 += RPS;
     // Everything beside the rows -- new pairs, frame resets, the look-ahead,
@@ -494,14 +501,15 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         for (int j = 0; j < K; ++j) {
           const int c = t * K + j;
           const uint32_t h0 = (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
-          H[j] = (MODE == SW) ? 0u : h0;
-          E[j] = (MODE == SW) ? 0u : h0 + EOPEN_SUM;  // row 0's frame is one ext above row -1's
+          H[j] = (MODE == SW) ? FLOOR : h0;
+          E[j] = (MODE == SW) ? FLOOR : h0 + EOPEN_SUM;  // row 0's frame is one ext above row -1's
         }
         {
           const int c = t * K - 1;
-          prevH = (MODE == SW) ? 0u : (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
+          prevH = (MODE == SW) ? FLOOR : (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
         }
-        best = (MODE == SG && t != G - 1) ? 0xffffffffu : 0u;
+        best = (MODE == SW) ? FLOOR : (t != G - 1 ? 0xffffffffu : 0u);
+        left_best = FLOOR;
         rowA = rowB = -1;
       } else {
         if (MODE == SG && (q4 & fmask) == 0) {
@@ -574,17 +582,17 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       wA >>= 16;
       wB >>= 16;
     }
-    // thread 0: what enters the padding from the left, H at its boundary and
-    // F below every value (semi-global: 0; local: F + open = open)
+    // thread 0: what enters the padding from the left, H at its boundary (local:
+    // the floor) and F below every value
     if (t0) {
-      const uint32_t hf = LEFT0 + (MODE == SG ? (uint32_t)(q4 & fmask) * LEFT_EXT : 0u);
-      if (MODE == SG) prevH = hf - LEFT_EXT;
+      const uint32_t hf = MODE == SG ? LEFT0 + (uint32_t)(q4 & fmask) * LEFT_EXT : FLOOR;
+      prevH = MODE == SG ? hf - LEFT_EXT : hf;
 #pragma unroll
       for (int k = 0; k < RPS; ++k) {
-        msgH[k] = hf + (uint32_t)k * LEFT_EXT;
-        msgF[k] = (MODE == SG) ? 0u : p.pk_fsin;
-        msgB[k] = 0u;
+        msgH[k] = MODE == SG ? hf + (uint32_t)k * LEFT_EXT : hf;
+        msgF[k] = MODE == SG ? 0u : FLOOR + NOPEN_SUM;
       }
+      msgB = FLOOR;
     }
     if (MODE == SG && qe && ends) {
       // ---- free query end, a record of the warp ends: one row at a time, with
@@ -612,6 +620,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       prevH = d;
     } else {
       // ---- the step's rows ----
+      uint32_t thr = __vmaxu2(best, left_best);  // (local alignment)
 #pragma unroll
       for (int k = 0; k < RPS; ++k) {
         const uint32_t fs = row_step(__byte_perm(wA, 0u, 0x4440 + k), __byte_perm(wB, 0u, 0x4440 + k),
@@ -620,12 +629,14 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         outF[k] = fs;
         if (MODE == SW) {
           uint32_t live = 0xffffffffu;  // a record that ended in this step has no further rows
-          if (k > 0 && ends) live = (q4 + k == lenA ? 0u : 0xffffu) | (q4 + k == lenB ? 0u : 0xffff0000u);
-          outB[k] = sw_track(q4 + k, msgB[k], live);
+          if (k > 0 && ends) live = (q4 + k >= lenA ? 0u : 0xffffu) | (q4 + k >= lenB ? 0u : 0xffff0000u);
+          sw_track(q4 + k, thr, live);
         }
       }
       prevH = msgH[RPS - 1];
       if (MODE == SW) {
+        outB = __vmaxu2(best, msgB);
+        left_best = msgB;
         if (endA || endB) sw_event(msgC, iR0, iR1, iR2, iR3);
       } else if (!ends) {
         if (te) {
