@@ -77,7 +77,8 @@ struct WaveParams {
   uint32_t pk_left;        // semi-global: H entering the padding from the left at frame 0
   uint32_t pk_left_ext;    // ... and its rise per row (0 with a fixed target start)
   uint32_t pk_drop;        // -(R * ext) in both halves as one 32-bit integer: a frame reset
-  uint32_t row_bytes;      // profile bytes between consecutive codes' rows ((G * kp) words)
+  int slots;               // thread slices per profile row: G, or 8 for narrower groups (profile_slots)
+  uint32_t row_bytes;      // profile bytes between consecutive codes' rows ((slots * kp) words)
   uint32_t first, count;   // sorted entries [first, first + count) are scored
   uint32_t pair_stride, pair_phase;  // of those, record pairs phase, phase + stride, ... (stride 0: every pair)
   uint32_t *counter;       // work counter (record pairs), zeroed before launch

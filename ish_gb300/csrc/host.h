@@ -52,6 +52,7 @@ struct DevBuf {
 
 struct WaveLayout {
   int G = 0, K = 0, d = 0, kp = 0, layout = 0;
+  int slots = 0;            // thread slices per profile row (profile_slots)
   uint32_t prof_bytes = 0;  // profile rows, then (if remapped) the 256-byte code -> row table
   uint32_t remap_off = 0;   // byte offset of that table, 0: codes are rows
   DevBuf prof;
@@ -272,8 +273,7 @@ struct LoadTimer {
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 int frame_rows(int ext);
-int wave_lean(const ish_ctx *ctx, int K, int mode, int G);
-int batch_lean(const ish_ctx *ctx, int K, int mode, int G);
+int wave_lean(const ish_ctx *ctx, int K, int mode);
 uint64_t window_overlap(const Query &q);
 int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, OutDev out, cudaStream_t s, bool *done);
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode);
@@ -291,9 +291,10 @@ void recycle_set(ish_ctx *ctx, RecordSet &rs);
 void take_spare_set(ish_ctx *ctx, RecordSet &rs, size_t codes_bytes);
 int wave_k_available(int k);
 // Shape of the wavefront kernel for a query: the autotuner's choice when one
-// exists, else the cost model; forced options override both.
-void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout);
-void choose_shape(int Q, int force_G, int force_K, int *G, int *K);
+// exists, else the cost model, for the records of `set` if one is given
+// (scored by `share` queries at once); forced options override both.
+void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const RecordSet *set = nullptr,
+                double share = 1);
 uint64_t tune_key(int mode, int alphabet, int Q);
 int layout_stride(int layout, int K);
 size_t layout_bytes(int layout, int alphabet, int G, int K);
@@ -321,10 +322,8 @@ int device_encoding(ish_ctx *ctx, int kind, const uint8_t **out);
 void encoding_table(int kind, uint8_t t[256]);
 uint32_t count_longer(const RecordSet &rs, uint64_t len);
 // Checks that query q may run on the wavefront kernels against set rs with
-// shape (G, K): 0 or a status with the reason in msg.  check_fast picks the
-// shape and records the reason as the context's error.
+// shape (G, K): 0 or a status with the reason in msg.
 int fast_check(const Query &q, const RecordSet &rs, int G, int K, char *msg, size_t len);
-int check_fast(ish_ctx *ctx, const Query &q, const RecordSet &rs);
 // Fills the per-query part of the wavefront parameters (not first/count/counter).
 void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDev out, int *error, WaveParams *p);
 int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uint32_t count, OutDev out, int G, int K,

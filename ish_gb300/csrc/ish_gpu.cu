@@ -127,51 +127,23 @@ int matrix_alphabet_ok(uint32_t alphabet) { return alphabet >= 1 && alphabet <= 
 // gap_open > gap_extend and no lane value of the reference can saturate or
 // wrap.  Bounds are conservative.
 
+// Whether (K, mode) runs the lean kernel variant, as measured on GB300 (300,000
+// proteins, G = 8, Q = 8K - 2; see the kernels' launch bounds in kernels.cuh).
+// Semi-global rows need so few registers that the builds with more warps are
+// ahead or level everywhere: 256 x 2 against 128 x 3 within 1 % at K = 25..32
+// (nucleotide pairs up to 3 % ahead), 128 x 3 against 128 x 2 by 2-8 % at K =
+// 34..48.  Local alignment keeps a row maximum and more state: 128 x 3 is ahead
+// of 256 x 2 by 1-5 % at K = 27..32, and from K = 42 on 128 x 3 spills and 128 x
+// 2 is ahead by 13-47 %.
+int wave_lean(const ish_ctx *ctx, int K, int mode) {
+  if (!wave_has_lean(K)) return 0;
+  if (ctx->force_lean >= 0) return ctx->force_lean;
+  return mode == SW && ((K >= 27 && K <= 32) || K >= 42);
+}
+
 // Semi-global rows are held in frames that rise by ext per row and drop back
 // to 0 every R rows, R a power of two with R * ext <= 2048 (the headroom the
 // regime keeps above the largest score).
-// Whether (K, mode) runs the lean kernel variant (128 x 2 blocks with more
-// registers instead of 128 x 3, whose parameters come from shared memory),
-// as measured on GB300 for the protein search (blosum62, 400k records,
-// G = 8, Q = 8K - 2): lean is ahead for semi-global at K = 34..40 (+0.5 to
-// +5.7 %) and local at 34..38 (+1.3 to +2.4 %), behind from there on (up to
-// -15 %).
-int wave_lean(const ish_ctx *ctx, int K, int mode, int G) {
-  if (!wave_has_lean(K)) return 0;
-  if (ctx->force_lean >= 0) return ctx->force_lean;
-  // Measured per K (protein records, Q = G * K - 2).  G <= 8 (200k records):
-  // the 128 x 3 build beats 256 x 2 from K = 27 (semi-global) / 30 (local)
-  // on, by up to 16 %; from K = 34 the 128 x 3 default build beats the 128 x
-  // 2 lean one by 3-19 % up to K = 44, and loses at 46-48.  Wider groups
-  // (300k records): at G = 32 the 256 x 2 build wins up to K = 30 (by 7-20 %)
-  // and ties at K = 32; at G = 16 the lean build wins from K = 44
-  // (semi-global, +7 %) / 40 (local, +15 %; 2.6x at K = 48).
-  if (G <= 8) {
-    if (K <= 32) return mode == SW ? K >= 30 : K >= 27;
-    return K >= 46;
-  }
-  if (K <= 32) return mode == SG && K == 32 && G >= 32;
-  return mode == SW ? K >= 40 : K >= 44;
-}
-
-// The same choice for the batched kernel (parameters in shared memory, one
-// more live pointer), measured the same way through ish_gpu_score_multi.
-// G <= 8: the 128 x 3 build wins everywhere but local alignment at K = 36
-// (+2.0 %) and K = 48 (+6.7 %); the lean build loses 12-17 % from K = 38 on.
-// Wider groups: at G = 32 the lean build wins semi-global K = 32 (+10 %),
-// the default one K = 26-30; at G = 16 the lean build wins from K = 44
-// (semi-global) / 36 (local, 2.9x at K = 48).  G is the class's narrowest.
-int batch_lean(const ish_ctx *ctx, int K, int mode, int G) {
-  if (!wave_has_lean(K)) return 0;
-  if (ctx->force_lean >= 0) return ctx->force_lean;
-  if (G <= 8) {
-    if (K <= 32) return 0;
-    return mode == SW && (K == 36 || K == 48);
-  }
-  if (K <= 32) return mode == SG && K == 32 && G >= 32;
-  return mode == SW ? K >= 36 : K >= 44;
-}
-
 int frame_rows(int ext) {
   int R = 1;
   while (R < (1 << 20) && (long)2 * R * std::max(ext, 1) <= 2048) R *= 2;
@@ -210,25 +182,50 @@ int neg_limit_of(int open, int mmin) {
   return (int16_t)(-32768 - mmin + 1);
 }
 
-// Columns per thread (K) and threads per group (G) for a query length: the
-// smallest modelled cost with G*K >= Q + 1.  Per thread-row the kernel spends
-// about five DPX instructions per column plus ~50 instructions of fixed work
-// (pipeline, codes, tracking), i.e. ROW_OVERHEAD column-equivalents; K <= 48
-// keeps 12-16 warps per SM, wider rows run at 8 (charged 25% more).  Kernels
-// exist for every K <= 32 and even K up to 64.
+// Scheduler clocks of one warp-row (one row of 32 / G record pairs) with the
+// warps of a full SM taking turns, and of one row of a warp that has its
+// scheduler to itself (the chain of its columns, shuffles and loads).  Straight
+// lines through measurements at G = 8, proteins, K = 4..64 (semi-global 87 at K =
+// 4, 180 at 16, 326 at 32, 384 at 38, 631 at 60; local 184, 258, 468, 561, 941;
+// alone 451 / 752 at K = 32, 619 / 1,074 at 48), with what the builds with fewer
+// warps add.
+static double warp_row_clocks(int mode, int K) {
+  if (mode == SG) return (50 + 8.6 * K) * (K > 48 ? 1.1 : 1.0);
+  return (50 + 13.3 * K) * (K > 40 ? 1.08 : 1.0);
+}
+static double lone_row_clocks(int mode, int K) { return mode == SG ? 150 + 9.5 * K : 200 + 17.5 * K; }
+
+// Modelled time of one query against `set` (null: many records of any length)
+// with G threads x K columns: every warp's share of the rows at the rate of the
+// warps in flight, or the longest pair alone, whichever takes longer.  `share`
+// queries run at once.
+static double shape_clocks(const ish_ctx *ctx, int mode, int G, int K, const RecordSet *set, double share) {
+  const double row = warp_row_clocks(mode, K);
+  if (!set) return G * row;
+  const double schedulers = 4.0 * ctx->num_sms;
+  const double pairs = std::max(1.0, (set->n - set->n_empty) / 2.0) * share, rows = set->total / 2.0 * share;
+  const double full = schedulers * (K <= 32 ? 4 : K <= 48 ? 3 : 2);
+  const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), full));
+  const double per_row = std::max(lone_row_clocks(mode, K), std::max(1.0, warps / schedulers) * row);
+  const double all = rows * G / 32 / warps * per_row;
+  const double last = ((double)set->max_len + 4 * G) * std::max(lone_row_clocks(mode, K), row);
+  return std::max(all, last) + 0.1 * all;
+}
+
+// Columns per thread (K) and threads per group (G) with the smallest modelled
+// time among those with G*K >= Q + 1.  Kernels exist for every K <= 32 and even
+// K up to 64.
 int wave_k_available(int k) { return (k >= 1 && k <= 32) || (k > 32 && k <= WAVE_KMAX && !(k & 1)); }
 
-void choose_shape(int Q, int force_G, int force_K, int *G, int *K) {
-  const double ROW_OVERHEAD = 8.0;
+static void choose_shape(const ish_ctx *ctx, int mode, int Q, const RecordSet *set, double share, int *G, int *K) {
   double bestc = 1e30;
   int bg = 0, bk = 0;
   for (int g = 1; g <= 32; g <<= 1) {
-    if (force_G && g != force_G) continue;
-    int k = force_K ? force_K : (Q + 1 + g - 1) / g;
-    if (!force_K && k > 32) k = (k + 1) & ~1;
+    if (ctx->force_G && g != ctx->force_G) continue;
+    int k = ctx->force_K ? ctx->force_K : (Q + 1 + g - 1) / g;
+    if (!ctx->force_K && k > 32) k = (k + 1) & ~1;
     if (!wave_k_available(k) || g * k < Q + 1) continue;
-    double c = (double)g * k * (1.0 + ROW_OVERHEAD / k);
-    if (k > 48) c *= 1.25;
+    const double c = shape_clocks(ctx, mode, g, k, set, share);
     if (c < bestc) {
       bestc = c;
       bg = g;
@@ -254,11 +251,28 @@ int layout_stride(int layout, int K) {
   return ((kp / 4) & 1) ? kp : kp + 4;
 }
 
+static size_t slots_bytes(int layout, int alphabet, int slots, int K) {
+  const size_t per = (size_t)slots * layout_stride(layout, K);
+  if (layout == PROF_PAIR) return (size_t)alphabet * alphabet * per * 4;
+  if (layout == PROF_S32) return (size_t)alphabet * per * 4;
+  return (size_t)alphabet * per * 2;
+}
+
+// Thread slices per profile row.  A quarter-warp loads 16 bytes per thread, and
+// eight consecutive slices of a row lie in different banks, so groups of eight
+// threads or more never conflict; narrower groups of a quarter-warp read rows
+// of different codes that start at the same banks.  Their slices are repeated
+// up to eight per row, one set for each group of the quarter-warp, as long as
+// the profile stays at 44 KB (three blocks per SM of local alignment's widest
+// rows still fit beside it).  Measured on 100,000 proteins, semi-global, 16
+// columns per thread: one thread per pair 1,117 -> 1,932 GCUPS, four threads
+// 4,155 -> 6,300.
+int profile_slots(int layout, int alphabet, int G, int K) {
+  return G < 8 && slots_bytes(layout, alphabet, 8, K) <= 44 * 1024 ? 8 : G;
+}
+
 size_t layout_bytes(int layout, int alphabet, int G, int K) {
-  const size_t kp = (size_t)layout_stride(layout, K);
-  if (layout == PROF_PAIR) return (size_t)alphabet * alphabet * G * kp * 4;
-  if (layout == PROF_S32) return (size_t)alphabet * G * kp * 4;
-  return (size_t)alphabet * G * kp * 2;
+  return slots_bytes(layout, alphabet, profile_slots(layout, alphabet, G, K), K);
 }
 
 // The pair layout (no per-column work to assemble a record pair's word) when
@@ -271,7 +285,12 @@ int choose_layout(int alphabet, int G, int K, int mode) {
   return PROF_S16;
 }
 
-void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout) {
+// For a set with few or very unequal records a wider group can finish sooner
+// than the shape with the highest rate: 3,000 proteins against 120 residues ran
+// 31 columns per thread at the pace of the longest record's one group.  The
+// padded query counts towards the fast regime's bounds, so a shape for the set is
+// taken only where it keeps the query and the set's longest record inside them.
+void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const RecordSet *set, double share) {
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
   auto it = ctx->tuned.find(tune_key(mode, q.rows, q.Q));
   if (!ctx->force_G && !ctx->force_K && ctx->force_layout < 0 && it != ctx->tuned.end()) {
@@ -280,8 +299,21 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout) {
     *layout = it->second.layout >= 0 ? it->second.layout : choose_layout(q.rows, *G, *K, mode);
     return;
   }
-  choose_shape(q.Q, ctx->force_G, ctx->force_K, G, K);
-  *layout = ctx->force_layout >= 0 ? ctx->force_layout : (*G ? choose_layout(q.rows, *G, *K, mode) : PROF_S16);
+  auto layout_of = [&](int g, int k) {
+    return ctx->force_layout >= 0 ? ctx->force_layout : (g ? choose_layout(q.rows, g, k, mode) : (int)PROF_S16);
+  };
+  choose_shape(ctx, mode, q.Q, nullptr, 1, G, K);
+  *layout = layout_of(*G, *K);
+  if (!set || !*G) return;
+  int g = 0, k = 0;
+  choose_shape(ctx, mode, q.Q, set, share, &g, &k);
+  // (within a tenth the model does not tell shapes apart)
+  if (!g || shape_clocks(ctx, mode, g, k, set, share) > 0.9 * shape_clocks(ctx, mode, *G, *K, set, share)) return;
+  const Regime r = regime(q, g * k);
+  if (!r.fast || set->max_len > r.max_safe_len || !wave_fits(q, g, k, layout_of(g, k))) return;
+  *G = g;
+  *K = k;
+  *layout = layout_of(g, k);
 }
 
 int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayout **out) {
@@ -297,6 +329,7 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
   L.d = G * K - q.Q;
   L.layout = layout;
   L.kp = layout_stride(layout, K);
+  L.slots = profile_slots(layout, q.rows, G, K);
   // profile rows: one per class of codes with equal scores against the
   // query (q.rep), addressed through q.rowmap when the classes merge codes
   const int A = q.rows;
@@ -311,33 +344,34 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
   };
   std::vector<uint8_t> host;
   if (layout == PROF_PAIR) {
-    std::vector<uint32_t> w((size_t)A * A * G * L.kp, 0u);
+    std::vector<uint32_t> w((size_t)A * A * L.slots * L.kp, 0u);
     for (int a = 0; a < A; ++a)
       for (int b = 0; b < A; ++b)
-        for (int t = 0; t < G; ++t)
+        for (int t = 0; t < L.slots; ++t)
           for (int j = 0; j < K; ++j) {
-            const int col = t * K + j - L.d;
-            w[((size_t)(a * A + b) * G + t) * L.kp + j] =
+            const int col = (t & (G - 1)) * K + j - L.d;
+            w[((size_t)(a * A + b) * L.slots + t) * L.kp + j] =
                 sg ? ((uint32_t)P(b, col) << 16) + (uint32_t)P(a, col)
                    : ((uint32_t)P(a, col) & 0xffffu) | ((uint32_t)P(b, col) << 16);
           }
     host.resize(w.size() * 4);
     memcpy(host.data(), w.data(), host.size());
   } else if (layout == PROF_S32) {
-    std::vector<uint32_t> w((size_t)A * G * L.kp, 0u);
+    std::vector<uint32_t> w((size_t)A * L.slots * L.kp, 0u);
     for (int a = 0; a < A; ++a)
-      for (int t = 0; t < G; ++t)
+      for (int t = 0; t < L.slots; ++t)
         for (int j = 0; j < K; ++j) {
-          const uint32_t v = (uint32_t)P(a, t * K + j - L.d);
-          w[((size_t)a * G + t) * L.kp + j] = sg ? v : v & 0xffffu;
+          const uint32_t v = (uint32_t)P(a, (t & (G - 1)) * K + j - L.d);
+          w[((size_t)a * L.slots + t) * L.kp + j] = sg ? v : v & 0xffffu;
         }
     host.resize(w.size() * 4);
     memcpy(host.data(), w.data(), host.size());
   } else {
-    std::vector<int16_t> w((size_t)A * G * L.kp, 0);
+    std::vector<int16_t> w((size_t)A * L.slots * L.kp, 0);
     for (int a = 0; a < A; ++a)
-      for (int t = 0; t < G; ++t)
-        for (int j = 0; j < K; ++j) w[((size_t)a * G + t) * L.kp + j] = (int16_t)P(a, t * K + j - L.d);
+      for (int t = 0; t < L.slots; ++t)
+        for (int j = 0; j < K; ++j)
+          w[((size_t)a * L.slots + t) * L.kp + j] = (int16_t)P(a, (t & (G - 1)) * K + j - L.d);
     host.resize(w.size() * 2);
     memcpy(host.data(), w.data(), host.size());
   }
@@ -730,7 +764,8 @@ void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDe
   p.pk_left = sg ? (ts ? (uint32_t)p.bias : (uint32_t)q.open) * 0x10001u : 0u;
   p.pk_left_ext = sg && ts ? (uint32_t)q.ext * 0x10001u : 0u;
   p.pk_drop = sg ? (uint32_t)(-(p.frame_mask + 1) * q.ext) * 0x10001u : 0u;
-  p.row_bytes = (uint32_t)(L.G * L.kp * (L.layout == PROF_S16 ? 2 : 4));
+  p.slots = L.slots;
+  p.row_bytes = (uint32_t)(L.slots * L.kp * (L.layout == PROF_S16 ? 2 : 4));
   p.error = error;
   p.rec = RecordsDev{rs.codes.as<const uint8_t>(), rs.off_s.as<const uint64_t>(), rs.len_s.as<const uint32_t>(),
                      rs.orig_s.as<const uint32_t>(), rs.n};
@@ -753,7 +788,7 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
   int rc = build_wave_layout(ctx, q, G, K, layout, &L);
   if (rc) return rc;
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
-  const int lean = wave_lean(ctx, K, mode, G);
+  const int lean = wave_lean(ctx, K, mode);
   WaveFn fn = wave_fn(K, mode, L->layout, lean);
   if (!fn) return fail(ctx, ISH_EOVERFLOW, "no wavefront kernel for K=%d", K);
   const int threads = wave_threads_lean(K, mode, lean);
@@ -866,17 +901,9 @@ int fast_check(const Query &q, const RecordSet &rs, int G, int K, char *msg, siz
 
 bool fast_regime(ish_ctx *ctx, const Query &q, const RecordSet &rs) {
   int G, K, layout;
-  pick_shape(ctx, q, &G, &K, &layout);
+  pick_shape(ctx, q, &G, &K, &layout, &rs);
   char msg[256];
   return fast_check(q, rs, G, K, msg, sizeof msg) == ISH_OK;
-}
-
-int check_fast(ish_ctx *ctx, const Query &q, const RecordSet &rs) {
-  int G, K, layout;
-  pick_shape(ctx, q, &G, &K, &layout);
-  char msg[256];
-  const int rc = fast_check(q, rs, G, K, msg, sizeof msg);
-  return rc ? fail(ctx, rc, "%s", msg) : ISH_OK;
 }
 
 // Whether the wavefront kernel's shared memory (profile, code -> row table,
@@ -894,7 +921,7 @@ bool wave_fits(const Query &q, int G, int K, int layout) {
 // kernel was asked for.
 int launch_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uint32_t count, OutDev out, cudaStream_t s) {
   int G, K, layout;
-  pick_shape(ctx, q, &G, &K, &layout);
+  pick_shape(ctx, q, &G, &K, &layout, &rs);
   if (ctx->kernel == ISH_KERNEL_PLAIN || ctx->kernel == ISH_KERNEL_PLAIN16 || !wave_fits(q, G, K, layout)) {
     if (s != ctx->stream) return fail(ctx, ISH_EINVAL, "the plain kernel runs on the context stream only");
     return launch_plain(ctx, q, rs, first, count, out);

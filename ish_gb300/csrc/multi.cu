@@ -20,7 +20,7 @@ namespace ish {
 namespace host {
 
 struct MultiClass {
-  int K = 0, mode = 0, layout = 0, threads = 0, Gmin = 32;
+  int K = 0, mode = 0, layout = 0, threads = 0;
   BatchFn fn = nullptr;
   size_t smem = 0;
   uint32_t grid = 0, ntiles = 0, prof_area = 0, counter_base = 0;
@@ -134,9 +134,13 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
                   q.alphabet, qids[i]);
     Member m;
     m.pos = i;
-    pick_shape(ctx, q, &m.G, &m.K, &m.layout);
     m.mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
-    if (!fast_regime(ctx, q, rs) || !wave_fits(q, m.G, m.K, m.layout)) {
+    pick_shape(ctx, q, &m.G, &m.K, &m.layout);
+    const uint64_t overlap = windowable_whole(q) ? window_overlap(q) : 0;
+    if (!overlap || !m.G || !window_stride(ctx, rs, overlap, m.G, m.K, m.mode))  // (windows even the records out)
+      pick_shape(ctx, q, &m.G, &m.K, &m.layout, &rs, nq);
+    char why[256];
+    if (fast_check(q, rs, m.G, m.K, why, sizeof why) != ISH_OK || !wave_fits(q, m.G, m.K, m.layout)) {
       // outside the wavefront kernels' exact regime, or a profile that fits
       // no layout: the lane-exact kernels score this query in the same graph
       int rc = exact_prepare(ctx, q, nonempty, P.exact);
@@ -199,13 +203,12 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
     }
     MultiClass &c = P.classes[it->second];
     c.members.push_back(m.pos);
-    c.Gmin = std::min(c.Gmin, m.G);
     c.prof_area = std::max(c.prof_area, (m.L->prof_bytes + 15u) & ~15u);
   }
 
   // ---- per class: kernel, occupancy, parameters, tiles ----
   for (MultiClass &c : P.classes) {
-    const int lean = batch_lean(ctx, c.K, c.mode, c.Gmin);
+    const int lean = wave_lean(ctx, c.K, c.mode);
     c.fn = batch_fn(c.K, c.mode, c.layout, lean);
     if (!c.fn) return fail(ctx, ISH_EOVERFLOW, "no batch kernel for K=%d", c.K);
     c.threads = wave_threads_lean(c.K, c.mode, lean);

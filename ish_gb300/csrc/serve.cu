@@ -315,7 +315,7 @@ int step(Server &S, char *msg) {
   cudaStream_t s = S.s;
   // ---- classes of this step ----
   struct Cls {
-    int K, mode, layout, Gmin = 32;
+    int K, mode, layout;
     uint32_t prof_area = 0, first = 0, count = 0;
   };
   std::vector<Cls> cls;
@@ -329,7 +329,6 @@ int step(Server &S, char *msg) {
       cls.push_back(Cls{r->K, r->mode, r->layout});
       members.emplace_back();
     }
-    cls[c].Gmin = std::min(cls[c].Gmin, r->G);
     cls[c].prof_area = std::max(cls[c].prof_area, (r->L->prof_bytes + 15u) & ~15u);
     members[c].push_back(r);
   }
@@ -366,7 +365,7 @@ int step(Server &S, char *msg) {
     }
     for (size_t c = 0; c < cls.size(); ++c) {
       const Cls &C = cls[c];
-      const int lean = batch_lean(S.ctx, C.K, C.mode, C.Gmin);
+      const int lean = wave_lean(S.ctx, C.K, C.mode);
       BatchFn fn = batch_fn(C.K, C.mode, C.layout, lean);
       if (!fn) {
         snprintf(msg, 256, "no batch kernel for K=%d", C.K);

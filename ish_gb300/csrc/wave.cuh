@@ -109,7 +109,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   const uint32_t LEFT_EXT = (MODE == SG) ? p.pk_left_ext : 0u;
   // this thread's part of every profile row, and the bytes between the rows
   // of consecutive codes: a row's address is one multiply-add
-  const unsigned char *prof_t = prof + (uint32_t)(t * kp) * (LAYOUT == PROF_S16 ? 2u : 4u);
+  const unsigned char *prof_t = prof + (uint32_t)((lane & (p.slots - 1)) * kp) * (LAYOUT == PROF_S16 ? 2u : 4u);
   const uint32_t row_bytes = p.row_bytes;
 
   uint32_t H[K], E[K];

@@ -112,7 +112,7 @@ uint64_t window_overlap(const Query &q) {
 // when windows would not help: the longest records must exceed twice the
 // rows a group scores on average (they would bound the pass) and one window.
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode) {
-  const int lean = wave_lean(ctx, K, mode, G);
+  const int lean = wave_lean(ctx, K, mode);
   // groups in flight and the rows each would score on average (two records
   // per pair share their rows)
   const uint64_t groups =
@@ -242,7 +242,7 @@ int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, Out
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
   int G, K, layout;
   pick_shape(ctx, q, &G, &K, &layout);
-  if (!G || !wave_fits(q, G, K, layout)) return ISH_OK;
+  if (!G || !wave_fits(q, G, K, layout) || !regime(q, G * K).fast) return ISH_OK;
   const uint64_t W = window_stride(ctx, rs, O, G, K, mode);
   if (!W) return ISH_OK;
   WindowView &V = rs.windows;
@@ -255,6 +255,7 @@ int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, Out
   CU(R.tend.ensure((size_t)nw * 4));
   CU(R.hit.ensure((size_t)nw));
   RecordSet view = window_set(rs, V);
+  pick_shape(ctx, q, &G, &K, &layout, &view);  // the windows may be few
   OutDev wout{R.score.as<int32_t>(), R.qend.as<int32_t>(), R.tend.as<int32_t>(), R.hit.as<uint8_t>()};
   Query &qc = fixed_start_of(q);
   if (&qc == &q) {
