@@ -195,20 +195,28 @@ static double warp_row_clocks(int mode, int K) {
 }
 static double lone_row_clocks(int mode, int K) { return mode == SG ? 150 + 9.5 * K : 200 + 17.5 * K; }
 
+// Warps per scheduler of a full SM, by the kernels' launch bounds.
+static double full_warps(int K) { return K <= 32 ? 4 : K <= 48 ? 3 : 2; }
+
+// Clocks in which each of `warps` warps on the device advances by one row: from
+// one warp per scheduler to a full SM about linear (K = 32: 451 alone, 740 with
+// two, 1,300 with four).
+double row_clocks(const ish_ctx *ctx, int mode, int K, double warps) {
+  const double w = std::max(1.0, warps / (4.0 * ctx->num_sms)), cap = full_warps(K), lone = lone_row_clocks(mode, K);
+  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * warp_row_clocks(mode, K) - lone);
+}
+
 // Modelled time of one query against `set` (null: many records of any length)
 // with G threads x K columns: every warp's share of the rows at the rate of the
 // warps in flight, or the longest pair alone, whichever takes longer.  `share`
 // queries run at once.
 static double shape_clocks(const ish_ctx *ctx, int mode, int G, int K, const RecordSet *set, double share) {
-  const double row = warp_row_clocks(mode, K);
-  if (!set) return G * row;
-  const double schedulers = 4.0 * ctx->num_sms;
+  if (!set) return G * warp_row_clocks(mode, K);
   const double pairs = std::max(1.0, (set->n - set->n_empty) / 2.0) * share, rows = set->total / 2.0 * share;
-  const double full = schedulers * (K <= 32 ? 4 : K <= 48 ? 3 : 2);
+  const double full = 4.0 * ctx->num_sms * full_warps(K);
   const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), full));
-  const double per_row = std::max(lone_row_clocks(mode, K), std::max(1.0, warps / schedulers) * row);
-  const double all = rows * G / 32 / warps * per_row;
-  const double last = ((double)set->max_len + 4 * G) * std::max(lone_row_clocks(mode, K), row);
+  const double all = rows * G / 32 / warps * row_clocks(ctx, mode, K, warps);
+  const double last = ((double)set->max_len + 4 * G) * row_clocks(ctx, mode, K, 1);
   return std::max(all, last) + 0.1 * all;
 }
 

@@ -34,6 +34,7 @@
 // first), scores it with the wavefront kernel into per-window results, and
 // folds them per record on the device.
 #include <algorithm>
+#include <cmath>
 #include <numeric>
 #include <vector>
 
@@ -109,8 +110,15 @@ uint64_t window_overlap(const Query &q) {
 #endif
 
 // The window stride for scoring `rs` with groups of the given shape, or 0
-// when windows would not help: the longest records must exceed twice the
-// rows a group scores on average (they would bound the pass) and one window.
+// when windows would not help: the longest record must exceed 1.25x the rows a
+// group scores on average (see above) and one window.  Narrow windows spread
+// the records over more groups and wide ones repeat fewer rows, so strides are
+// compared by a model.  With pairs of windows for less than half the groups, a
+// pass takes one window at the rate of that many warps; with more, all rows at
+// the full device's rate and 0.4 windows for the uneven end (0.3 to 0.5 measured
+// alike, 0.8 and 1.2 worse; one round that just fits is not trusted to).  With a
+// stride of at least 8 x O, 10 records of 10 kb - 1 Mb made 32 windows for 1,000
+// nt (11.4 ms; 2.2 ms with this rule), 200 records 1,102 (11.7 ms; 8.4 ms).
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode) {
   const int lean = wave_lean(ctx, K, mode);
   // groups in flight and the rows each would score on average (two records
@@ -118,12 +126,35 @@ uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int 
   const uint64_t groups =
       (uint64_t)ctx->num_sms * wave_blocks_lean(K, mode, lean) * (wave_threads_lean(K, mode, lean) / G);
   const uint64_t avg_rows = rs.total / 2 / std::max<uint64_t>(groups, 1);
-  // window stride: about four pairs of windows per group, and at least 8x
-  // the overlap so that windowing adds at most an eighth of the work
-  uint64_t W = std::max<uint64_t>(8 * O, rs.total / std::max<uint64_t>(8 * groups, 1));
-  W = (W + 15) & ~15ull;
-  if (rs.max_len * 4 <= avg_rows * ISH_WINDOW_QUARTERS || rs.max_len <= W + O) return 0;
-  return W;
+  if (rs.max_len * 4 <= avg_rows * ISH_WINDOW_QUARTERS) return 0;
+  // rows in records longer than 2^(i/8) (all of them where the set has no
+  // histogram)
+  constexpr int BINS = 8 * 33;
+  std::vector<double> above(BINS + 1, 0.0);
+  auto bin_of = [](double len) { return std::min(BINS - 1, std::max(0, (int)(8 * std::log2(std::max(len, 1.0))))); };
+  for (uint32_t b = 1; b < rs.hist.size(); ++b)
+    if (rs.hist[b]) {
+      const double len = b < 32768 ? b : 32768 + 32.0 * (b - 32768) + 16;
+      above[bin_of(len)] += len * rs.hist[b];
+    }
+  if (rs.hist.empty()) above[BINS - 1] = (double)rs.total;
+  for (int i = BINS - 1; i >= 0; --i) above[i] += above[i + 1];
+  const double warps = (double)groups * G / 32;
+  uint64_t best = 0;
+  double best_t = 1e300;
+  for (double w = 256; w + O < rs.max_len; w *= 1.08) {
+    const double cut = above[bin_of(w + O)];  // rows that are cut into windows
+    const double work = (rs.total + cut * (double)O / w) / 2;
+    const double pairs = std::ceil((cut / w + rs.n) / 2);
+    const double full = row_clocks(ctx, mode, K, warps);
+    const double t = 2 * pairs >= groups ? work / groups * full + 0.4 * (w + O) * full
+                                         : 1.15 * (w + O) * row_clocks(ctx, mode, K, pairs * G / 32);
+    if (t < best_t) {
+      best_t = t;
+      best = ((uint64_t)w + 15) & ~15ull;
+    }
+  }
+  return best + O < rs.max_len ? best : 0;
 }
 
 // Builds the window view of sorted entries [0, nonempty) of rs (stride W,
@@ -150,12 +181,14 @@ int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint
       woff.push_back(off[e]);
       continue;
     }
-    for (uint64_t k = 0; k * W < L; ++k) {
-      const uint64_t st = k == 0 ? 0 : ((k * W - O) & ~15ull);
-      const uint64_t en = std::min<uint64_t>(L, (k + 1) * W);
+    // window k covers [k * W, (k + 1) * W + O): the cells it adds to the windows
+    // before it lie O rows or more below its start
+    for (uint64_t st = 0;; st += W) {
+      const uint64_t en = std::min<uint64_t>(L, st + W + O);
       wstart.push_back((uint32_t)st);
       wlen.push_back((uint32_t)(en - st));
       woff.push_back(off[e] + st);
+      if (en == L) break;
     }
   }
   const uint32_t nw = (uint32_t)wstart.size();
