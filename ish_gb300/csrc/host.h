@@ -10,6 +10,8 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -238,6 +240,9 @@ struct ish_ctx {
   // kernels launched by the library on this context (graph replays count
   // their kernel nodes; the serving thread adds its own)
   std::atomic<uint64_t> launches{0};
+  // kernels whose shared memory limit has been raised (also by the serving thread)
+  std::set<const void *> smem_allowed;
+  std::mutex smem_mu;
 };
 
 
@@ -274,7 +279,7 @@ inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1)
 
 int frame_rows(int ext);
 int wave_lean(const ish_ctx *ctx, int K, int mode);
-double row_clocks(const ish_ctx *ctx, int mode, int K, double warps);
+double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps);
 uint64_t window_overlap(const Query &q);
 int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, OutDev out, cudaStream_t s, bool *done);
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode);
@@ -299,7 +304,7 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
 uint64_t tune_key(int mode, int alphabet, int Q);
 int layout_stride(int layout, int K);
 size_t layout_bytes(int layout, int alphabet, int G, int K);
-int choose_layout(int alphabet, int G, int K, int mode);
+int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode);
 int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayout **out);
 int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, uint32_t n, RecordSet &rs,
                  const uint8_t *enc, cudaStream_t s = nullptr, bool defer = false);
@@ -342,7 +347,13 @@ void drop_plans(ish_ctx *ctx, int32_t query_id, int32_t set_id);  // multi.cu
 void free_plans(ish_ctx *ctx);                                   // multi.cu
 void stop_server(ish_ctx *ctx);                                  // serve.cu
 bool server_uses_set(const ish_ctx *ctx, int32_t set_id);        // serve.cu
-size_t wave_smem(uint32_t prof_area, int threads, int G, int K, int mode);
+// Threads per block, blocks and dynamic shared memory of a batched launch.
+struct BatchLaunch {
+  int threads = 0;
+  uint32_t grid = 0;
+  size_t smem = 0;
+};
+int batch_launch(ish_ctx *ctx, BatchFn fn, int K, int mode, int lean, size_t prof_area, BatchLaunch *out);
 
 }  // namespace host
 }  // namespace ish

@@ -188,10 +188,12 @@ int neg_limit_of(int open, int mmin) {
 // lines through measurements at G = 8, proteins, K = 4..64 (semi-global 87 at K =
 // 4, 180 at 16, 326 at 32, 384 at 38, 631 at 60; local 184, 258, 468, 561, 941;
 // alone 451 / 752 at K = 32, 619 / 1,074 at 48), with what the builds with fewer
-// warps add.
-static double warp_row_clocks(int mode, int K) {
-  if (mode == SG) return (50 + 8.6 * K) * (K > 48 ? 1.1 : 1.0);
-  return (50 + 13.3 * K) * (K > 40 ? 1.08 : 1.0);
+// warps add, and wide groups (32 threads 9 % at K = 16..32 on proteins: most
+// steps of a warp start a pair in one of its threads).
+static double warp_row_clocks(int mode, int K, int G) {
+  const double wide = 1.0 + 0.1 * (G / 32.0) * (G / 32.0);
+  if (mode == SG) return (50 + 8.6 * K) * (K > 48 ? 1.1 : 1.0) * wide;
+  return (50 + 13.3 * K) * (K > 40 ? 1.08 : 1.0) * wide;
 }
 static double lone_row_clocks(int mode, int K) { return mode == SG ? 150 + 9.5 * K : 200 + 17.5 * K; }
 
@@ -201,9 +203,9 @@ static double full_warps(int K) { return K <= 32 ? 4 : K <= 48 ? 3 : 2; }
 // Clocks in which each of `warps` warps on the device advances by one row: from
 // one warp per scheduler to a full SM about linear (K = 32: 451 alone, 740 with
 // two, 1,300 with four).
-double row_clocks(const ish_ctx *ctx, int mode, int K, double warps) {
+double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps) {
   const double w = std::max(1.0, warps / (4.0 * ctx->num_sms)), cap = full_warps(K), lone = lone_row_clocks(mode, K);
-  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * warp_row_clocks(mode, K) - lone);
+  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * warp_row_clocks(mode, K, G) - lone);
 }
 
 // Modelled time of one query against `set` (null: many records of any length)
@@ -211,12 +213,12 @@ double row_clocks(const ish_ctx *ctx, int mode, int K, double warps) {
 // warps in flight, or the longest pair alone, whichever takes longer.  `share`
 // queries run at once.
 static double shape_clocks(const ish_ctx *ctx, int mode, int G, int K, const RecordSet *set, double share) {
-  if (!set) return G * warp_row_clocks(mode, K);
+  if (!set) return G * warp_row_clocks(mode, K, G);
   const double pairs = std::max(1.0, (set->n - set->n_empty) / 2.0) * share, rows = set->total / 2.0 * share;
   const double full = 4.0 * ctx->num_sms * full_warps(K);
   const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), full));
-  const double all = rows * G / 32 / warps * row_clocks(ctx, mode, K, warps);
-  const double last = ((double)set->max_len + 4 * G) * row_clocks(ctx, mode, K, 1);
+  const double all = rows * G / 32 / warps * row_clocks(ctx, mode, K, G, warps);
+  const double last = ((double)set->max_len + 4 * G) * row_clocks(ctx, mode, K, G, 1);
   return std::max(all, last) + 0.1 * all;
 }
 
@@ -272,9 +274,8 @@ static size_t slots_bytes(int layout, int alphabet, int slots, int K) {
 // of different codes that start at the same banks.  Their slices are repeated
 // up to eight per row, one set for each group of the quarter-warp, as long as
 // the profile stays at 44 KB (three blocks per SM of local alignment's widest
-// rows still fit beside it).  Measured on 100,000 proteins, semi-global, 16
-// columns per thread: one thread per pair 1,117 -> 1,932 GCUPS, four threads
-// 4,155 -> 6,300.
+// rows still fit beside it).  Measured on 300,000 proteins, semi-global: four
+// threads x 16 columns 4,155 -> 6,565 GCUPS, x 38 columns 4,661 -> 7,924.
 int profile_slots(int layout, int alphabet, int G, int K) {
   return G < 8 && slots_bytes(layout, alphabet, 8, K) <= 44 * 1024 ? 8 : G;
 }
@@ -283,13 +284,39 @@ size_t layout_bytes(int layout, int alphabet, int G, int K) {
   return slots_bytes(layout, alphabet, profile_slots(layout, alphabet, G, K), K);
 }
 
-// The pair layout (no per-column work to assemble a record pair's word) when
-// it takes at most 64 KB; else 32-bit single-code words (one IMAD per column)
-// when a block still fits twice on an SM; else 16-bit words (one PRMT).
-int choose_layout(int alphabet, int G, int K, int mode) {
-  if (layout_bytes(PROF_PAIR, alphabet, G, K) <= 64 * 1024) return PROF_PAIR;
-  if (wave_smem((uint32_t)layout_bytes(PROF_S32, alphabet, G, K), wave_block_threads(K, mode), G, K, mode) <= 112 * 1024)
-    return PROF_S32;
+// Shared memory of a wavefront block: the profile, a slot word per thread, and
+// (local alignment) wave_save_words(K) save words per thread (see wave.cuh).
+static size_t wave_smem(size_t prof_area, int threads, int K, int mode) {
+  return prof_area + (size_t)threads * 4 * (1 + (mode == SW ? wave_save_words(K) : 0));
+}
+// What a block may ask for: 227 KB less the kernels' static copy of their
+// parameters.
+static constexpr size_t WAVE_SMEM_MAX = 226 * 1024;
+
+// Threads of the largest block of this shape that fits beside the profile: all
+// the SM's registers allow, or fewer where their saved rows do not fit.
+static int wave_fit_threads(size_t prof_area, int K, int mode, int lean) {
+  int t = wave_sm_threads(K, lean);
+  while (t > 0 && wave_smem(prof_area, t, K, mode) > WAVE_SMEM_MAX) t -= 32;
+  return t;
+}
+
+// The pair layout (no per-column work to assemble a record pair's word, half
+// the shared-memory loads of the 32-bit one) while all of an SM's threads fit
+// beside it; else 32-bit single-code words under the same rule; else 16-bit
+// words, whose PRMT per column costs what up to a quarter of the warps do.
+// Measured: 1,000 nt x 200,000 reads, semi-global, 7,820 GCUPS with the 115 KB
+// pair profile, 6,920 with 32-bit words, 5,930 with 16-bit ones; 1,501 residues x
+// 100,000 proteins 7,440 with the 160 KB 32-bit profile, 6,600 with 16-bit words;
+// 1,900 residues, local, where 96 of 256 threads fit beside the 32-bit profile,
+// 3,165 against 4,670 with 16-bit words.
+int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode) {
+  const int lean = wave_lean(ctx, K, mode), all = wave_sm_threads(K, lean);
+  auto fit = [&](int layout) {
+    return wave_fit_threads(((layout_bytes(layout, rows, G, K) + 15) & ~(size_t)15) + 256, K, mode, lean);
+  };
+  if (fit(PROF_PAIR) == all) return PROF_PAIR;
+  if (4 * fit(PROF_S32) >= 3 * all) return PROF_S32;
   return PROF_S16;
 }
 
@@ -304,11 +331,11 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
   if (!ctx->force_G && !ctx->force_K && ctx->force_layout < 0 && it != ctx->tuned.end()) {
     *G = it->second.G;
     *K = it->second.K;
-    *layout = it->second.layout >= 0 ? it->second.layout : choose_layout(q.rows, *G, *K, mode);
+    *layout = it->second.layout >= 0 ? it->second.layout : choose_layout(ctx, q.rows, *G, *K, mode);
     return;
   }
   auto layout_of = [&](int g, int k) {
-    return ctx->force_layout >= 0 ? ctx->force_layout : (g ? choose_layout(q.rows, g, k, mode) : (int)PROF_S16);
+    return ctx->force_layout >= 0 ? ctx->force_layout : (g ? choose_layout(ctx, q.rows, g, k, mode) : (int)PROF_S16);
   };
   choose_shape(ctx, mode, q.Q, nullptr, 1, G, K);
   *layout = layout_of(*G, *K);
@@ -781,11 +808,13 @@ void wave_params(const Query &q, const WaveLayout &L, const RecordSet &rs, OutDe
   p.dec = Decision{q.max_score, q.thr};
 }
 
-// Shared memory of a wavefront block: the profile, a slot word per thread,
-// and (local alignment) wave_save_words(K) save words per thread (see wave.cuh).
-size_t wave_smem(uint32_t prof_area, int threads, int G, int K, int mode) {
-  const size_t save = mode == SW ? (size_t)threads * wave_save_words(K) * 4 : 0;
-  return prof_area + (size_t)threads * 4 + save;
+// Sets a kernel's dynamic shared memory limit, once per kernel and context.
+static cudaError_t allow_smem(ish_ctx *ctx, const void *fn) {
+  std::lock_guard<std::mutex> lk(ctx->smem_mu);
+  if (ctx->smem_allowed.count(fn)) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WAVE_SMEM_MAX);
+  if (e == cudaSuccess) ctx->smem_allowed.insert(fn);
+  return e;
 }
 
 int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uint32_t count, OutDev out, int G, int K,
@@ -799,11 +828,8 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
   const int lean = wave_lean(ctx, K, mode);
   WaveFn fn = wave_fn(K, mode, L->layout, lean);
   if (!fn) return fail(ctx, ISH_EOVERFLOW, "no wavefront kernel for K=%d", K);
-  const int threads = wave_threads_lean(K, mode, lean);
-  const int groups = threads / G;
-  const size_t smem = wave_smem((L->prof_bytes + 15) & ~15u, threads, G, K, mode);
   {
-    const cudaError_t e = cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(ctx, (const void *)fn);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       cudaFuncAttributes a{};
@@ -812,17 +838,21 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
       return fail(ctx, ISH_EDEVICE,
                   "wavefront kernel K=%d mode=%d layout=%d: dynamic shared memory %zu bytes refused (%s); kernel "
                   "attributes (%s): static %zu, max dynamic %d, %d registers",
-                  K, mode, L->layout, smem, cudaGetErrorString(e), cudaGetErrorString(ea), a.sharedSizeBytes,
+                  K, mode, L->layout, WAVE_SMEM_MAX, cudaGetErrorString(e), cudaGetErrorString(ea), a.sharedSizeBytes,
                   a.maxDynamicSharedSizeBytes, a.numRegs);
     }
   }
-  int per_sm = 0;
-  CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, threads, smem));
-  if (per_sm < 1) return fail(ctx, ISH_EOVERFLOW, "wavefront kernel K=%d does not fit (smem %zu)", K, smem);
-  if (ctx->force_blocks) per_sm = std::min(per_sm, ctx->force_blocks);
+  // One block per SM with as many warps as the SM holds, or as the range's
+  // record pairs need when spread over all SMs.
+  const size_t prof_area = (L->prof_bytes + 15) & ~15u;
+  int most = wave_fit_threads(prof_area, K, mode, lean);
+  if (most < 32) return fail(ctx, ISH_EOVERFLOW, "wavefront kernel K=%d does not fit (profile %zu)", K, prof_area);
+  if (ctx->force_blocks) most = std::min(most, ctx->force_blocks * (K <= 32 ? 256 : 128));
   const uint32_t pairs = (count + 1) / 2;
-  const uint32_t want = ceil_div(pairs, groups);
-  const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(want, (uint32_t)(per_sm * ctx->num_sms)));
+  const uint32_t warps = ceil_div((uint64_t)pairs * G, 32);
+  const int threads = (int)std::min<uint32_t>(most, 32 * ceil_div(warps, ctx->num_sms));
+  const uint32_t grid = std::min<uint32_t>(ctx->num_sms, ceil_div(warps, threads / 32));
+  const size_t smem = wave_smem(prof_area, threads, K, mode);
   WaveParams p;
   wave_params(q, *L, rs, out, ctx->error.as<int>(), &p);
   p.first = first;
@@ -834,6 +864,28 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
   ++ctx->launches;
   CU(cudaGetLastError());
   return ISH_OK;
+}
+
+// Blocks of a persistent batched launch: the size among 128 and 256 threads and
+// all of an SM's that keeps most threads resident, the smaller one where equal
+// (a block waits for its slowest pair at every query switch; small blocks of an
+// SM switch at different times).
+int batch_launch(ish_ctx *ctx, BatchFn fn, int K, int mode, int lean, size_t prof_area, BatchLaunch *out) {
+  CU(allow_smem(ctx, (const void *)fn));
+  const int all = wave_sm_threads(K, lean);
+  int best = 0;
+  for (int t : {128, 256, wave_fit_threads(prof_area, K, mode, lean)}) {
+    if (t < 32 || t > all) continue;
+    const size_t smem = wave_smem(prof_area, t, K, mode);
+    if (smem > WAVE_SMEM_MAX) continue;
+    int per_sm = std::min<int>(all / t, (int)((228 * 1024) / (smem + 2048)));
+    if (ctx->force_blocks) per_sm = std::min(per_sm, ctx->force_blocks);
+    if (per_sm * t > best) {
+      best = per_sm * t;
+      *out = BatchLaunch{t, (uint32_t)(std::max(per_sm, 1) * ctx->num_sms), smem};
+    }
+  }
+  return best ? ISH_OK : fail(ctx, ISH_EOVERFLOW, "batch kernel K=%d does not fit (profile %zu)", K, prof_area);
 }
 
 int launch_plain(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uint32_t count, OutDev out) {
@@ -921,7 +973,7 @@ bool wave_fits(const Query &q, int G, int K, int layout) {
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
   size_t prof = (layout_bytes(layout, q.rows, G, K) + 15) & ~(size_t)15;
   if (q.rows < q.alphabet) prof += 256;
-  return wave_smem((uint32_t)prof, wave_block_threads(K, mode), G, K, mode) <= 227 * 1024;
+  return wave_smem(prof, 128, K, mode) <= WAVE_SMEM_MAX;
 }
 
 // The wavefront kernel, or the plain kernel when the wavefront profile does

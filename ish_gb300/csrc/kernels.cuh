@@ -70,28 +70,17 @@ __global__ void k_gather_hits(const uint32_t *idx, const uint32_t *count, const 
 // Wavefront kernels are instantiated for K = 2, 4, ..., WAVE_KMAX columns per
 // thread, both modes and both profile layouts.
 constexpr int WAVE_KMAX = 64;
-// Threads per block and blocks per SM (the register budget): 256 x 2 up to
-// K = 32 columns per thread, 128 x 3 up to K = 48 (12 warps per SM for wide
-// rows), above that 128 x 2 for semi-global and 256 x 1 for local alignment
-// (whose long-query profiles and saved rows would otherwise fit only one
-// 128-thread block per SM: +46 % at Q = 1900).
-__host__ __device__ constexpr int wave_block_threads(int K, int mode) {
-  return K <= 32 ? 256 : (K <= 48 ? 128 : (mode == 1 ? 256 : 128));
-}
-__host__ __device__ constexpr int wave_blocks_per_sm(int K, int mode) {
-  return K <= 32 ? 2 : (K <= 48 ? 3 : (mode == 1 ? 1 : 2));
-}
-// Register-lean builds trade warps for registers per thread: for
-// 25 <= K <= 32, 128 x 3 (12 warps, 170 registers) instead of 256 x 2 (16
-// warps, 128); for 34 <= K <= 48, 128 x 2 instead of 128 x 3 (168).  Which
-// build runs is chosen per (K, mode) from measurements (wave_lean, batch_lean).
+// Threads an SM holds (the register budget): 512 up to K = 32 columns per
+// thread (128 registers), 384 up to K = 48 (168), 256 above.  Register-lean
+// builds trade warps for registers per thread: 384 threads for 25 <= K <= 32 and
+// 256 for 34 <= K <= 48.  Which build runs is chosen per (K, mode) from
+// measurements (wave_lean).  The launch bound is one block of all of them, so the
+// host may launch them as one block that shares one profile, or as smaller ones
+// (wave_launch, batch_launch).
 constexpr int WAVE_LEAN_KMIN = 25, WAVE_LEAN_KMAX = 48;
 __host__ __device__ constexpr bool wave_has_lean(int K) { return K >= WAVE_LEAN_KMIN && K <= WAVE_LEAN_KMAX && K != 33; }
-__host__ __device__ constexpr int wave_threads_lean(int K, int mode, int lean) {
-  return (lean && wave_has_lean(K) && K <= 32) ? 128 : wave_block_threads(K, mode);
-}
-__host__ __device__ constexpr int wave_blocks_lean(int K, int mode, int lean) {
-  return (lean && wave_has_lean(K)) ? (K <= 32 ? 3 : 2) : wave_blocks_per_sm(K, mode);
+__host__ __device__ constexpr int wave_sm_threads(int K, int lean) {
+  return lean && wave_has_lean(K) ? (K <= 32 ? 384 : 256) : (K <= 32 ? 512 : K <= 48 ? 384 : 256);
 }
 // wave_kernel reads its parameters from a shared-memory copy for these
 // (K, mode, lean build) (see wave.cuh).  Measured on the protein search

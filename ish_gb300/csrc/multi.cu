@@ -212,15 +212,12 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
     const int lean = wave_lean(ctx, c.K, c.mode);
     c.fn = batch_fn(c.K, c.mode, c.layout, lean);
     if (!c.fn) return fail(ctx, ISH_EOVERFLOW, "no batch kernel for K=%d", c.K);
-    c.threads = wave_threads_lean(c.K, c.mode, lean);
-    const size_t save = c.mode == SW ? (size_t)c.threads * wave_save_words(c.K) * 4 : 0;
-    c.smem = c.prof_area + (size_t)c.threads * 4 + save;
-    CU(cudaFuncSetAttribute((const void *)c.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c.smem));
-    int per_sm = 0;
-    CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)c.fn, c.threads, c.smem));
-    if (per_sm < 1) return fail(ctx, ISH_EOVERFLOW, "batch kernel K=%d does not fit (smem %zu)", c.K, c.smem);
-    if (ctx->force_blocks) per_sm = std::min(per_sm, ctx->force_blocks);
-    c.grid = (uint32_t)(per_sm * ctx->num_sms);
+    BatchLaunch launch;
+    int rc = batch_launch(ctx, c.fn, c.K, c.mode, lean, c.prof_area, &launch);
+    if (rc) return rc;
+    c.threads = launch.threads;
+    c.smem = launch.smem;
+    c.grid = launch.grid;
 
     std::vector<WaveParams> params(c.members.size());
     std::vector<BatchTile> tiles;
@@ -534,12 +531,10 @@ int ish_gpu_autotune(ish_ctx *ctx, int32_t set_id, const int32_t *query_ids, uin
         // the layout rule's pick, and the 16/32-bit alternative to it (the
         // 32-bit profile saves an ALU instruction per column but can cost
         // occupancy)
-        const int pick = choose_layout(q.rows, g, k, mode);
+        const int pick = choose_layout(ctx, q.rows, g, k, mode);
         cands.push_back({g, k, pick, m});
         const int other = pick == PROF_S32 ? PROF_S16 : (pick == PROF_S16 ? PROF_S32 : -1);
-        if (other >= 0 &&
-            wave_smem((uint32_t)layout_bytes(other, q.rows, g, k), wave_block_threads(k, mode), g, k, mode) <= 227 * 1024)
-          cands.push_back({g, k, other, m});
+        if (other >= 0 && wave_fits(q, g, k, other)) cands.push_back({g, k, other, m});
       }
       cands.erase(std::remove_if(cands.begin(), cands.end(), [&](const Cand &c) { return c.model > 1.6 * best_model; }),
                   cands.end());

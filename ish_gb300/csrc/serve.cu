@@ -371,15 +371,10 @@ int step(Server &S, char *msg) {
         snprintf(msg, 256, "no batch kernel for K=%d", C.K);
         return ISH_EOVERFLOW;
       }
-      const int threads = wave_threads_lean(C.K, C.mode, lean);
-      const size_t save = C.mode == SW ? (size_t)threads * wave_save_words(C.K) * 4 : 0;
-      const size_t smem = C.prof_area + (size_t)threads * 4 + save;
-      SCU(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      int per_sm = 0;
-      SCU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void *)fn, threads, smem));
-      if (per_sm < 1) {
-        snprintf(msg, 256, "batch kernel K=%d does not fit (smem %zu)", C.K, smem);
-        return ISH_EOVERFLOW;
+      BatchLaunch launch;
+      if (int rc = batch_launch(S.ctx, fn, C.K, C.mode, lean, C.prof_area, &launch)) {
+        snprintf(msg, 256, "%s", ish_gpu_last_error(S.ctx));
+        return rc;
       }
       BatchParams b{};
       b.queries = S.step_params.as<const WaveParams>() + C.first;
@@ -390,7 +385,7 @@ int step(Server &S, char *msg) {
       b.step_cap = S.ctx->step_budget;
       cudaStream_t cs = c == 0 ? s : S.side[c - 1];
       if (c > 0) SCU(cudaStreamWaitEvent(cs, S.fork, 0));
-      fn<<<per_sm * S.ctx->num_sms, threads, smem, cs>>>(b);
+      fn<<<launch.grid, launch.threads, launch.smem, cs>>>(b);
       ++S.ctx->launches;
       SCU(cudaGetLastError());
       if (c > 0) {

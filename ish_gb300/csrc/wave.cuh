@@ -495,18 +495,35 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         // row -1: H(-1, c) is 0 in the padding and with a free query start,
         // -open - ext * q else; with its frame c * ext (column frame less one
         // row's) that is bias + c * ext, or one value for all of the query
-        const int h_query = p.bias + p.d * ext - p.open;
-        const bool qs = p.ends & 1;
+        if (MODE == SG) {
+          const bool qs = p.ends & 1;
+          const uint32_t step = qs ? (uint32_t)ext * 0x10001u : 0u;
+          const uint32_t h0 = (uint32_t)(qs ? p.bias + t * K * ext : p.bias + p.d * ext - p.open) * 0x10001u;
 #pragma unroll
-        for (int j = 0; j < K; ++j) {
-          const int c = t * K + j;
-          const uint32_t h0 = (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
-          H[j] = (MODE == SW) ? FLOOR : h0;
-          E[j] = (MODE == SW) ? FLOOR : h0 + EOPEN_SUM;  // row 0's frame is one ext above row -1's
-        }
-        {
-          const int c = t * K - 1;
-          prevH = (MODE == SW) ? FLOOR : (uint32_t)(!qs && c >= p.d ? h_query : p.bias + c * ext) * 0x10001u;
+          for (int j = 0; j < K; ++j) {
+            H[j] = h0 + (uint32_t)j * step;
+            E[j] = H[j] + EOPEN_SUM;  // row 0's frame is one ext above row -1's
+          }
+          prevH = h0 - step;
+          if (!qs && t * K <= p.d) {  // (the padding is this thread's, or ends at its left)
+#pragma unroll
+            for (int j = -1; j < K; ++j) {
+              const int c = t * K + j;
+              if (c < p.d) {
+                const uint32_t v = (uint32_t)(p.bias + c * ext) * 0x10001u;
+                if (j < 0) {
+                  prevH = v;
+                } else {
+                  H[j > 0 ? j : 0] = v;
+                  E[j > 0 ? j : 0] = v + EOPEN_SUM;
+                }
+              }
+            }
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < K; ++j) H[j] = E[j] = FLOOR;
+          prevH = FLOOR;
         }
         best = (MODE == SW) ? FLOOR : (t != G - 1 ? 0xffffffffu : 0u);
         left_best = FLOOR;
@@ -722,7 +739,7 @@ __device__ __forceinline__ void wave_rows_smem_params(const WaveParams &p, const
 // Shared memory of a block: the profile, then a slot word per thread, then
 // (local alignment) wave_save_words(K) save words per thread.
 template <int K, int MODE, int LAYOUT, int LEAN = 0>
-__global__ void __launch_bounds__(wave_threads_lean(K, MODE, LEAN), wave_blocks_lean(K, MODE, LEAN))
+__global__ void __launch_bounds__(wave_sm_threads(K, LEAN), 1)
     wave_kernel(const __grid_constant__ WaveParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   {
@@ -750,7 +767,7 @@ __global__ void __launch_bounds__(wave_threads_lean(K, MODE, LEAN), wave_blocks_
 // a profile reload happen only at a query switch, where the pairs left are the
 // shortest of the set.  Queries whose counter is already exhausted are skipped.
 template <int K, int MODE, int LAYOUT, int LEAN = 0>
-__global__ void __launch_bounds__(wave_threads_lean(K, MODE, LEAN), wave_blocks_lean(K, MODE, LEAN))
+__global__ void __launch_bounds__(wave_sm_threads(K, LEAN), 1)
     batch_kernel(const __grid_constant__ BatchParams b) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ WaveParams sp;

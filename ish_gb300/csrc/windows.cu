@@ -123,8 +123,7 @@ uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int 
   const int lean = wave_lean(ctx, K, mode);
   // groups in flight and the rows each would score on average (two records
   // per pair share their rows)
-  const uint64_t groups =
-      (uint64_t)ctx->num_sms * wave_blocks_lean(K, mode, lean) * (wave_threads_lean(K, mode, lean) / G);
+  const uint64_t groups = (uint64_t)ctx->num_sms * wave_sm_threads(K, lean) / G;
   const uint64_t avg_rows = rs.total / 2 / std::max<uint64_t>(groups, 1);
   if (rs.max_len * 4 <= avg_rows * ISH_WINDOW_QUARTERS) return 0;
   // rows in records longer than 2^(i/8) (all of them where the set has no
@@ -146,9 +145,9 @@ uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int 
     const double cut = above[bin_of(w + O)];  // rows that are cut into windows
     const double work = (rs.total + cut * (double)O / w) / 2;
     const double pairs = std::ceil((cut / w + rs.n) / 2);
-    const double full = row_clocks(ctx, mode, K, warps);
+    const double full = row_clocks(ctx, mode, K, G, warps);
     const double t = 2 * pairs >= groups ? work / groups * full + 0.4 * (w + O) * full
-                                         : 1.15 * (w + O) * row_clocks(ctx, mode, K, pairs * G / 32);
+                                         : 1.15 * (w + O) * row_clocks(ctx, mode, K, G, pairs * G / 32);
     if (t < best_t) {
       best_t = t;
       best = ((uint64_t)w + 15) & ~15ull;
