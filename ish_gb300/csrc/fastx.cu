@@ -115,38 +115,6 @@ __device__ uint32_t block_excl_maps(uint32_t m, uint32_t *total) {
   return map_then(wp, excl);
 }
 
-// First '>' or '@' of every line (the header a SEEK line starts), by
-// atomicMin; hc is preset to all ones.  block_offsets: newlines before each
-// LINE_TILE-byte tile (exclusive scan of k_count_newlines).
-__global__ void __launch_bounds__(1024) k_fx_header_chars(const uint8_t *text, uint64_t bytes,
-                                                          const uint32_t *block_offsets, unsigned long long *hc) {
-  __shared__ uint32_t wsum[32];
-  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint64_t w0 = (uint64_t)blockIdx.x * LINE_TILE + (uint64_t)wid * LINE_WARP;
-  uint32_t run = warp_newline_base(text, bytes, block_offsets, w0, lane, wid, wsum);
-  for (uint32_t k = 0; k < LINE_WARP; k += 128) {
-    const uint64_t i = w0 + k + 4 * lane;
-    uint32_t nl = 0, h = 0;
-    if (i < bytes) {
-      nl = byte_bits(text, bytes, i, '\n');
-      h = byte_bits(text, bytes, i, '>') | byte_bits(text, bytes, i, '@');
-    }
-    const uint32_t cnt = __popc(nl);
-    uint32_t incl = cnt;
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= (uint32_t)o) incl += y;
-    }
-    const uint32_t before = run + incl - cnt;  // newlines before this lane's 4 bytes
-    while (h) {
-      const uint32_t bit = (uint32_t)(__ffs(h) - 1);
-      atomicMin(hc + before + __popc(nl & ((1u << bit) - 1u)), (unsigned long long)(i + bit));
-      h &= h - 1;
-    }
-    run += __shfl_sync(0xffffffffu, incl, 31);
-  }
-}
-
 // Composition of the maps of each tile of FX_TILE lines.
 __global__ void k_fx_tile_maps(const uint8_t *text, uint64_t bytes, const uint64_t *nl, uint32_t n_nl, uint32_t n,
                                const unsigned long long *hc, uint32_t *tile_map) {
@@ -239,11 +207,14 @@ __global__ void k_fx_roles(const uint8_t *text, uint64_t bytes, const uint64_t *
   }
 }
 
-// Per record: sequence offset, name and quality bounds, FASTQ flags.
+// Per record: sequence offset, name and quality bounds, FASTQ flags, and where
+// its sequence line lies in the text.  totals[3] is raised when some record's
+// sequence is not one line of the text (several lines, or empty ones).
 // rec_excl: headers before each line; pos: sequence bytes before each line.
 __global__ void k_fx_records(const uint8_t *text, uint64_t bytes, const uint64_t *nl, uint32_t n_nl, uint32_t n,
                              const uint8_t *role, const uint64_t *rec_excl, const uint64_t *pos, uint64_t *rec_off,
-                             uint64_t *bounds, uint32_t *flags, const uint64_t *src) {
+                             uint64_t *bounds, uint32_t *flags, const uint64_t *src, const uint64_t *len,
+                             uint64_t *seq_start, uint64_t *seq_end, uint64_t *totals) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const uint8_t r = role[i];
     if (r == R_HEADER) {
@@ -271,6 +242,12 @@ __global__ void k_fx_records(const uint8_t *text, uint64_t bytes, const uint64_t
       bounds[4 * rec + 2] = L.s;
       bounds[4 * rec + 3] = qe;
       atomicOr(flags + rec, F_QUAL | (i + 1 < n ? F_QUAL_MORE : 0u));
+    } else if (r == R_SEQ && role[i - 1] == R_HEADER) {
+      const uint64_t rec = rec_excl[i] - 1;
+      seq_start[rec] = src[i];
+      seq_end[rec] = src[i] + len[i];
+    } else if (r == R_SEQ || r == R_EMPTY || r == R_ABS) {
+      totals[3] = 1;
     }
   }
 }
@@ -279,8 +256,9 @@ __global__ void k_fx_records(const uint8_t *text, uint64_t bytes, const uint64_t
 // a quality of the wrong length or a missing one), as 2 * record + (1 if the
 // cause is a quality continued on the next line, which the device does not
 // split); records from there on are not part of the set.
-__global__ void k_fx_check(uint32_t nrec, const uint64_t *rec_off, const uint64_t *bounds, const uint32_t *flags,
-                           unsigned long long *first_bad) {
+__global__ void k_fx_check(const uint64_t *totals, const uint64_t *rec_off, const uint64_t *bounds,
+                           const uint32_t *flags, unsigned long long *first_bad) {
+  const uint32_t nrec = (uint32_t)totals[0];
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < nrec; r += gridDim.x * blockDim.x) {
     const uint64_t seqlen = rec_off[r + 1] - rec_off[r];
     const uint32_t f = flags[r];
@@ -296,6 +274,13 @@ __global__ void k_fx_check(uint32_t nrec, const uint64_t *rec_off, const uint64_
     }
     if (stop || unsupported) atomicMin(first_bad, 2ull * r + (unsupported ? 1ull : 0ull));
   }
+}
+
+// totals[4], [5]: the records before the first stop and their sequence bytes.
+__global__ void k_fx_keep(const uint64_t *rec_off, uint64_t *totals) {
+  const uint64_t keep = totals[2] == ~0ull ? totals[0] : min(totals[0], totals[2] >> 1);
+  totals[4] = keep;
+  totals[5] = rec_off[keep];
 }
 
 // Sequence bytes of every line into their records' places: one warp per
@@ -325,6 +310,8 @@ __global__ void k_fx_totals(uint32_t n, const uint64_t *len, const uint64_t *pos
   rec_off[nrec] = seq;
   totals[0] = nrec;
   totals[1] = seq;
+  totals[2] = ~0ull;  // the first stop (k_fx_check)
+  totals[3] = 0;      // sequences of several lines (k_fx_records)
 }
 
 }  // namespace
@@ -386,9 +373,10 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   ++ctx->launches;
   k_scan_counts<<<1, 1024, 0, s>>>(ctx->block_counts.as<uint32_t>(), btiles, ctx->nhits.as<uint32_t>());
   ++ctx->launches;
-  uint32_t n_nl = 0;
-  CU(cudaMemcpyAsync(&n_nl, ctx->nhits.p, 4, cudaMemcpyDeviceToHost, s));
+  uint32_t *hs = reinterpret_cast<uint32_t *>(ctx->h_small);
+  CU(cudaMemcpyAsync(hs, ctx->nhits.p, 4, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
+  const uint32_t n_nl = hs[0];
   const uint64_t lines64 = (uint64_t)n_nl + (text[bytes - 1] != '\n' ? 1 : 0);
   if (lines64 >= 0xfffff000ull) return fail(ctx, ISH_EINVAL, "too many lines (%llu)", (unsigned long long)lines64);
   const uint32_t n = (uint32_t)lines64;
@@ -404,11 +392,9 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   CU(fx.tiles.ensure((size_t)ltiles * 5 + 16));
   CU(fx.scan.ensure(scan_u64_scratch(n)));
   CU(fx.totals.ensure(64));
-  k_write_newlines<<<btiles, 1024, 0, s>>>(dtext, bytes, ctx->block_counts.as<uint32_t>(), ctx->nl_pos.as<uint64_t>());
-  ++ctx->launches;
-  CU(cudaMemsetAsync(fx.hc.p, 0xff, (size_t)n * 8, s));
-  k_fx_header_chars<<<btiles, 1024, 0, s>>>(dtext, bytes, ctx->block_counts.as<uint32_t>(),
-                                            fx.hc.as<unsigned long long>());
+  CU(cudaMemsetAsync(fx.hc.p, 0xff, (size_t)n * 8 + 8, s));
+  write_newlines_fn(true)<<<btiles, 1024, 0, s>>>(dtext, bytes, ctx->block_counts.as<uint32_t>(),
+                                                  ctx->nl_pos.as<uint64_t>(), fx.hc.as<unsigned long long>());
   ++ctx->launches;
   // ---- the reader's state at every line ----
   const uint64_t *nl = ctx->nl_pos.as<uint64_t>();
@@ -431,39 +417,36 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   CU(fx.rec_off.ensure((size_t)(n + 2) * 8));
   CU(fx.bounds.ensure((size_t)(n + 1) * 32));
   CU(fx.flags.ensure((size_t)(n + 1) * 4));
+  CU(fx.seq_start.ensure((size_t)(n + 1) * 8));
+  CU(fx.seq_end.ensure((size_t)(n + 1) * 8));
   k_fx_totals<<<1, 1, 0, s>>>(n, fx.len.as<uint64_t>(), fx.pos.as<uint64_t>(), fx.hdr.as<uint64_t>(),
                               fx.rec.as<uint64_t>(), fx.rec_off.as<uint64_t>(), fx.totals.as<uint64_t>());
   ++ctx->launches;
   CU(cudaMemsetAsync(fx.flags.p, 0, (size_t)(n + 1) * 4, s));
   CU(cudaMemsetAsync(fx.bounds.p, 0, (size_t)(n + 1) * 32, s));
-  CU(cudaMemsetAsync(fx.totals.as<uint64_t>() + 2, 0xff, 8, s));
   const uint32_t gb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256), (uint32_t)ctx->num_sms * 16));
   k_fx_records<<<gb, 256, 0, s>>>(dtext, bytes, nl, n_nl, n, fx.role.as<uint8_t>(), fx.rec.as<uint64_t>(),
                                   fx.pos.as<uint64_t>(), fx.rec_off.as<uint64_t>(), fx.bounds.as<uint64_t>(),
-                                  fx.flags.as<uint32_t>(), fx.src.as<uint64_t>());
+                                  fx.flags.as<uint32_t>(), fx.src.as<uint64_t>(), fx.len.as<uint64_t>(),
+                                  fx.seq_start.as<uint64_t>(), fx.seq_end.as<uint64_t>(), fx.totals.as<uint64_t>());
   ++ctx->launches;
-  uint64_t tot[3] = {0, 0, 0};
-  CU(cudaMemcpyAsync(tot, fx.totals.p, 16, cudaMemcpyDeviceToHost, s));
+  k_fx_check<<<gb, 256, 0, s>>>(fx.totals.as<uint64_t>(), fx.rec_off.as<uint64_t>(), fx.bounds.as<uint64_t>(),
+                                fx.flags.as<uint32_t>(),
+                                reinterpret_cast<unsigned long long *>(fx.totals.as<uint64_t>() + 2));
+  ++ctx->launches;
+  k_fx_keep<<<1, 1, 0, s>>>(fx.rec_off.as<uint64_t>(), fx.totals.as<uint64_t>());
+  ++ctx->launches;
+  CU(cudaGetLastError());
+  const uint64_t *tot = ctx->h_small;  // pinned
+  CU(cudaMemcpyAsync(ctx->h_small, fx.totals.p, 48, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
-  const uint64_t nrec = tot[0], seq_bytes = tot[1];
-  if (nrec > 0) {
-    k_fx_check<<<std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(nrec, 256), (uint32_t)ctx->num_sms * 16)), 256, 0,
-                 s>>>((uint32_t)nrec, fx.rec_off.as<uint64_t>(), fx.bounds.as<uint64_t>(), fx.flags.as<uint32_t>(),
-                      reinterpret_cast<unsigned long long *>(fx.totals.as<uint64_t>() + 2));
-    ++ctx->launches;
-  }
-  CU(cudaMemcpyAsync(&tot[2], fx.totals.as<uint64_t>() + 2, 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  uint64_t keep = nrec;
-  if (tot[2] != ~0ull) {
-    const uint64_t r = tot[2] >> 1;
-    if (tot[2] & 1)
-      return fail(ctx, ISH_EINVAL,
-                  "FASTQ record %llu: its quality continues on the next line (one quality line per record is "
-                  "split on the device)",
-                  (unsigned long long)r);
-    keep = std::min(keep, r);
-  }
+  const uint64_t seq_bytes = tot[1], first_stop = tot[2], keep = tot[4], used = tot[5];
+  const bool one_line = tot[3] == 0;
+  if (first_stop != ~0ull && (first_stop & 1))
+    return fail(ctx, ISH_EINVAL,
+                "FASTQ record %llu: its quality continues on the next line (one quality line per record is "
+                "split on the device)",
+                (unsigned long long)(first_stop >> 1));
   if (keep > 0xffffffffull) return fail(ctx, ISH_EINVAL, "too many records (%llu)", (unsigned long long)keep);
   const uint32_t nr = (uint32_t)keep;
   if (bounds_out) {
@@ -471,25 +454,28 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
                                      (unsigned long long)bounds_cap);
     if (nr) CU(cudaMemcpyAsync(bounds_out, fx.bounds.p, (size_t)nr * 32, cudaMemcpyDeviceToHost, s));
   }
+  rs.total = used;
+  *n_out = nr;
+  if (nr == 0) {
+    CU(cudaStreamSynchronize(s));
+    return ISH_OK;
+  }
+  if (one_line) {
+    // every sequence is one line (FASTQ, unwrapped FASTA): packed from the text
+    // where it lies
+    std::swap(ctx->off_in, fx.seq_start);
+    return pack_set(ctx, nr, bytes, fx.seq_end.as<uint64_t>(), enc, rs);
+  }
   // ---- the kept records' sequences, contiguous, then the common packing ----
-  uint64_t used = 0;
-  if (nr) CU(cudaMemcpyAsync(&used, fx.rec_off.as<uint64_t>() + nr, 8, cudaMemcpyDeviceToHost, s));
   CU(fx.seq.ensure(seq_bytes + 32));
   const uint32_t gw = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div((uint64_t)n * 32, 256), (uint32_t)ctx->num_sms * 32));
   k_fx_gather<<<gw, 256, 0, s>>>(dtext, n, fx.role.as<uint8_t>(), fx.len.as<uint64_t>(), fx.src.as<uint64_t>(),
                                  fx.pos.as<uint64_t>(), fx.seq.as<uint8_t>());
   ++ctx->launches;
   CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(s));
-  CU(ctx->off_in.ensure((size_t)(nr + 1) * 8));
-  if (nr) {
-    CU(cudaMemcpyAsync(ctx->raw.p, fx.seq.p, used, cudaMemcpyDeviceToDevice, s));
-    CU(cudaMemcpyAsync(ctx->off_in.p, fx.rec_off.p, (size_t)nr * 8, cudaMemcpyDeviceToDevice, s));
-  }
-  rs.total = used;
-  *n_out = nr;
-  if (nr == 0) return ISH_OK;
-  return pack_set(ctx, nr, used, fx.rec_off.as<uint64_t>() + 1, enc, rs);
+  std::swap(ctx->raw, fx.seq);
+  std::swap(ctx->off_in, fx.rec_off);
+  return pack_set(ctx, nr, used, nullptr, enc, rs);
 }
 
 }  // namespace host

@@ -67,6 +67,7 @@ struct Query {
   std::vector<int8_t> M;
   std::vector<uint8_t> q;
   int mmin = 0, mmax = 0;
+  long long col_max_sum = 0, col_min_sum = 0;  // sums of the columns' largest (smallest) scores, at least (most) 0 each
   int neg_limit = 0;
   // Profile rows: codes whose matrix rows agree on every query column share
   // one row (for ascii, every byte that is not in the query); rowmap[c] is the
@@ -97,6 +98,8 @@ inline void clone_params(const Query &src, Query &dst) {
   dst.q = src.q;
   dst.mmin = src.mmin;
   dst.mmax = src.mmax;
+  dst.col_max_sum = src.col_max_sum;
+  dst.col_min_sum = src.col_min_sum;
   dst.neg_limit = src.neg_limit;
   dst.rows = src.rows;
   dst.rowmap = src.rowmap;
@@ -168,9 +171,10 @@ struct ExactRes {
 
 // Scratch of the FASTA/FASTQ splitter (fastx.cu): per line, per record.
 struct FastxScratch {
-  DevBuf hc, len, src, hdr, pos, rec, role, tiles, scan, totals, rec_off, bounds, flags, seq;
+  DevBuf hc, len, src, hdr, pos, rec, role, tiles, scan, totals, rec_off, bounds, flags, seq, seq_start, seq_end;
   void release() {
-    DevBuf *b[] = {&hc, &len, &src, &hdr, &pos, &rec, &role, &tiles, &scan, &totals, &rec_off, &bounds, &flags, &seq};
+    DevBuf *b[] = {&hc,     &len,     &src,    &hdr,   &pos, &rec,       &role,    &tiles,
+                   &scan,   &totals,  &rec_off, &bounds, &flags, &seq, &seq_start, &seq_end};
     for (DevBuf *x : b) x->release();
   }
 };

@@ -718,8 +718,8 @@ int load_lines(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   CU(ctx->nl_pos.ensure((size_t)n_nl * 8 + 8));
   CU(ctx->off_in.ensure((size_t)(n + 1) * 8));
   CU(ctx->line_end.ensure((size_t)n * 8 + 8));
-  k_write_newlines<<<tiles, 1024, 0, s>>>(ctx->raw.as<uint8_t>(), bytes, ctx->block_counts.as<uint32_t>(),
-                                          ctx->nl_pos.as<uint64_t>());
+  write_newlines_fn(false)<<<tiles, 1024, 0, s>>>(ctx->raw.as<uint8_t>(), bytes, ctx->block_counts.as<uint32_t>(),
+                                                  ctx->nl_pos.as<uint64_t>(), nullptr);
   ++ctx->launches;
   CU(cudaMemsetAsync(ctx->nhits.p, 0, 16, s));
   k_line_bounds<<<std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256), (uint32_t)ctx->num_sms * 16)), 256, 0,
@@ -727,12 +727,15 @@ int load_lines(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
                        ctx->line_end.as<uint64_t>(), reinterpret_cast<unsigned long long *>(ctx->nhits.p));
   ++ctx->launches;
   CU(cudaGetLastError());
-  // residues: the text minus the newlines and the dropped carriage returns
+  // residues: the text minus the newlines and the dropped carriage returns;
+  // the exact count comes back with the set's summary, packing only needs a
+  // bound
   CU(cudaMemcpyAsync(ctx->h_small, ctx->nhits.p, 8, cudaMemcpyDeviceToHost, s));
-  CU(cudaStreamSynchronize(s));
-  rs.total = ctx->h_small[0];
+  rs.total = bytes - n_nl;
   *n_out = n;
-  return pack_set(ctx, n, bytes, ctx->line_end.as<uint64_t>(), enc, rs);
+  const int rc = pack_set(ctx, n, bytes, ctx->line_end.as<uint64_t>(), enc, rs);
+  if (!rc) rs.total = ctx->h_small[0];
+  return rc;
 }
 
 // Number of records (a prefix of the descending order) whose length bucket
@@ -1271,6 +1274,18 @@ int ish_gpu_set_query(ish_ctx *ctx, const uint8_t *enc_query, uint32_t qlen, int
     q.mmax = std::max<int>(q.mmax, v);
   }
   q.neg_limit = neg_limit_of(q.open, q.mmin);
+  {
+    std::vector<int> hi(alphabet, 0), lo(alphabet, 0);  // per query code, over the record codes
+    for (uint32_t c = 0; c < alphabet; ++c)
+      for (uint32_t j = 0; j < alphabet; ++j) {
+        hi[j] = std::max<int>(hi[j], q.M[(size_t)c * alphabet + j]);
+        lo[j] = std::min<int>(lo[j], q.M[(size_t)c * alphabet + j]);
+      }
+    for (uint8_t c : q.q) {
+      q.col_max_sum += hi[c];
+      q.col_min_sum += lo[c];
+    }
+  }
   compute_rows(q);
   cudaSetDevice(ctx->device);
   const int32_t id = ctx->next_query++;

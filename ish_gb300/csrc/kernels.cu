@@ -376,7 +376,14 @@ __global__ void __launch_bounds__(256, 3) k_pack(const uint8_t *src, uint64_t sr
 __global__ void __launch_bounds__(1024) k_count_newlines(const uint8_t *text, uint64_t bytes, uint32_t *block_counts) {
   __shared__ uint32_t wsum[32];
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const uint32_t c = warp_newlines(text, bytes, (uint64_t)blockIdx.x * LINE_TILE + (uint64_t)wid * LINE_WARP, lane);
+  const uint64_t w0 = (uint64_t)blockIdx.x * LINE_TILE + (uint64_t)wid * LINE_WARP;
+  uint4 w[LINE_STEPS];
+  load_segment(text, bytes, w0, lane, w);
+  uint32_t c = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < LINE_STEPS; ++k)
+    c += __popc(byte_bits(w[k], 0x0a0a0a0au) & inside_bits(bytes, w0 + k * 512 + lane * 16));
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
   if (lane == 0) wsum[wid] = c;
   __syncthreads();
   if (wid == 0) {
@@ -387,29 +394,76 @@ __global__ void __launch_bounds__(1024) k_count_newlines(const uint8_t *text, ui
 }
 
 // Positions of the newlines, in order (block_offsets: exclusive scan of the
-// per-block counts).
+// per-block counts), and with HEADERS the first '>' or '@' of every line.  A
+// line's header characters after the first are dropped inside the warp, by the
+// ballots of the lanes between them and the line's start, so that a quality
+// line full of '@' costs one atomic per warp segment it spans.  Measured on
+// 104 MB of FASTQ (1 M lines): 127 + 159 us as two kernels of 4-byte loads that
+// read the text twice each, 75 us as this one; counting 63 -> 21 us (4.9 TB/s).
+template <bool HEADERS>
 __global__ void __launch_bounds__(1024) k_write_newlines(const uint8_t *text, uint64_t bytes,
-                                                         const uint32_t *block_offsets, uint64_t *pos) {
+                                                         const uint32_t *block_offsets, uint64_t *pos,
+                                                         unsigned long long *hc) {
   __shared__ uint32_t wsum[32];
+  const unsigned FULL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint64_t w0 = (uint64_t)blockIdx.x * LINE_TILE + (uint64_t)wid * LINE_WARP;
-  uint32_t run = warp_newline_base(text, bytes, block_offsets, w0, lane, wid, wsum);
-  for (uint32_t k = 0; k < LINE_WARP; k += 128) {
-    const uint64_t i = w0 + k + 4 * lane;
-    uint32_t m = i < bytes ? byte_bits(text, bytes, i, '\n') : 0u;
-    const uint32_t cnt = __popc(m);
+  uint4 w[LINE_STEPS];
+  load_segment(text, bytes, w0, lane, w);
+  uint32_t nl[LINE_STEPS], c = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < LINE_STEPS; ++k) {
+    nl[k] = byte_bits(w[k], 0x0a0a0a0au) & inside_bits(bytes, w0 + k * 512 + lane * 16);
+    c += __popc(nl[k]);
+  }
+  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(FULL, c, o);
+  if (lane == 0) wsum[wid] = c;
+  __syncthreads();
+  uint32_t x = wsum[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(FULL, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  uint32_t run = block_offsets[blockIdx.x] + __shfl_sync(FULL, x, wid) - c;  // newlines before the warp's segment
+  bool carry = false;  // the line open at the step's start has a header character in this segment
+#pragma unroll
+  for (uint32_t k = 0; k < LINE_STEPS; ++k) {
+    const uint64_t i = w0 + k * 512 + lane * 16;
+    const uint32_t cnt = __popc(nl[k]);
     uint32_t incl = cnt;
     for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      const uint32_t y = __shfl_up_sync(FULL, incl, o);
       if (lane >= (uint32_t)o) incl += y;
     }
-    uint32_t p = run + incl - cnt;
-    while (m) {
-      pos[p++] = i + (uint32_t)(__ffs(m) - 1);
-      m &= m - 1;
+    const uint32_t before = run + incl - cnt;
+    if (HEADERS) {
+      const uint32_t h = (byte_bits(w[k], 0x3e3e3e3eu) | byte_bits(w[k], 0x40404040u)) & inside_bits(bytes, i);
+      // the lane's bytes of the line open at its first byte, and of the line
+      // open at its last
+      const uint32_t first = nl[k] ? h & ((nl[k] & (0u - nl[k])) - 1u) : h;
+      const uint32_t last = nl[k] ? h & ~((2u << (31 - __clz(nl[k]))) - 1u) : h;
+      const uint32_t has_nl = __ballot_sync(FULL, nl[k] != 0), has_h = __ballot_sync(FULL, last != 0);
+      const uint32_t below = (1u << lane) - 1u, breaks = has_nl & below;
+      const uint32_t same = breaks ? below & ~((1u << (31 - __clz(breaks))) - 1u) : below;  // lanes holding this line
+      if (first && !(has_h & same) && (breaks || !carry)) atomicMin(hc + before, (unsigned long long)(i + __ffs(first) - 1));
+      // lines that start inside the lane's bytes
+      uint32_t line = before;
+      for (uint32_t rest = nl[k]; rest;) {
+        const uint32_t upto = rest & (0u - rest);  // this newline's bit
+        rest ^= upto;
+        ++line;
+        const uint32_t seg = h & ~(upto | (upto - 1u)) & (rest ? (rest & (0u - rest)) - 1u : 0xffffu);
+        if (seg) atomicMin(hc + line, (unsigned long long)(i + __ffs(seg) - 1));
+      }
+      carry = has_nl ? (has_h & ~((1u << (31 - __clz(has_nl))) - 1u)) != 0 : carry || has_h;
     }
-    run += __shfl_sync(0xffffffffu, incl, 31);
+    uint32_t p = before;
+    for (uint32_t m = nl[k]; m; m &= m - 1) pos[p++] = i + (uint32_t)(__ffs(m) - 1);
+    run += __shfl_sync(FULL, incl, 31);
   }
+}
+NewlinesFn write_newlines_fn(bool headers) {
+  return headers ? (NewlinesFn)k_write_newlines<true> : (NewlinesFn)k_write_newlines<false>;
 }
 
 // Line i's bounds; *total accumulates the residues of all lines.

@@ -26,7 +26,11 @@ __global__ void k_pack(const uint8_t *src, uint64_t src_bytes, const uint64_t *o
                        const uint64_t *poff, uint32_t n, const uint32_t *len_s, const uint32_t *orig_s,
                        uint32_t *long_counter, const uint8_t *enc, uint8_t *dst, uint32_t *max_code, uint32_t gw);
 __global__ void k_count_newlines(const uint8_t *text, uint64_t bytes, uint32_t *block_counts);
-__global__ void k_write_newlines(const uint8_t *text, uint64_t bytes, const uint32_t *block_offsets, uint64_t *pos);
+// k_write_newlines<headers>: with headers, also the first '>' or '@' of every
+// line (hc, preset to all ones)
+typedef void (*NewlinesFn)(const uint8_t *text, uint64_t bytes, const uint32_t *block_offsets, uint64_t *pos,
+                           unsigned long long *hc);
+NewlinesFn write_newlines_fn(bool headers);
 __global__ void k_line_bounds(const uint8_t *text, uint64_t bytes, const uint64_t *nl, uint32_t n_nl, uint32_t n_lines,
                               uint64_t *start, uint64_t *end, unsigned long long *total);
 __global__ void k_scan64_block(const uint64_t *in, uint64_t *out, uint32_t n, uint64_t *block_sums);
@@ -106,49 +110,37 @@ BatchFn batch_fn(int K, int mode, int layout, int lean = 0);  // batch_kernel<K,
 
 // The splitting kernels take the text in tiles of LINE_TILE bytes per
 // 1024-thread block; warp w of a block covers LINE_WARP consecutive bytes of
-// its tile, 128 per step and 4 per lane, so no block-wide barrier runs inside
-// a loop.  The text lies in a buffer with at least 3 bytes of slack past its
-// end (every 4-byte word that starts inside it can be loaded) and starts
-// 4-byte aligned.
-constexpr uint32_t LINE_WARP = LINE_TILE / 32;
+// its tile, 512 per step and 16 per lane, all of them loaded before any is
+// looked at (they are bound by the loads in flight), and no block-wide barrier
+// runs inside a loop.  The text lies in a buffer with at least 15 bytes of slack
+// past its end (every 16-byte word that starts inside it can be loaded) and
+// starts 16-byte aligned.
+constexpr uint32_t LINE_WARP = LINE_TILE / 32, LINE_STEPS = LINE_WARP / 512;
 
-// Bit k set where byte k of the 4 at text[i] (i < bytes, i % 4 == 0) is c and
-// lies inside the text.
-__device__ __forceinline__ uint32_t byte_bits(const uint8_t *text, uint64_t bytes, uint64_t i, uint32_t c) {
-  const uint32_t w = *reinterpret_cast<const uint32_t *>(text + i);
+// Bit k set where byte k of the 16 in w is c (four times in c4).
+__device__ __forceinline__ uint32_t byte_bits(const uint4 &w, uint32_t c4) {
+  const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
   uint32_t m = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) m |= (uint32_t)(((w >> (8 * k)) & 0xffu) == c) << k;
-  const uint64_t left = bytes - i;
-  return left >= 4 ? m : m & ((1u << left) - 1u);
-}
-
-// Newlines of the warp's segment starting at byte w0 (every lane gets the count).
-__device__ __forceinline__ uint32_t warp_newlines(const uint8_t *text, uint64_t bytes, uint64_t w0, uint32_t lane) {
-  uint32_t c = 0;
-#pragma unroll 4
-  for (uint32_t k = 0; k < LINE_WARP; k += 128) {
-    const uint64_t i = w0 + k + 4 * lane;
-    if (i < bytes) c += __popc(byte_bits(text, bytes, i, '\n'));
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t t = ww[k] ^ c4;  // a zero byte where equal
+    const uint32_t z = ~(((t & 0x7f7f7f7fu) + 0x7f7f7f7fu) | t) & 0x80808080u;
+    m |= (((z >> 7) * 0x01020408u) >> 24 & 0xfu) << (4 * k);  // bits 0, 8, 16, 24 to 0..3
   }
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  return c;
+  return m;
 }
-
-// Newlines before each warp's segment: block_offsets (exclusive scan of the
-// per-tile counts) plus the tile's earlier warps.
-__device__ __forceinline__ uint32_t warp_newline_base(const uint8_t *text, uint64_t bytes,
-                                                      const uint32_t *block_offsets, uint64_t w0, uint32_t lane,
-                                                      uint32_t wid, uint32_t *wsum) {
-  const uint32_t c = warp_newlines(text, bytes, w0, lane);
-  if (lane == 0) wsum[wid] = c;
-  __syncthreads();
-  uint32_t x = wsum[lane];
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= (uint32_t)o) x += y;
+// The bits of the 16 bytes from byte i that lie inside the text.
+__device__ __forceinline__ uint32_t inside_bits(uint64_t bytes, uint64_t i) {
+  return i >= bytes ? 0u : bytes - i >= 16 ? 0xffffu : (1u << (uint32_t)(bytes - i)) - 1u;
+}
+// This lane's words of the warp's segment starting at byte w0 (zero past the text).
+__device__ __forceinline__ void load_segment(const uint8_t *text, uint64_t bytes, uint64_t w0, uint32_t lane,
+                                             uint4 (&w)[LINE_STEPS]) {
+#pragma unroll
+  for (uint32_t k = 0; k < LINE_STEPS; ++k) {
+    const uint64_t i = w0 + k * 512 + lane * 16;
+    w[k] = i < bytes ? __ldg(reinterpret_cast<const uint4 *>(text + i)) : make_uint4(0, 0, 0, 0);
   }
-  return block_offsets[blockIdx.x] + __shfl_sync(0xffffffffu, x, wid) - c;
 }
 
 }  // namespace ish

@@ -194,3 +194,36 @@ def test_packing_round_trip_short_and_long_records(ctx):
     ctx.records_free(sid)
     for i, r in enumerate(recs):
         assert np.array_equal(codes[int(got[i]):int(got[i + 1])], r), ("raw", i, len(r))
+
+
+@pytest.mark.parametrize("tail", [0, 1, 15, 16, 17, 511, 2047])
+def test_texts_whose_records_outnumber_the_sampled_lines(tail):
+    # long lines where the text is sampled, and then dense two-line records:
+    # the room for the bounds is first estimated too small; the text ends at
+    # every place of a 16-byte load
+    long_lines = b"".join(b">long\n" + b"A" * 199_990 + b"\n" for _ in range(40))
+    text = long_lines + b"".join(b">%d\nACGTN\n" % i for i in range(60_000)) + b">end\nAC" + b"G" * tail
+    with native.Context(0) as c:
+        sid, n, bounds = c.records_load_fastx(text, 1)
+        assert n == 60_041 and bounds.shape == (n, 4)
+        names = [text[int(a):int(b)] for a, b in bounds[[0, 39, 40, 41, n - 2, n - 1], :2]]
+        assert names == [b"long", b"long", b"0", b"1", b"59999", b"end"]
+        codes, off = c.records_get(sid, n - 2, 2)
+        assert codes.tolist() == [0, 1, 2, 3, 4, 0, 1] + [2] * tail and off.tolist() == [0, 5, 7 + tail]
+
+
+@pytest.mark.parametrize("line", [60, 61, 4096])
+def test_wrapped_and_unwrapped_sequences_pack_alike(line):
+    # one sequence line per record (packed from the text) and the same
+    # sequences wrapped (gathered first)
+    rng = np.random.default_rng(line)
+    seqs = [bytes(rng.choice(np.frombuffer(b"ACGTN", np.uint8), int(k))) for k in rng.integers(1, 400, 700)]
+    whole = b"".join(b">r\n" + s + b"\n" for s in seqs)
+    wrapped = b"".join(b">r\n" + b"".join(s[i:i + line] + b"\r\n" for i in range(0, len(s), line)) for s in seqs)
+    with native.Context(0) as c:
+        got = []
+        for text in (whole, wrapped, b"@" + whole.replace(b">r\n", b"@r\n", 1)[1:]):
+            sid, n, _ = c.records_load_fastx(text, 1)
+            assert n == len(seqs) and c.records_info(sid)[1] == sum(map(len, seqs))
+            got.append([a.tolist() for a in c.records_get(sid)])
+        assert got[0] == got[1] == got[2]
