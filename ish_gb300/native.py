@@ -136,6 +136,17 @@ def pack_records(records):
     return buf, off
 
 
+def _line_room(buf: np.ndarray) -> int:
+    """Lines to expect in a text: exact for short ones, else a quarter more
+    than 64 evenly spaced samples of 1 KB suggest."""
+    n = len(buf)
+    if n <= 1 << 17:
+        return int(np.count_nonzero(buf == 10)) + 1
+    at = np.linspace(0, n - 1024, 64).astype(np.int64)
+    seen = sum(int(np.count_nonzero(buf[i:i + 1024] == 10)) for i in at)
+    return int(1.25 * n * (seen / 65536.0)) + 4096
+
+
 class Context:
     """One engine context on one CUDA device (one per host thread)."""
 
@@ -280,13 +291,22 @@ class Context:
             np.ascontiguousarray(text, np.uint8)
         sid = C.c_int32()
         n = C.c_uint32()
-        # every record needs a header line: at most one record per newline + 1
-        cap = int(np.count_nonzero(buf == 10)) + 1 if bounds else 0
-        bnd = np.zeros((cap, 4), np.uint64) if bounds else None
-        self._check(self._L.ish_gpu_records_load_fastx(
-            self._h, _p(buf, C.c_uint8) if len(buf) else None, len(buf), matrix_kind, C.byref(sid), C.byref(n),
-            _p(bnd, C.c_uint64) if bounds else None, cap))
-        return sid.value, n.value, (bnd[:n.value].copy() if bounds else None)
+        # every record needs a header line: at most one record per newline + 1.
+        # Counting them took longer than the whole load, so the room is
+        # estimated from a sample, and counted where the text overflows it
+        # (a failed call loads nothing).
+        room = _line_room(buf) if bounds else 0
+        while True:
+            bnd = np.empty((room, 4), np.uint64) if bounds else None
+            rc = self._L.ish_gpu_records_load_fastx(
+                self._h, _p(buf, C.c_uint8) if len(buf) else None, len(buf), matrix_kind, C.byref(sid), C.byref(n),
+                _p(bnd, C.c_uint64) if bounds else None, room)
+            most = int(np.count_nonzero(buf == 10)) + 1 if rc == EOVERFLOW else 0
+            if rc != EOVERFLOW or room >= most:
+                break
+            room = most
+        self._check(rc)
+        return sid.value, n.value, (bnd[:n.value] if bounds else None)
 
     def records_get(self, sid: int, first: int = 0, count: int | None = None):
         """Records [first, first + count) of a resident set, as stored
