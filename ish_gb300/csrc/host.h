@@ -208,6 +208,7 @@ struct ish_ctx {
   cudaEvent_t raw_ev = nullptr;
   cudaEvent_t off_ev = nullptr;  // the offsets are on the device
   bool raw_overlapped = false;  // the last load used copy_stream
+  bool load_times_due = false;  // last_load_ms is still to be read from the last load's events
   std::string err;
   int kernel = ISH_KERNEL_AUTO;
   int sg_lanes = 8, sw_u8_lanes = 16, sw_u16_lanes = 8;
@@ -311,7 +312,7 @@ size_t layout_bytes(int layout, int alphabet, int G, int K);
 int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode);
 int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayout **out);
 int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, uint32_t n, RecordSet &rs,
-                 const uint8_t *enc, cudaStream_t s = nullptr, bool defer = false);
+                 const uint8_t *enc, cudaStream_t s = nullptr, bool defer = false, uint32_t limit = 0);
 // Sorts and packs the n records in ctx->raw ([off_in[i], end[i]) or, with end
 // NULL, [off_in[i], off_in[i + 1])) into rs on stream s (NULL: the context's
 // stream).  defer: the host-side summary of the set (histogram, largest code)

@@ -491,7 +491,23 @@ void load_phase_times(ish_ctx *ctx) {
   if (cudaEventElapsedTime(&a, ctx->load_ev[0], mid) == cudaSuccess) ctx->last_load_ms[0] = a;
   if (cudaEventElapsedTime(&b, mid, ctx->load_ev[2]) == cudaSuccess) ctx->last_load_ms[1] = b;
   (void)cudaGetLastError();
+  ctx->load_times_due = false;
 }
+
+// Lanes per record of k_pack: the power of two nearest above the average
+// 16-byte chunks per record, 4 to 32.
+static uint32_t pack_group(uint32_t n, uint64_t total) {
+  uint32_t gw = 4;
+  while (gw < 32 && (uint64_t)gw * 16 * n < total) gw <<= 1;
+  return gw;
+}
+// Its blocks: one group per record, or a block per 64 KB for sets of long records.
+static uint32_t pack_blocks(const ish_ctx *ctx, uint32_t n, uint64_t total) {
+  return (uint32_t)std::min<uint64_t>(
+      std::max<uint64_t>(ceil_div((uint64_t)n * pack_group(n, total), 256), (total >> 16) + 1),
+      (uint64_t)ctx->num_sms * 3);
+}
+static cudaError_t ensure_codes(ish_ctx *ctx, RecordSet &rs, size_t bytes);
 
 // Sort and pack n records held in ctx->raw (raw_bytes bytes): record i is
 // raw[off_in[i] .. end[i]) with `end` on the device, or raw[off_in[i] ..
@@ -542,28 +558,14 @@ int pack_set(ish_ctx *ctx, uint32_t n, uint64_t raw_bytes, const uint64_t *end, 
   ++ctx->launches;
   CU(cudaGetLastError());
   ctx->pack_dirty = false;
-  {
-    cudaError_t e = rs.codes.ensure(packed);
-    if (e == cudaErrorMemoryAllocation && !ctx->spare_sets.empty()) {  // give the cached buffers back first
-      (void)cudaGetLastError();
-      for (RecordSet &sp : ctx->spare_sets) release_set(sp);
-      ctx->spare_sets.clear();
-      e = rs.codes.ensure(packed);
-    }
-    CU(e);
-  }
-  // lanes per record: the power of two nearest above the average 16-byte
-  // chunks per record, 4 to 32
-  uint32_t gw = 4;
-  while (gw < 32 && (uint64_t)gw * 16 * n < rs.total) gw <<= 1;
+  CU(ensure_codes(ctx, rs, packed));
+  const uint32_t gw = pack_group(n, rs.total);
   ctx->raw_overlapped = raw_pending;
   if (raw_pending) CU(cudaStreamWaitEvent(s, ctx->raw_ev, 0));  // the records' bytes are on the device
-  // one group per record, or a block per 64 KB for sets of long records
-  const uint32_t pb = (uint32_t)std::min<uint64_t>(
-      std::max<uint64_t>(ceil_div((uint64_t)n * gw, 256), (rs.total >> 16) + 1), (uint64_t)ctx->num_sms * 3);
+  const uint32_t pb = pack_blocks(ctx, n, rs.total);
   k_pack<<<pb, 256, 0, s>>>(ctx->raw.as<uint8_t>(), raw_bytes, ctx->off_in.as<uint64_t>(), end,
                             ctx->poff_tmp.as<uint64_t>(), n, rs.len_s.as<uint32_t>(), rs.orig_s.as<uint32_t>(),
-                            max_bucket + 1, enc, rs.codes.as<uint8_t>(), summary, gw);
+                            max_bucket + 1, enc, rs.codes.as<uint8_t>(), summary, gw, 0);
   ++ctx->launches;
   CU(cudaGetLastError());
   CU(cudaEventRecord(ctx->load_ev[2], s));
@@ -592,19 +594,110 @@ int pack_set(ish_ctx *ctx, uint32_t n, uint64_t raw_bytes, const uint64_t *end, 
   return ISH_OK;
 }
 
+static void set_lengths(RecordSet &rs);
+
 // A set's host-side summary from the device's {largest code, largest bucket,
 // counts}; counts above the largest bucket are not read (they are zero).
 void set_summary(RecordSet &rs, const uint32_t *h) {
   rs.max_code = h[0];
   const uint32_t maxb = std::min<uint32_t>(h[1], NBUCKETS - 1);
   rs.hist.assign(h + 2, h + 2 + maxb + 1);
+  set_lengths(rs);
+}
+
+// What follows from the histogram.
+static void set_lengths(RecordSet &rs) {
+  const uint32_t maxb = top_bucket(rs);
   rs.n_empty = rs.hist[0];
   rs.max_len = maxb < 32768 ? maxb : (uint32_t)(32768 + ((uint64_t)(maxb - 32768) << 5) + 31);
 }
 
+// The length bucket of a record, as the device counts it (len_bucket).
+static uint32_t length_bucket(uint64_t len) {
+  if (len < 32768) return (uint32_t)len;
+  return (uint32_t)std::min<uint64_t>(32768 + ((len - 32768) >> 5), NBUCKETS - 1);
+}
+
+// Allocates the codes of a set, giving the cached buffers of freed sets back
+// first when memory is short.
+static cudaError_t ensure_codes(ish_ctx *ctx, RecordSet &rs, size_t bytes) {
+  cudaError_t e = rs.codes.ensure(bytes);
+  if (e == cudaErrorMemoryAllocation && !ctx->spare_sets.empty()) {
+    (void)cudaGetLastError();
+    for (RecordSet &sp : ctx->spare_sets) release_set(sp);
+    ctx->spare_sets.clear();
+    e = rs.codes.ensure(bytes);
+  }
+  return e;
+}
+
+// Upload and pack a set of at most SORT_SMALL records: two kernels, and the
+// histogram from the caller's offsets (which have to ascend: their differences
+// index it), so that of the set's summary only the largest code comes from the
+// device.  With `limit` (the alphabet of the query
+// that is scored next) the call does not wait for it: codes outside the alphabet
+// are stored as 0, and the caller reads the largest code, at ctx->summary, with
+// its results.
+static int load_small(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, uint32_t n, RecordSet &rs,
+                      const uint8_t *enc, cudaStream_t s, bool defer, uint32_t limit) {
+  const uint64_t base = offsets[0], bytes = offsets[n] - base;
+  uint32_t top = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    if (offsets[i + 1] < offsets[i]) return fail(ctx, ISH_EINVAL, "offsets are not monotone");
+    top = std::max(top, length_bucket(offsets[i + 1] - offsets[i]));
+  }
+  rs.hist.assign(top + 1, 0);
+  for (uint32_t i = 0; i < n; ++i) ++rs.hist[length_bucket(offsets[i + 1] - offsets[i])];
+  set_lengths(rs);
+  rs.n = n;
+  rs.max_code = 0;
+  const uint64_t packed = bytes + 16ull * n + 16;
+  take_spare_set(ctx, rs, packed);
+  CU(ctx->raw.ensure(bytes + 32));
+  CU(ctx->off_in.ensure((size_t)(n + 1) * 8));
+  CU(ctx->poff_tmp.ensure((size_t)n * 8));
+  CU(ctx->hist.ensure((size_t)NBUCKETS * 4 * 2 + 16));
+  CU(ctx->summary.ensure((size_t)(2 + NBUCKETS) * 4));
+  CU(rs.len_s.ensure((size_t)n * 4));
+  CU(rs.off_s.ensure((size_t)n * 8));
+  CU(rs.orig_s.ensure((size_t)n * 4));
+  CU(ensure_codes(ctx, rs, packed));
+  uint32_t *long_counter = ctx->hist.as<uint32_t>() + 2 * NBUCKETS + 1, *max_code = ctx->summary.as<uint32_t>();
+  CU(cudaEventRecord(ctx->load_ev[0], s));
+  CU(cudaMemcpyAsync(ctx->off_in.p, offsets, (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, s));
+  if (bytes) CU(cudaMemcpyAsync(ctx->raw.p, records + base, bytes, cudaMemcpyHostToDevice, s));
+  ctx->raw_overlapped = false;
+  CU(cudaEventRecord(ctx->load_ev[1], s));
+  uint32_t threads = 32;
+  while (threads * 4 < n) threads *= 2;
+  k_sort_small<<<1, threads, 0, s>>>(ctx->off_in.as<uint64_t>(), n, base, ctx->poff_tmp.as<uint64_t>(),
+                                     rs.len_s.as<uint32_t>(), rs.off_s.as<uint64_t>(), rs.orig_s.as<uint32_t>(),
+                                     long_counter, max_code);
+  ++ctx->launches;
+  k_pack<<<pack_blocks(ctx, n, bytes), 256, 0, s>>>(
+      ctx->raw.as<uint8_t>(), bytes, ctx->off_in.as<uint64_t>(), nullptr, ctx->poff_tmp.as<uint64_t>(), n,
+      rs.len_s.as<uint32_t>(), rs.orig_s.as<uint32_t>(), long_counter, enc, rs.codes.as<uint8_t>(), max_code,
+      pack_group(n, bytes), limit);
+  ++ctx->launches;
+  CU(cudaGetLastError());
+  CU(cudaEventRecord(ctx->load_ev[2], s));
+  ctx->load_times_due = true;
+  if (limit) return ISH_OK;
+  CU(cudaMemcpyAsync(ctx->h_summary, max_code, 4, cudaMemcpyDeviceToHost, s));
+  if (defer) {
+    CU(cudaEventRecord(ctx->load_done, s));
+    rs.pending = true;
+    return ISH_OK;
+  }
+  CU(cudaStreamSynchronize(s));
+  rs.max_code = ctx->h_summary[0];
+  return ISH_OK;
+}
+
 // Upload and pack a record set given as concatenated records + n+1 offsets.
+// limit: see load_small (0: wait for the set's summary).
 int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, uint32_t n, RecordSet &rs,
-                 const uint8_t *enc, cudaStream_t stream, bool defer) {
+                 const uint8_t *enc, cudaStream_t stream, bool defer, uint32_t limit) {
   if (n == 0) {
     rs.n = 0;
     rs.total = 0;
@@ -617,6 +710,7 @@ int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, 
   if (bytes && !records) return fail(ctx, ISH_EINVAL, "records is NULL");
   rs.total = bytes;
   cudaStream_t s = stream ? stream : ctx->stream;
+  if (n <= SORT_SMALL) return load_small(ctx, records, offsets, n, rs, enc, s, defer, limit);
   // The offsets go first on s; the records' bytes (+16 slack for the
   // realigning pack loads) follow on the copy stream once the offsets are in
   // (everything before this load on s, which includes the previous pack's
@@ -667,7 +761,8 @@ int finish_pending_load(ish_ctx *ctx) {
     return fail(ctx, ISH_EDEVICE, "asynchronous load of record set %d failed: %s (the set is gone)", id,
                 cudaGetErrorString(e));
   }
-  set_summary(rs, ctx->h_summary);
+  if (rs.hist.empty()) set_summary(rs, ctx->h_summary);
+  else rs.max_code = ctx->h_summary[0];  // (load_small has counted the lengths)
   load_phase_times(ctx);
   return ISH_OK;
 }
@@ -1030,22 +1125,35 @@ int run_scoring(ish_ctx *ctx, Query &q, RecordSet &rs) {
   return ISH_OK;
 }
 
+// max_code: the set's largest code where the host has not seen it yet (load_small
+// with a limit), checked against the query's alphabet; NULL else.
 int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32_t *tend, uint8_t *hit,
-                  uint32_t *hit_idx, uint32_t *n_hits) {
+                  uint32_t *hit_idx, uint32_t *n_hits, const uint32_t *max_code = nullptr, int alphabet = 0) {
   cudaStream_t s = ctx->stream;
   const bool compact = (hit_idx || n_hits) && n;
+  CU(ctx->nhits.ensure(16));
+  uint32_t *out3 = ctx->nhits.as<uint32_t>();  // hits, error flags, largest code
   if (compact) {
     const uint32_t nb = ceil_div(n, HIT_TILE);
-    CU(ctx->block_counts.ensure((size_t)nb * 4 + 8));
     CU(ctx->hit_idx.ensure((size_t)n * 4 + 4));
-    CU(ctx->nhits.ensure(16));
-    k_count_hits<<<nb, 1024, 0, s>>>(ctx->out_hit.as<uint8_t>(), n, ctx->block_counts.as<uint32_t>());
-    ++ctx->launches;
-    k_scan_counts<<<1, 1024, 0, s>>>(ctx->block_counts.as<uint32_t>(), nb, ctx->nhits.as<uint32_t>());
-    ++ctx->launches;
-    k_write_hits<<<nb, 1024, 0, s>>>(ctx->out_hit.as<uint8_t>(), n, ctx->block_counts.as<uint32_t>(),
-                                     ctx->hit_idx.as<uint32_t>());
-    ++ctx->launches;
+    const uint8_t *flags = ctx->out_hit.as<uint8_t>();
+    if (n <= COMPACT_ONE) {
+      k_compact_one<<<1, 1024, 0, s>>>(flags, n, ctx->hit_idx.as<uint32_t>(), ctx->error.as<int>(), max_code, out3);
+      ++ctx->launches;
+    } else {
+      CU(ctx->block_counts.ensure((size_t)nb * 4 + 8));
+      uint32_t *counts = ctx->block_counts.as<uint32_t>();
+      k_count_hits<<<nb, 1024, 0, s>>>(flags, n, counts);
+      ++ctx->launches;
+      if (nb <= 1024) {
+        k_write_hits_sum<<<nb, 1024, 0, s>>>(flags, n, counts, ctx->hit_idx.as<uint32_t>(), ctx->error.as<int>(), out3);
+      } else {
+        k_scan_counts<<<1, 1024, 0, s>>>(counts, nb, out3);
+        ++ctx->launches;
+        k_write_hits<<<nb, 1024, 0, s>>>(flags, n, counts, ctx->hit_idx.as<uint32_t>());
+      }
+      ++ctx->launches;
+    }
     CU(cudaGetLastError());
   }
   CU(cudaEventRecord(ctx->ev1, s));
@@ -1053,20 +1161,24 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
   if (n && qend) CU(cudaMemcpyAsync(qend, ctx->out_qend.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
   if (n && tend) CU(cudaMemcpyAsync(tend, ctx->out_tend.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
   if (n && hit) CU(cudaMemcpyAsync(hit, ctx->out_hit.p, (size_t)n, cudaMemcpyDeviceToHost, s));
-  // error flags and hit count into pinned staging, so that every copy of the
-  // call stays asynchronous until the one synchronisation below
+  // hit count, error flags and largest code into pinned staging, so that every
+  // copy of the call stays asynchronous until the one synchronisation below
   uint32_t *hs = reinterpret_cast<uint32_t *>(ctx->h_small);
-  hs[1] = 0;
-  CU(cudaMemcpyAsync(hs, ctx->error.p, 4, cudaMemcpyDeviceToHost, s));
-  if (compact) CU(cudaMemcpyAsync(hs + 1, ctx->nhits.p, 4, cudaMemcpyDeviceToHost, s));
+  hs[0] = hs[1] = hs[2] = 0;
+  if (compact) CU(cudaMemcpyAsync(hs, out3, 12, cudaMemcpyDeviceToHost, s));
+  if (!compact || ceil_div(n, HIT_TILE) > 1024)
+    CU(cudaMemcpyAsync(hs + 1, ctx->error.p, 4, cudaMemcpyDeviceToHost, s));
+  if (max_code && !(compact && n <= COMPACT_ONE)) CU(cudaMemcpyAsync(hs + 2, max_code, 4, cudaMemcpyDeviceToHost, s));
   // the first hit indices travel with the count (hit_idx holds n entries, so
   // the prefix fits whatever the count); the rest, if any, after it
   constexpr uint32_t HIT_PREFIX = 4096;
   const uint32_t prefix = std::min<uint32_t>(n, HIT_PREFIX);
   if (hit_idx && compact) CU(cudaMemcpyAsync(hit_idx, ctx->hit_idx.p, (size_t)prefix * 4, cudaMemcpyDeviceToHost, s));
   CU(cudaStreamSynchronize(s));
-  const int herr = (int)hs[0];
-  const uint32_t total = hs[1];
+  const int herr = (int)hs[1];
+  const uint32_t total = hs[0];
+  if (max_code && hs[2] >= (uint32_t)alphabet)
+    return fail(ctx, ISH_EINVAL, "a record contains code %u >= the alphabet size %d of the query", hs[2], alphabet);
   if (hit_idx && total > prefix) {
     CU(cudaMemcpyAsync(hit_idx + prefix, ctx->hit_idx.as<uint32_t>() + prefix, (size_t)(total - prefix) * 4,
                        cudaMemcpyDeviceToHost, s));
@@ -1330,6 +1442,7 @@ int ish_gpu_records_load_async(ish_ctx *ctx, const uint8_t *records, const uint6
   LoadTimer timer(ctx);
   cudaSetDevice(ctx->device);
   RecordSet rs;
+  if (ctx->load_times_due) load_phase_times(ctx);  // before its events are used again
   // the load stream starts after the work already queued on the context's
   // stream (a set freed just before may still be read there)
   CU(cudaEventRecord(ctx->load_ev[0], ctx->stream));
@@ -1442,9 +1555,13 @@ int ish_gpu_score(ish_ctx *ctx, int32_t query_id, const uint8_t *records, const 
   cudaSetDevice(ctx->device);
   if (int rc0 = finish_pending_load(ctx)) return rc0;
   RecordSet rs;
-  int rc = load_records(ctx, records, offsets, n, rs, nullptr);
+  const int alphabet = qi->second.alphabet;
+  const uint32_t limit = n && n <= SORT_SMALL && alphabet < 256 ? (uint32_t)alphabet : 0;
+  int rc = load_records(ctx, records, offsets, n, rs, nullptr, nullptr, false, limit);
   if (!rc) rc = run_scoring(ctx, qi->second, rs);
-  if (!rc) rc = fetch_outputs(ctx, n, score, query_end, target_end, hit, hit_idx, n_hits);
+  if (!rc)
+    rc = fetch_outputs(ctx, n, score, query_end, target_end, hit, hit_idx, n_hits,
+                       limit && qi->second.Q ? ctx->summary.as<uint32_t>() : nullptr, alphabet);
   cudaStreamSynchronize(ctx->stream);
   recycle_set(ctx, rs);  // the next call's set takes these buffers
   return rc;
@@ -1516,6 +1633,7 @@ int ish_gpu_last_kernel_ms(ish_ctx *ctx, double *ms) {
 
 int ish_gpu_last_load_ms(ish_ctx *ctx, double *upload_ms, double *pack_ms, double *wall_ms) {
   if (!ctx) return ISH_EINVAL;
+  if (ctx->load_times_due) load_phase_times(ctx);
   if (upload_ms) *upload_ms = ctx->last_load_ms[0];
   if (pack_ms) *pack_ms = ctx->last_load_ms[1];
   if (wall_ms) *wall_ms = ctx->last_load_ms[2];

@@ -240,6 +240,91 @@ __global__ void __launch_bounds__(1024) k_scatter(const uint32_t *len, const uin
   }
 }
 
+// Sets of at most SORT_SMALL records: lengths, packed offsets and sorted
+// positions in one block, where the four kernels above spend most of their time
+// being launched; what the host needs to know of the set (its histogram) it has
+// counted from its own offsets.  Each thread holds four consecutive keys
+// (longest bucket first, then record order) of a bitonic network: steps of 1
+// and 2 stay in the thread, of 4 to 64 in the warp, and only those from 128 (15
+// of 78 at 4,096 records) meet at a barrier.  The block has a quarter of the
+// next power of two in threads.  Rebases off by `base` for k_pack.  (The whole
+// load of 500 lines 60 us -> 51 with it and one stream, one synchronisation
+// less; a network in shared memory alone took 23 us longer at 3,000 proteins.)
+__global__ void __launch_bounds__(1024) k_sort_small(uint64_t *off, uint32_t n, uint64_t base, uint64_t *poff,
+                                                     uint32_t *len_s, uint64_t *off_s, uint32_t *orig_s,
+                                                     uint32_t *long_counter, uint32_t *max_code) {
+  __shared__ uint4 cross[2][SORT_SMALL / 4];
+  __shared__ uint64_t warp_sums[32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, e0 = tid * 4;
+  if (tid == 0) *long_counter = *max_code = 0;
+  uint64_t o[5], sum = 0;
+  uint32_t v[4];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) o[k] = e0 + k <= n ? off[e0 + k] - base : 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint64_t len = e0 + k < n ? o[k + 1] - o[k] : 0;
+    v[k] = e0 + k < n ? (NBUCKETS - 1 - len_bucket(len)) * SORT_SMALL + e0 + k : 0xffffffffu;
+    sum += (len + 15) & ~(uint64_t)15;
+  }
+  uint64_t x = sum;
+  for (int s = 1; s < 32; s <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, x, s);
+    if (lane >= (uint32_t)s) x += y;
+  }
+  if (lane == 31) warp_sums[wid] = x;
+  __syncthreads();  // (also: every thread has read its offsets)
+  uint64_t before = lane < wid ? warp_sums[lane] : 0;
+  for (int s = 16; s > 0; s >>= 1) before += __shfl_xor_sync(0xffffffffu, before, s);
+  uint64_t run = before + x - sum;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const uint32_t i = e0 + k;
+    if (i < n) {
+      poff[i] = run;
+      run += (o[k + 1] - o[k] + 15) & ~(uint64_t)15;
+    }
+    if (i <= n && base) off[i] = o[k];
+  }
+  if (base && e0 + 4 == n && tid == blockDim.x - 1) off[n] = o[4];
+
+  auto keep = [&](int k, uint32_t other, bool low) { v[k] = low ? min(v[k], other) : max(v[k], other); };
+  int buf = 0;
+  for (uint32_t width = 2; width <= blockDim.x * 4; width <<= 1) {
+    for (uint32_t step = width >> 1; step >= 128; step >>= 1) {
+      cross[buf][tid] = make_uint4(v[0], v[1], v[2], v[3]);
+      __syncthreads();
+      const uint4 p = cross[buf][tid ^ (step >> 2)];
+      const bool low = ((e0 & step) == 0) == ((e0 & width) == 0);
+      keep(0, p.x, low), keep(1, p.y, low), keep(2, p.z, low), keep(3, p.w, low);
+      buf ^= 1;
+    }
+    for (uint32_t step = min(width >> 1, 64u); step >= 4; step >>= 1) {
+      const bool low = ((e0 & step) == 0) == ((e0 & width) == 0);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) keep(k, __shfl_xor_sync(0xffffffffu, v[k], step >> 2), low);
+    }
+    auto order = [&](int a, int b) {
+      const bool up = ((e0 + a) & width) == 0;
+      const uint32_t lo = min(v[a], v[b]), hi = max(v[a], v[b]);
+      v[a] = up ? lo : hi;
+      v[b] = up ? hi : lo;
+    };
+    if (width >= 4) order(0, 2), order(1, 3);
+    order(0, 1), order(2, 3);
+  }
+  __syncthreads();  // the offsets of every record are written
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    if (e0 + k < n) {
+      const uint32_t i = v[k] % SORT_SMALL;
+      len_s[e0 + k] = (uint32_t)(off[i + 1] - off[i]);
+      off_s[e0 + k] = poff[i];
+      orig_s[e0 + k] = i;
+    }
+  }
+}
+
 // Copies every record to dst[poff[i] ..) in 16-byte chunks realigned with
 // funnel shifts, optionally encoded through a 256-entry byte table (ish's
 // convert_ascii_to_encoding, done per byte on the host by the runners,
@@ -252,14 +337,16 @@ __global__ void __launch_bounds__(1024) k_scatter(const uint32_t *len, const uin
 // record quickly.  The other records go to groups of `gw` lanes (a power of
 // two up to 32, chosen by the host near the set's average 16-byte chunks per
 // record, so that short lines do not leave most of a warp idle), PACK_U
-// records per group at a time.
+// records per group at a time.  With `limit`, codes from it up are stored as 0
+// (after they went into the largest code): a caller that scores before it has
+// seen that code reads no profile row outside the alphabet.
 constexpr uint64_t PACK_LONG = 16384;
 
 __global__ void __launch_bounds__(256, 3) k_pack(const uint8_t *src, uint64_t src_bytes, const uint64_t *off,
                                                  const uint64_t *end, const uint64_t *poff, uint32_t n,
                                                  const uint32_t *len_s, const uint32_t *orig_s,
                                                  uint32_t *long_counter, const uint8_t *enc, uint8_t *dst,
-                                                 uint32_t *max_code, uint32_t gw) {
+                                                 uint32_t *max_code, uint32_t gw, uint32_t limit) {
   __shared__ uint8_t table[256];
   __shared__ uint32_t s_item;
   if (enc) {
@@ -297,8 +384,12 @@ __global__ void __launch_bounds__(256, 3) k_pack(const uint8_t *src, uint64_t sr
         else if (keep < 4) o[k] &= (1u << (8 * keep)) - 1u;
       }
     }
-    d[c] = make_uint4(o[0], o[1], o[2], o[3]);
     mx = __vmaxu4(mx, __vmaxu4(__vmaxu4(o[0], o[1]), __vmaxu4(o[2], o[3])));
+    if (limit) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] &= __vcmpltu4(o[k], limit * 0x01010101u);
+    }
+    d[c] = make_uint4(o[0], o[1], o[2], o[3]);
   };
   auto load = [&](uint64_t b, uint32_t (&w)[5]) {
     const uint64_t w0 = b >> 2;
@@ -792,6 +883,88 @@ __global__ void __launch_bounds__(1024) k_write_hits(const uint8_t *hit, uint32_
     if (lane >= (uint32_t)o) x += y;
   }
   uint32_t run = block_offsets[blockIdx.x] + __shfl_sync(0xffffffffu, x, wid) - c;
+  if (!c) return;
+  const uint32_t below = (1u << lane) - 1u;
+  for (uint32_t k = 0; k < HIT_WARP; k += 32) {
+    const uint64_t i = w0 + k + lane;
+    const bool h = i < n && hit[i];
+    const uint32_t m = __ballot_sync(0xffffffffu, h);
+    if (h) idx[run + __popc(m & below)] = (uint32_t)i;
+    run += __popc(m);
+  }
+}
+
+// The whole compaction of up to COMPACT_ONE records in one block: out = {hits,
+// *error, *max_code or 0}, which the host reads back together.  (One launch
+// and one copy instead of three and two: scoring 500 resident lines 87 us -> 81.)
+__global__ void __launch_bounds__(1024) k_compact_one(const uint8_t *hit, uint32_t n, uint32_t *idx, const int *error,
+                                                      const uint32_t *max_code, uint32_t *out) {
+  __shared__ uint32_t wsum[32];
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t per = ((n + 1023) / 1024) * 32, w0 = wid * per;  // consecutive records of each warp
+  uint32_t c = 0;
+#pragma unroll 4
+  for (uint32_t k = 0; k < per; k += 32) {
+    const uint32_t i = w0 + k + lane;
+    c += __popc(__ballot_sync(0xffffffffu, i < n && hit[i]));
+  }
+  if (lane == 0) wsum[wid] = c;
+  __syncthreads();
+  uint32_t x = wsum[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  uint32_t run = __shfl_sync(0xffffffffu, x, wid) - c;
+  if (threadIdx.x == 31) {
+    out[0] = x;
+    out[1] = (uint32_t)*error;
+    out[2] = max_code ? *max_code : 0u;
+  }
+  if (!c) return;
+  const uint32_t below = (1u << lane) - 1u;
+  for (uint32_t k = 0; k < per; k += 32) {
+    const uint32_t i = w0 + k + lane;
+    const bool h = i < n && hit[i];
+    const uint32_t m = __ballot_sync(0xffffffffu, h);
+    if (h) idx[run + __popc(m & below)] = i;
+    run += __popc(m);
+  }
+}
+
+// k_write_hits without the scan between it and k_count_hits: every block adds
+// the counts of the tiles before its own, at most 1,024 of them, and the last
+// writes out = {hits, *error, 0}.  (100,000 resident lines 122 us -> 118.)
+__global__ void __launch_bounds__(1024) k_write_hits_sum(const uint8_t *hit, uint32_t n, const uint32_t *block_counts,
+                                                         uint32_t *idx, const int *error, uint32_t *out) {
+  __shared__ uint32_t wsum[32], bsum[32];
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  uint32_t before = threadIdx.x < blockIdx.x ? block_counts[threadIdx.x] : 0u;
+  for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+  const uint64_t w0 = (uint64_t)blockIdx.x * HIT_TILE + wid * HIT_WARP;
+  uint32_t c = 0;
+#pragma unroll
+  for (uint32_t k = 0; k < HIT_WARP; k += 32) {
+    const uint64_t i = w0 + k + lane;
+    c += __popc(__ballot_sync(0xffffffffu, i < n && hit[i]));
+  }
+  if (lane == 0) {
+    wsum[wid] = c;
+    bsum[wid] = before;
+  }
+  __syncthreads();
+  uint32_t x = wsum[lane], b = bsum[lane];
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= (uint32_t)o) x += y;
+  }
+  for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+  uint32_t run = b + __shfl_sync(0xffffffffu, x, wid) - c;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 31) {
+    out[0] = b + x;
+    out[1] = (uint32_t)*error;
+    out[2] = 0;
+  }
   if (!c) return;
   const uint32_t below = (1u << lane) - 1u;
   for (uint32_t k = 0; k < HIT_WARP; k += 32) {

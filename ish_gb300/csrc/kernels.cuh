@@ -22,9 +22,13 @@ __global__ void k_bucket_cursors(const uint32_t *hist, const uint32_t *max_bucke
 __global__ void k_scatter(const uint32_t *len, const uint64_t *poff, uint32_t n, uint32_t *cursor, uint32_t *len_s,
                           uint64_t *off_s, uint32_t *orig_s, uint32_t *hist, uint32_t *max_bucket,
                           const uint32_t *summary);
+constexpr uint32_t SORT_SMALL = 4096;    // records that k_sort_small takes
+__global__ void k_sort_small(uint64_t *off, uint32_t n, uint64_t base, uint64_t *poff, uint32_t *len_s,
+                             uint64_t *off_s, uint32_t *orig_s, uint32_t *long_counter, uint32_t *max_code);
 __global__ void k_pack(const uint8_t *src, uint64_t src_bytes, const uint64_t *off, const uint64_t *end,
                        const uint64_t *poff, uint32_t n, const uint32_t *len_s, const uint32_t *orig_s,
-                       uint32_t *long_counter, const uint8_t *enc, uint8_t *dst, uint32_t *max_code, uint32_t gw);
+                       uint32_t *long_counter, const uint8_t *enc, uint8_t *dst, uint32_t *max_code, uint32_t gw,
+                       uint32_t limit);
 __global__ void k_count_newlines(const uint8_t *text, uint64_t bytes, uint32_t *block_counts);
 // k_write_newlines<headers>: with headers, also the first '>' or '@' of every
 // line (hc, preset to all ones)
@@ -50,6 +54,11 @@ __global__ void k_dpx_peak(uint32_t *out, int iters, uint32_t b, uint32_t c);
 typedef void (*LaneFn)(uint32_t *out, int rows, uint32_t p0, uint32_t popen, uint32_t pext, uint32_t bias);
 LaneFn lane_rows_fn(bool u8);
 __global__ void k_write_hits(const uint8_t *hit, uint32_t n, const uint32_t *block_offsets, uint32_t *idx);
+constexpr uint32_t COMPACT_ONE = 16384;  // records that k_compact_one takes
+__global__ void k_compact_one(const uint8_t *hit, uint32_t n, uint32_t *idx, const int *error,
+                              const uint32_t *max_code, uint32_t *out);
+__global__ void k_write_hits_sum(const uint8_t *hit, uint32_t n, const uint32_t *block_counts, uint32_t *idx,
+                                 const int *error, uint32_t *out);
 __global__ void k_gather_hits(const uint32_t *idx, const uint32_t *count, const int32_t *score, const int32_t *qend,
                               const int32_t *tend, int32_t *hit_score, int32_t *hit_qend, int32_t *hit_tend);
 
