@@ -123,6 +123,9 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // leaving it; local alignment: the best of this thread's and all earlier
   // columns up to the step's last row, which the next thread uses a step later
   uint32_t outH[RPS], outF[RPS], outB = 0, left_best = 0;
+  // local alignment: the best of all later columns in the rows that the next
+  // thread, a step behind, had left when this step began
+  uint32_t right_best = 0;
 #pragma unroll
   for (int k = 0; k < RPS; ++k) outH[k] = outF[k] = 0;
   uint32_t outC = CTL_IDLE;
@@ -165,10 +168,6 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // arrives, which keeps few of them in registers), and returns F leaving the
   // last column.
   auto row_step = [&](uint32_t cA, uint32_t cB, uint32_t diag, uint32_t fs) -> uint32_t {
-    if (remap) {  // codes that score alike share a profile row
-      cA = prof[remap_off + cA];
-      cB = prof[remap_off + cB];
-    }
     // one column: `dp` is the pair's scores, semi-global (but for PROF_S16)
     // with H of the row above one column to the left added
     auto cell = [&](int j, uint32_t dp) {
@@ -239,11 +238,13 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
 
   // Local alignment, after row `row` (`live`: the halves of the lanes whose
   // record holds that row): a row maximum that does not beat every cell so far
-  // in this thread AND in the columns to its left can never be the first row of
-  // the record's maximum at its smallest column (it is smaller, or equal in a
-  // later row or a larger column), so only the others are recorded.  `thr` is
-  // that bar: this thread's rows up to the last, the left columns' rows up to
-  // the last step (a later row of theirs may tie without winning).
+  // in this thread, in the columns to its left AND in earlier rows of those to
+  // its right can never be the first row of the record's maximum at its smallest
+  // column (it is smaller, or equal in a later row or a larger column), so only
+  // the others are recorded.  `thr` is that bar: this thread's rows up to the
+  // last, the left columns' rows up to the last step (a later row of theirs may
+  // tie without winning), and the rows the right columns have reached (they run
+  // behind).
   auto sw_track = [&](int row, uint32_t &thr, uint32_t live) {
     uint32_t cm = H[0];
 #pragma unroll
@@ -430,13 +431,16 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // final, and a new pair resets all of its state.
   while (true) {
     __syncwarp();
-    uint32_t msgH[RPS], msgF[RPS], msgB = 0;
+    uint32_t msgH[RPS], msgF[RPS], msgB = 0, msgR = 0;
 #pragma unroll
     for (int k = 0; k < RPS; ++k) {
       msgH[k] = __shfl_up_sync(FULL, outH[k], 1, G);
       msgF[k] = __shfl_up_sync(FULL, outF[k], 1, G);
     }
-    if (MODE == SW) msgB = __shfl_up_sync(FULL, outB, 1, G);
+    if (MODE == SW) {
+      msgB = __shfl_up_sync(FULL, outB, 1, G);
+      msgR = __shfl_down_sync(FULL, __vmaxu2(best, right_best), 1, G);
+    }
     uint32_t msgC = __shfl_up_sync(FULL, outC, 1, G);
     if (t0) msgC &= ~CTL_NEW;  // its own last control word
     // partial results of records that ended in thread t-1's previous step
@@ -599,6 +603,19 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       wA >>= 16;
       wB >>= 16;
     }
+    // Codes that score alike share a profile row.  Mapped once per step: a test
+    // in every row keeps the compiler from starting a row's loads in the row
+    // above (38 columns, no mapping, 400,000 proteins: semi-global 6,440 -> 6,280
+    // us, local 1 % on top of the wider bar's 1 %).
+    if (remap && (RPS == 4 || (q4 & 3) == 0)) {
+      const unsigned char *map = prof + remap_off;
+      const auto rows_of = [&](uint32_t w) {
+        return (uint32_t)map[w & 0xffu] | (uint32_t)map[(w >> 8) & 0xffu] << 8 |
+               (uint32_t)map[(w >> 16) & 0xffu] << 16 | (uint32_t)map[w >> 24] << 24;
+      };
+      wA = rows_of(wA);
+      wB = rows_of(wB);
+    }
     // thread 0: what enters the padding from the left, H at its boundary (local:
     // the floor) and F below every value
     if (t0) {
@@ -637,7 +654,10 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
       prevH = d;
     } else {
       // ---- the step's rows ----
-      uint32_t thr = __vmaxu2(best, left_best);  // (local alignment)
+      // (local alignment; in a pair's first two steps the next thread's word is
+      // still of the pair before)
+      if (MODE == SW) right_best = t == G - 1 || q4 < 2 * RPS ? 0u : msgR;
+      uint32_t thr = MODE == SW ? __vimax3_u16x2(best, left_best, right_best) : 0u;
 #pragma unroll
       for (int k = 0; k < RPS; ++k) {
         const uint32_t fs = row_step(__byte_perm(wA, 0u, 0x4440 + k), __byte_perm(wB, 0u, 0x4440 + k),
