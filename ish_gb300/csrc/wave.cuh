@@ -61,10 +61,16 @@ namespace ish {
 
 // Scores sorted entries [p.first, p.first + p.count) of the record set: the
 // groups of the calling block take record pairs from *counter until none are
-// left.  `prof` is the profile in shared memory; `slots_all` holds one word per
-// thread (a group's G pair indices in flight), `save_all` wave_save_words(K)
-// words per thread (local alignment only).
-template <int K, int MODE, int LAYOUT>
+// left.  With DEAL (the launch's blocks all start on this range) a group's first
+// pair is dealt instead: the longest pairs to the first warp of every block, the
+// next to the second, and the counter hands out what is left.  When the groups
+// took them from the counter the first blocks got all the longest pairs, and a
+// set of little more than a pair per group was bound by those blocks (100,000
+// lines 215 -> 205 us, 3,000 proteins with match starts 887 -> 860).  `prof` is
+// the profile in shared memory; `slots_all` holds one word per thread (a group's
+// G pair indices in flight), `save_all` wave_save_words(K) words per thread
+// (local alignment only).
+template <int K, int MODE, int LAYOUT, bool DEAL>
 __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned char *prof, uint32_t *slots_all,
                                           uint32_t *save_all, uint32_t *counter) {
   constexpr int RPS = (MODE == SG) ? WAVE_RPS_SG : WAVE_RPS_SW;
@@ -157,7 +163,12 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
   // before the current pair ends, late enough that a group with a long pair
   // leaves the next ones to the others, and early enough that neither the
   // counter nor the new pair's lengths and codes are waited for
-  uint32_t f_next = t0 ? atomicAdd(counter, 1u) : 0u;
+  uint32_t f_next = 0;
+  const auto claim = [&]() -> uint32_t {  // the pairs dealt come before the counter's
+    return atomicAdd(counter, 1u) + (DEAL ? (gridDim.x * blockDim.x) >> __popc(G - 1) : 0u);
+  };
+  const int lgG = __popc(G - 1);
+  if (t0) f_next = DEAL ? ((tid >> 5) * gridDim.x + blockIdx.x) * (32u >> lgG) + (lane >> lgG) : claim();
   constexpr int CHK = 8 / RPS;  // steps between termination checks
   constexpr int CLAIM = 32, LOOK_META = 20, LOOK_CODES = 8;  // rows before a pair's end (see below)
   uint32_t step = 0;
@@ -492,7 +503,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         }
         if (t0) {
           end_q = (max(max(lenA, lenB), 1) + RPS - 1) & ~(RPS - 1);
-          if (max(lenA, lenB) < CLAIM + RPS) f_next = atomicAdd(counter, 1u);
+          if (max(lenA, lenB) < CLAIM + RPS) f_next = claim();
         }
         nA = __ldg(reinterpret_cast<const uint32_t *>(pa));
         nB = lenB ? __ldg(reinterpret_cast<const uint32_t *>(pb)) : 0u;
@@ -546,7 +557,7 @@ __device__ __forceinline__ void wave_rows(const WaveParams &p, const unsigned ch
         }
         // thread 0: the next pair is claimed, and what it needs first is
         // fetched into L1
-        if (t0 && at(CLAIM)) f_next = atomicAdd(counter, 1u);
+        if (t0 && at(CLAIM)) f_next = claim();
         if (t0 && (at(LOOK_META) || at(LOOK_CODES)) && f_next < npairs) {
           const uint32_t sA = p.first + 2 * (f_next * pstride + pphase);
           if (at(LOOK_META)) {
@@ -753,7 +764,7 @@ __device__ __forceinline__ void wave_rows_smem_params(const WaveParams &p, const
   __shared__ WaveParams sp;
   if (threadIdx.x == 0) sp = p;
   __syncthreads();
-  wave_rows<K, MODE, LAYOUT>(sp, prof, slots_all, save_all, p.counter);
+  wave_rows<K, MODE, LAYOUT, true>(sp, prof, slots_all, save_all, p.counter);
 }
 
 // Copies a query's profile to shared memory (the caller's barrier follows).  All
@@ -780,7 +791,7 @@ __global__ void __launch_bounds__(wave_sm_threads(K, LEAN), 1)
     wave_rows_smem_params<K, MODE, LAYOUT>(p, smem_raw, slots_all, save_all);
   } else {
     __syncthreads();
-    wave_rows<K, MODE, LAYOUT>(p, smem_raw, slots_all, save_all, p.counter);
+    wave_rows<K, MODE, LAYOUT, true>(p, smem_raw, slots_all, save_all, p.counter);
   }
 }
 
@@ -831,7 +842,7 @@ __global__ void __launch_bounds__(wave_sm_threads(K, LEAN), 1)
     }
     load_profile(smem_raw, qp->prof, qp->prof_bytes);
     __syncthreads();
-    wave_rows<K, MODE, LAYOUT>(sp, smem_raw, slots_all, save_all, counter);
+    wave_rows<K, MODE, LAYOUT, false>(sp, smem_raw, slots_all, save_all, counter);
     __syncthreads();
   }
 }
