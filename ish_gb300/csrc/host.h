@@ -197,6 +197,7 @@ struct ish_ctx {
   cudaEvent_t load_done = nullptr;     // end of the asynchronous load in flight
   uint32_t *h_summary = nullptr;       // pinned: its largest code, largest bucket, then the histogram
   uint64_t *h_small = nullptr;         // pinned: small results read back by a call (error flags, counts)
+  uint32_t *h_stage = nullptr;         // pinned: the results of a small call (StageOut)
   int32_t pending_set = 0;             // the set whose asynchronous load is in flight (0: none)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   cudaEvent_t load_ev[3] = {nullptr, nullptr, nullptr};  // last load: start, packing start, end

@@ -1130,7 +1130,7 @@ int run_scoring(ish_ctx *ctx, Query &q, RecordSet &rs) {
 int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32_t *tend, uint8_t *hit,
                   uint32_t *hit_idx, uint32_t *n_hits, const uint32_t *max_code = nullptr, int alphabet = 0) {
   cudaStream_t s = ctx->stream;
-  const bool compact = (hit_idx || n_hits) && n;
+  const bool compact = (hit_idx || n_hits) && n, staged = compact && n <= SORT_SMALL;
   CU(ctx->nhits.ensure(16));
   uint32_t *out3 = ctx->nhits.as<uint32_t>();  // hits, error flags, largest code
   if (compact) {
@@ -1138,7 +1138,16 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
     CU(ctx->hit_idx.ensure((size_t)n * 4 + 4));
     const uint8_t *flags = ctx->out_hit.as<uint8_t>();
     if (n <= COMPACT_ONE) {
-      k_compact_one<<<1, 1024, 0, s>>>(flags, n, ctx->hit_idx.as<uint32_t>(), ctx->error.as<int>(), max_code, out3);
+      StageOut stage;
+      if (staged) {
+        stage.to = ctx->h_stage;
+        stage.hit = hit != nullptr;
+        if (score) stage.from[0] = ctx->out_score.as<int32_t>();
+        if (qend) stage.from[1] = ctx->out_qend.as<int32_t>();
+        if (tend) stage.from[2] = ctx->out_tend.as<int32_t>();
+      }
+      k_compact_one<<<1, 1024, 0, s>>>(flags, n, ctx->hit_idx.as<uint32_t>(), ctx->error.as<int>(), max_code, out3,
+                                       stage);
       ++ctx->launches;
     } else {
       CU(ctx->block_counts.ensure((size_t)nb * 4 + 8));
@@ -1157,29 +1166,39 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
     CU(cudaGetLastError());
   }
   CU(cudaEventRecord(ctx->ev1, s));
-  if (n && score) CU(cudaMemcpyAsync(score, ctx->out_score.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-  if (n && qend) CU(cudaMemcpyAsync(qend, ctx->out_qend.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-  if (n && tend) CU(cudaMemcpyAsync(tend, ctx->out_tend.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
-  if (n && hit) CU(cudaMemcpyAsync(hit, ctx->out_hit.p, (size_t)n, cudaMemcpyDeviceToHost, s));
-  // hit count, error flags and largest code into pinned staging, so that every
-  // copy of the call stays asynchronous until the one synchronisation below
-  uint32_t *hs = reinterpret_cast<uint32_t *>(ctx->h_small);
-  hs[0] = hs[1] = hs[2] = 0;
-  if (compact) CU(cudaMemcpyAsync(hs, out3, 12, cudaMemcpyDeviceToHost, s));
-  if (!compact || ceil_div(n, HIT_TILE) > 1024)
-    CU(cudaMemcpyAsync(hs + 1, ctx->error.p, 4, cudaMemcpyDeviceToHost, s));
-  if (max_code && !(compact && n <= COMPACT_ONE)) CU(cudaMemcpyAsync(hs + 2, max_code, 4, cudaMemcpyDeviceToHost, s));
-  // the first hit indices travel with the count (hit_idx holds n entries, so
-  // the prefix fits whatever the count); the rest, if any, after it
+  // Results of a small call were written to pinned memory by the compaction;
+  // those of a larger one are copied: hit count, error flags and largest code go
+  // into pinned staging too, so that every copy stays asynchronous until the one
+  // synchronisation, and the first hit indices travel with the count (hit_idx
+  // holds n entries, so the prefix fits whatever the count).
+  uint32_t *hs = staged ? ctx->h_stage : reinterpret_cast<uint32_t *>(ctx->h_small);
   constexpr uint32_t HIT_PREFIX = 4096;
   const uint32_t prefix = std::min<uint32_t>(n, HIT_PREFIX);
-  if (hit_idx && compact) CU(cudaMemcpyAsync(hit_idx, ctx->hit_idx.p, (size_t)prefix * 4, cudaMemcpyDeviceToHost, s));
+  if (!staged) {
+    if (n && score) CU(cudaMemcpyAsync(score, ctx->out_score.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
+    if (n && qend) CU(cudaMemcpyAsync(qend, ctx->out_qend.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
+    if (n && tend) CU(cudaMemcpyAsync(tend, ctx->out_tend.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s));
+    if (n && hit) CU(cudaMemcpyAsync(hit, ctx->out_hit.p, (size_t)n, cudaMemcpyDeviceToHost, s));
+    hs[0] = hs[1] = hs[2] = 0;
+    if (compact) CU(cudaMemcpyAsync(hs, out3, 12, cudaMemcpyDeviceToHost, s));
+    if (!compact || ceil_div(n, HIT_TILE) > 1024)
+      CU(cudaMemcpyAsync(hs + 1, ctx->error.p, 4, cudaMemcpyDeviceToHost, s));
+    if (max_code && !(compact && n <= COMPACT_ONE)) CU(cudaMemcpyAsync(hs + 2, max_code, 4, cudaMemcpyDeviceToHost, s));
+    if (hit_idx && compact) CU(cudaMemcpyAsync(hit_idx, ctx->hit_idx.p, (size_t)prefix * 4, cudaMemcpyDeviceToHost, s));
+  }
   CU(cudaStreamSynchronize(s));
   const int herr = (int)hs[1];
   const uint32_t total = hs[0];
   if (max_code && hs[2] >= (uint32_t)alphabet)
     return fail(ctx, ISH_EINVAL, "a record contains code %u >= the alphabet size %d of the query", hs[2], alphabet);
-  if (hit_idx && total > prefix) {
+  if (staged) {
+    const uint32_t *v = hs + STAGE_HEAD;
+    if (score) memcpy(score, v, (size_t)n * 4);
+    if (qend) memcpy(qend, v + SORT_SMALL, (size_t)n * 4);
+    if (tend) memcpy(tend, v + 2 * SORT_SMALL, (size_t)n * 4);
+    if (hit_idx) memcpy(hit_idx, v + 3 * SORT_SMALL, (size_t)total * 4);
+    if (hit) memcpy(hit, v + 4 * SORT_SMALL, n);
+  } else if (hit_idx && total > prefix) {
     CU(cudaMemcpyAsync(hit_idx + prefix, ctx->hit_idx.as<uint32_t>() + prefix, (size_t)(total - prefix) * 4,
                        cudaMemcpyDeviceToHost, s));
     CU(cudaStreamSynchronize(s));
@@ -1241,6 +1260,8 @@ int ish_gpu_open(int device, ish_ctx **out) {
     return bail(e, "cudaHostAlloc");
   if ((e = cudaHostAlloc((void **)&ctx->h_small, 64 * 8, cudaHostAllocDefault)) != cudaSuccess)
     return bail(e, "cudaHostAlloc");
+  if ((e = cudaHostAlloc((void **)&ctx->h_stage, STAGE_WORDS * 4, cudaHostAllocDefault)) != cudaSuccess)
+    return bail(e, "cudaHostAlloc");
   *out = ctx;
   return ISH_OK;
 }
@@ -1272,6 +1293,7 @@ void ish_gpu_close(ish_ctx *ctx) {
   if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
   cudaFreeHost(ctx->h_summary);
   if (ctx->h_small) cudaFreeHost(ctx->h_small);
+  if (ctx->h_stage) cudaFreeHost(ctx->h_stage);
   for (cudaEvent_t ev : ctx->load_ev) cudaEventDestroy(ev);
   cudaStreamDestroy(ctx->stream);
   delete ctx;

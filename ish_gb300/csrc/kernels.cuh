@@ -55,8 +55,20 @@ typedef void (*LaneFn)(uint32_t *out, int rows, uint32_t p0, uint32_t popen, uin
 LaneFn lane_rows_fn(bool u8);
 __global__ void k_write_hits(const uint8_t *hit, uint32_t n, const uint32_t *block_offsets, uint32_t *idx);
 constexpr uint32_t COMPACT_ONE = 16384;  // records that k_compact_one takes
+// The results of a call on up to SORT_SMALL records in pinned host memory: three
+// counts of k_compact_one, then scores, query ends, target ends, hit indices
+// (SORT_SMALL words each) and hit flags.  The six copies it replaces cost a call
+// more than the bytes: 500 lines 116 -> 109 us, 3,000 proteins with match starts
+// 825 -> 781 (their arrays are pageable, whose copies the driver stages one by
+// one).
+struct StageOut {
+  uint32_t *to = nullptr;
+  const int32_t *from[3] = {nullptr, nullptr, nullptr};  // scores, query ends, target ends on the device (null: not wanted)
+  bool hit = false;                                      // the flags are wanted
+};
+constexpr uint32_t STAGE_HEAD = 4, STAGE_WORDS = STAGE_HEAD + 4 * SORT_SMALL + SORT_SMALL / 4;
 __global__ void k_compact_one(const uint8_t *hit, uint32_t n, uint32_t *idx, const int *error,
-                              const uint32_t *max_code, uint32_t *out);
+                              const uint32_t *max_code, uint32_t *out, StageOut stage);
 __global__ void k_write_hits_sum(const uint8_t *hit, uint32_t n, const uint32_t *block_counts, uint32_t *idx,
                                  const int *error, uint32_t *out);
 __global__ void k_gather_hits(const uint32_t *idx, const uint32_t *count, const int32_t *score, const int32_t *qend,
