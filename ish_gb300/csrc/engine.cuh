@@ -87,6 +87,7 @@ struct WaveParams {
   RecordsDev rec;
   OutDev out;
   Decision dec;
+  uint32_t dealt;          // wave_kernel: groups of the launch, each of which starts on a pair of its own
 };
 
 // One work range of the batched launch: sorted entries [first, first + count)

@@ -955,6 +955,7 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
   wave_params(q, *L, rs, out, ctx->error.as<int>(), &p);
   p.first = first;
   p.count = count;
+  p.dealt = grid * (uint32_t)threads / (uint32_t)G;
   p.counter = ctx->counter.as<uint32_t>();
   p.max_steps = ctx->step_budget ? ctx->step_budget : rs.total + 2ull * count + 1024;
   CU(cudaMemsetAsync(ctx->counter.p, 0, 4, s));
