@@ -288,6 +288,9 @@ int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, Out
   CU(R.qend.ensure((size_t)nw * 4));
   CU(R.tend.ensure((size_t)nw * 4));
   CU(R.hit.ensure((size_t)nw));
+  // Sets without a histogram (reversed prefixes) may hold empty entries, which no
+  // kernel writes: their end row is 0.
+  if (rs.hist.empty()) CU(cudaMemsetAsync(R.tend.p, 0, (size_t)nw * 4, s));
   RecordSet view = window_set(rs, V);
   pick_shape(ctx, q, &G, &K, &layout, &view);  // the windows may be few
   OutDev wout{R.score.as<int32_t>(), R.qend.as<int32_t>(), R.tend.as<int32_t>(), R.hit.as<uint8_t>()};
