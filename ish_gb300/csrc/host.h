@@ -122,6 +122,11 @@ struct WindowView {
     for (DevBuf *x : b) x->release();
     nw = 0;
   }
+  // Forgets the view, keeping its buffers for the next one unless they are large.
+  void clear() {
+    nw = 0;
+    if (off.cap + len.cap + slot.cap + start.cap + cs.cap > (size_t(64) << 20)) release();
+  }
 };
 
 // Per-window results of the last windowed pass (windows.cu).
@@ -144,7 +149,8 @@ struct RecordSet {
   std::vector<uint32_t> hist;  // length-bucket histogram (host copy) up to the largest bucket used
   uint32_t n_empty = 0;
   uint32_t max_code = 0;       // largest record code in the set
-  DevBuf inv;                  // sorted entry of each original record (built on first use)
+  DevBuf inv;                  // sorted entry of each original record, once inv_ready (built on first use)
+  bool inv_ready = false;
   WindowView windows;          // built on first windowed pass
 };
 
@@ -234,6 +240,8 @@ struct ish_ctx {
   ish::host::DevBuf enc_tables, nl_pos, line_end;  // encoding tables; line splitting scratch
   ish::host::FastxScratch fastx;                    // FASTA/FASTQ splitting scratch (fastx.cu)
   ish::host::ExactRes exact;                        // exact kernels (exact.cu)
+  ish::host::DevBuf starts_ws, starts_codes;        // start finding: per-hit arrays, reversed prefixes (starts.cu)
+  ish::host::WindowView starts_windows;             // its window view's buffers, between calls
   ish::host::WindowOut window_out;                  // windowed passes (windows.cu)
   uint32_t last_windows = 0;                        // windows of the last windowed pass
   float last_ms = 0.f;

@@ -65,8 +65,7 @@ static constexpr size_t kSpareSets = 2;
 static size_t spare_codes_max(const ish_ctx *ctx) { return std::max<size_t>(size_t(1) << 30, ctx->mem_total / 16); }
 
 void recycle_set(ish_ctx *ctx, RecordSet &rs) {
-  rs.inv.release();  // rebuilt on first use by the next set
-  rs.windows.release();
+  rs.windows.clear();
   if (!rs.codes.p || rs.codes.cap > spare_codes_max(ctx)) {
     release_set(rs);
     return;
@@ -80,8 +79,12 @@ void recycle_set(ish_ctx *ctx, RecordSet &rs) {
   keep.off_s = rs.off_s;
   keep.len_s = rs.len_s;
   keep.orig_s = rs.orig_s;
+  keep.inv = rs.inv;  // (inv_ready is not kept: the next set rebuilds it)
+  keep.windows = rs.windows;
   ctx->spare_sets.push_back(keep);
-  rs.codes = rs.off_s = rs.len_s = rs.orig_s = DevBuf{};
+  rs.codes = rs.off_s = rs.len_s = rs.orig_s = rs.inv = DevBuf{};
+  rs.inv_ready = false;
+  rs.windows = WindowView{};
 }
 
 // Hands `rs` the spare buffers with the smallest code area that holds
@@ -99,6 +102,8 @@ void take_spare_set(ish_ctx *ctx, RecordSet &rs, size_t codes_bytes) {
   rs.off_s = sp.off_s;
   rs.len_s = sp.len_s;
   rs.orig_s = sp.orig_s;
+  rs.inv = sp.inv;
+  rs.windows = sp.windows;
   ctx->spare_sets.erase(ctx->spare_sets.begin() + pick);
 }
 
@@ -1280,10 +1285,11 @@ void ish_gpu_close(ish_ctx *ctx) {
   DevBuf *bufs[] = {&ctx->raw, &ctx->off_in, &ctx->len_tmp, &ctx->poff_tmp, &ctx->hist, &ctx->summary,
                     &ctx->scan_tmp, &ctx->counter, &ctx->error, &ctx->out_score, &ctx->out_qend, &ctx->out_tend,
                     &ctx->out_hit, &ctx->hit_idx, &ctx->block_counts, &ctx->nhits, &ctx->plain_scratch,
-                    &ctx->enc_tables, &ctx->nl_pos, &ctx->line_end};
+                    &ctx->enc_tables, &ctx->nl_pos, &ctx->line_end, &ctx->starts_ws, &ctx->starts_codes};
   for (DevBuf *b : bufs) b->release();
   ctx->exact.release();
   ctx->window_out.release();
+  ctx->starts_windows.release();
   ctx->fastx.release();
   cudaEventDestroy(ctx->ev0);
   cudaEventDestroy(ctx->ev1);

@@ -64,10 +64,11 @@ int ish_gpu_records_get(ish_ctx *ctx, int32_t set_id, uint32_t first, uint32_t c
   cudaSetDevice(ctx->device);
   cudaStream_t s = ctx->stream;
   const uint32_t nb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(rs.n, 256), (uint32_t)ctx->num_sms * 8));
-  if (!rs.inv.p) {
+  if (!rs.inv_ready) {
     CU(rs.inv.ensure((size_t)rs.n * 4));
     k_invert<<<nb, 256, 0, s>>>(rs.orig_s.as<uint32_t>(), rs.n, rs.inv.as<uint32_t>());
     ++ctx->launches;
+    rs.inv_ready = true;
   }
   DevBuf len, off, scan, out;
   auto cleanup = [&] {

@@ -15,6 +15,7 @@
 // wavefront kernel and the reversed query, and turns the reverse end row j
 // into start = len(prefix) - 1 - j.
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 #include "host.h"
@@ -29,7 +30,7 @@ __global__ void k_invert(const uint32_t *orig_s, uint32_t n, uint32_t *inv) {
 // zero byte past the prefix and is never empty).
 __global__ void k_rev_lengths(const uint32_t *hits, const int32_t *tend, uint32_t nh, const uint32_t *inv,
                               const uint32_t *len_s, uint32_t n, uint32_t *rlen, uint64_t *slot, uint32_t *orig,
-                              int *error) {
+                              int32_t *rev_end, int *error) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
     const uint32_t h = hits[i];
     uint32_t r = 0;
@@ -44,6 +45,7 @@ __global__ void k_rev_lengths(const uint32_t *hits, const int32_t *tend, uint32_
     rlen[i] = r;
     slot[i] = ((uint64_t)r + 16) & ~(uint64_t)15;
     orig[i] = i;
+    rev_end[i] = 0;
   }
 }
 
@@ -62,13 +64,20 @@ __global__ void k_rev_pack(const uint32_t *hits, uint32_t nh, uint32_t n, const 
   }
 }
 
-__global__ void k_starts(const uint32_t *rlen, const int32_t *rev_end, uint32_t nh, int64_t *start) {
+// (start may be pinned host memory, as error_out always is)
+__global__ void k_starts(const uint32_t *rlen, const int32_t *rev_end, uint32_t nh, int64_t *start, const int *error,
+                         uint32_t *error_out) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *error_out = (uint32_t)*error;
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x)
     start[i] = (int64_t)rlen[i] - 1 - rev_end[i];
 }
 
 namespace host {
 namespace {
+
+// Reversed prefixes of up to this many bytes are allocated for by their bound and
+// kept for the next call.
+constexpr uint64_t STARTS_KEEP = uint64_t(256) << 20;
 
 // The reversed query: sequence reversed, free query/target start and end
 // swapped (semi_global_aln_start_end, striped.mojo:165-183).
@@ -110,8 +119,16 @@ extern "C" int ish_gpu_match_starts(ish_ctx *ctx, int32_t query_id, int32_t set_
   Query &q = qi->second;
   RecordSet &rs = *si_set;
   const uint32_t n = rs.n;
-  for (uint32_t i = 0; i < n_hits; ++i)
+  // Bounds of the reversed prefixes' rows and bytes, from the ends alone (a row
+  // count is also at most its record's, which the device knows).
+  uint64_t bound = 0;
+  uint32_t longest = 0;
+  for (uint32_t i = 0; i < n_hits; ++i) {
     if (hit_idx[i] >= n) return fail(ctx, ISH_EINVAL, "hit index %u >= %u records", hit_idx[i], n);
+    const uint32_t r = (uint32_t)std::min<int64_t>(std::max<int64_t>((int64_t)target_end[i] + 1, 0), rs.max_len);
+    longest = std::max(longest, r);
+    bound += ((uint64_t)r + 16) & ~(uint64_t)15;
+  }
   Query &rq = reverse_of(q);
   // the reverse pass runs where the forward pass ran: the wavefront kernels
   // in their exact regime, else the lane-exact emulation (exact.cu)
@@ -127,20 +144,24 @@ extern "C" int ish_gpu_match_starts(ish_ctx *ctx, int32_t query_id, int32_t set_
                 rq.alphabet);
   cudaStream_t s = ctx->stream;
   const uint32_t nb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256), (uint32_t)ctx->num_sms * 8));
-  if (!rs.inv.p) {
+  if (!rs.inv_ready) {
     CU(rs.inv.ensure((size_t)n * 4));
     k_invert<<<nb, 256, 0, s>>>(rs.orig_s.as<uint32_t>(), n, rs.inv.as<uint32_t>());
     ++ctx->launches;
     CU(cudaGetLastError());
+    rs.inv_ready = true;
   }
-  // scratch: hits, ends, lengths, slots, offsets, identity order, reverse ends, starts
-  DevBuf d_hits, d_tend, rlen, slot, poff, orig, rev_end, d_start, scan;
+  // The context keeps the call's buffers (unless large): allocating and freeing
+  // ten of them and waiting for lengths in between took 245 of the 375 us of
+  // 2,205 hits in reads.
   RecordSet rev;
+  rev.windows = ctx->starts_windows;
+  ctx->starts_windows = WindowView{};
   auto cleanup = [&] {
-    DevBuf *b[] = {&d_hits, &d_tend, &rlen, &slot, &poff, &orig, &rev_end, &d_start, &scan};
-    for (DevBuf *x : b) x->release();
-    rev.codes.release();
-    rev.windows.release();
+    rev.windows.clear();
+    ctx->starts_windows = rev.windows;
+    if (ctx->starts_ws.cap > (size_t(64) << 20)) ctx->starts_ws.release();
+    if (ctx->starts_codes.cap > STARTS_KEEP) ctx->starts_codes.release();
   };
   int rc = ISH_OK;
   do {
@@ -159,80 +180,86 @@ extern "C" int ish_gpu_match_starts(ish_ctx *ctx, int32_t query_id, int32_t set_
       break;                                                                                       \
     }                                                                                              \
   }
-    SCU(d_hits.ensure((size_t)n_hits * 4));
-    SCU(d_tend.ensure((size_t)n_hits * 4));
-    SCU(rlen.ensure((size_t)n_hits * 4));
-    SCU(slot.ensure((size_t)n_hits * 8));
-    SCU(poff.ensure((size_t)n_hits * 8 + 8));
-    SCU(orig.ensure((size_t)n_hits * 4));
-    SCU(rev_end.ensure((size_t)n_hits * 4));
-    SCU(d_start.ensure((size_t)n_hits * 8));
-    SCU(scan.ensure((size_t)(tiles + 1) * 16));
+    // per hit: slot, packed offset, start; hit, end, rows, order, reverse end
+    const size_t nh = ((size_t)n_hits + 3) & ~(size_t)3;
+    SCU(ctx->starts_ws.ensure(nh * 44 + (size_t)(tiles + 1) * 16 + 16));
+    uint64_t *slot = ctx->starts_ws.as<uint64_t>(), *poff = slot + nh, *bsum = poff + nh + 2;
+    uint64_t *boff = bsum + tiles + 1;
+    int64_t *d_start = reinterpret_cast<int64_t *>(boff + tiles + 1);
+    uint32_t *d_hits = reinterpret_cast<uint32_t *>(d_start + nh), *rlen = d_hits + 2 * nh, *orig = rlen + nh;
+    int32_t *d_tend = reinterpret_cast<int32_t *>(d_hits + nh), *rev_end = reinterpret_cast<int32_t *>(orig + nh);
     SCU(ctx->error.ensure(64));
     SCU(cudaMemsetAsync(ctx->error.p, 0, 4, s));
-    SCU(cudaMemcpyAsync(d_hits.p, hit_idx, (size_t)n_hits * 4, cudaMemcpyHostToDevice, s));
-    SCU(cudaMemcpyAsync(d_tend.p, target_end, (size_t)n_hits * 4, cudaMemcpyHostToDevice, s));
+    // few hits: both arrays in one copy from pinned memory, the starts written back there
+    const bool staged = nh * 8 + 16 <= STAGE_WORDS * 4;
+    if (staged) {
+      memcpy(ctx->h_stage, hit_idx, (size_t)n_hits * 4);
+      memcpy(ctx->h_stage + nh, target_end, (size_t)n_hits * 4);
+      SCU(cudaMemcpyAsync(d_hits, ctx->h_stage, nh * 8, cudaMemcpyHostToDevice, s));
+    } else {
+      SCU(cudaMemcpyAsync(d_hits, hit_idx, (size_t)n_hits * 4, cudaMemcpyHostToDevice, s));
+      SCU(cudaMemcpyAsync(d_tend, target_end, (size_t)n_hits * 4, cudaMemcpyHostToDevice, s));
+    }
     const uint32_t hb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n_hits, 256), (uint32_t)ctx->num_sms * 8));
-    k_rev_lengths<<<hb, 256, 0, s>>>(d_hits.as<uint32_t>(), d_tend.as<int32_t>(), n_hits, rs.inv.as<uint32_t>(),
-                                      rs.len_s.as<uint32_t>(), n, rlen.as<uint32_t>(), slot.as<uint64_t>(),
-                                      orig.as<uint32_t>(), ctx->error.as<int>());
+    k_rev_lengths<<<hb, 256, 0, s>>>(d_hits, d_tend, n_hits, rs.inv.as<uint32_t>(), rs.len_s.as<uint32_t>(), n, rlen,
+                                     slot, orig, rev_end, ctx->error.as<int>());
     ++ctx->launches;
-    uint64_t *bsum = scan.as<uint64_t>();
-    uint64_t *boff = bsum + tiles + 1;
-    k_scan64_block<<<tiles, 1024, 0, s>>>(slot.as<uint64_t>(), poff.as<uint64_t>(), n_hits, bsum);
+    k_scan64_block<<<tiles, 1024, 0, s>>>(slot, poff, n_hits, bsum);
     ++ctx->launches;
     if (tiles > 1) {
       k_scan64_block<<<1, 1024, 0, s>>>(bsum, boff, tiles, nullptr);
       ++ctx->launches;
-      k_scan64_add<<<tiles, 1024, 0, s>>>(poff.as<uint64_t>(), n_hits, boff);
+      k_scan64_add<<<tiles, 1024, 0, s>>>(poff, n_hits, boff);
       ++ctx->launches;
     }
     SCU(cudaGetLastError());
-    uint64_t last[2] = {0, 0};
-    SCU(cudaMemcpyAsync(&last[0], poff.as<uint64_t>() + n_hits - 1, 8, cudaMemcpyDeviceToHost, s));
-    SCU(cudaMemcpyAsync(&last[1], slot.as<uint64_t>() + n_hits - 1, 8, cudaMemcpyDeviceToHost, s));
-    SCU(cudaStreamSynchronize(s));
-    const uint64_t bytes = last[0] + last[1];
-    SCU(rev.codes.ensure(bytes + 16));
+    // (ends far past their records make the bounds too large to allocate for)
+    if (bound > STARTS_KEEP) {
+      uint64_t last[2] = {0, 0};
+      SCU(cudaMemcpyAsync(&last[0], poff + n_hits - 1, 8, cudaMemcpyDeviceToHost, s));
+      SCU(cudaMemcpyAsync(&last[1], slot + n_hits - 1, 8, cudaMemcpyDeviceToHost, s));
+      std::vector<uint32_t> hl(n_hits);
+      SCU(cudaMemcpyAsync(hl.data(), rlen, (size_t)n_hits * 4, cudaMemcpyDeviceToHost, s));
+      SCU(cudaStreamSynchronize(s));
+      bound = last[0] + last[1];
+      longest = *std::max_element(hl.begin(), hl.end());
+    }
+    SCU(ctx->starts_codes.ensure(bound + 16));
+    rev.codes = ctx->starts_codes;  // (borrowed, like the arrays below)
     k_rev_pack<<<std::max<uint32_t>(1, std::min<uint32_t>(ceil_div((uint64_t)n_hits * 32, 256),
                                                           (uint32_t)ctx->num_sms * 16)),
-                 256, 0, s>>>(d_hits.as<uint32_t>(), n_hits, n, rs.inv.as<uint32_t>(), rs.codes.as<uint8_t>(),
-                              rs.off_s.as<uint64_t>(), rlen.as<uint32_t>(), poff.as<uint64_t>(), slot.as<uint64_t>(),
-                              rev.codes.as<uint8_t>());
+                 256, 0, s>>>(d_hits, n_hits, n, rs.inv.as<uint32_t>(), rs.codes.as<uint8_t>(), rs.off_s.as<uint64_t>(),
+                              rlen, poff, slot, rev.codes.as<uint8_t>());
     ++ctx->launches;
     SCU(cudaGetLastError());
     // the reversed prefixes as a record set in hit order (empty prefixes keep
     // reverse end 0, i.e. start -1, as semi_global_aln gives for an empty
     // record)
     rev.n = n_hits;
-    rev.total = bytes;
-    rev.off_s.p = poff.p;
-    rev.len_s.p = rlen.p;
-    rev.orig_s.p = orig.p;
-    SCU(cudaMemsetAsync(rev_end.p, 0, (size_t)n_hits * 4, s));
-    OutDev out{nullptr, nullptr, rev_end.as<int32_t>(), nullptr};
+    rev.total = bound;
+    rev.off_s.p = poff;
+    rev.len_s.p = rlen;
+    rev.orig_s.p = orig;
+    OutDev out{nullptr, nullptr, rev_end, nullptr};
     if (rq.Q > 0 && fast) {
       // long prefixes (hits in long records) go through the window view like
       // a forward pass; it needs the longest prefix
-      std::vector<uint32_t> hl(n_hits);
-      SCU(cudaMemcpy(hl.data(), rlen.p, (size_t)n_hits * 4, cudaMemcpyDeviceToHost));
-      rev.max_len = *std::max_element(hl.begin(), hl.end());
+      rev.max_len = longest;
       bool windowed = false;
       rc = launch_windows(ctx, rq, rev, n_hits, out, s, &windowed);
       if (!rc && !windowed) rc = launch_range(ctx, rq, rev, 0, n_hits, out, s);
-      if (!rc) SCU(cudaStreamSynchronize(s));
     } else if (rq.Q > 0) {
       rc = launch_exact(ctx, rq, rev, 0, n_hits, out, s);
     }
-    rev.off_s.p = rev.len_s.p = rev.orig_s.p = nullptr;  // owned by poff / rlen / orig
     if (rc) break;
-    k_starts<<<hb, 256, 0, s>>>(rlen.as<uint32_t>(), rev_end.as<int32_t>(), n_hits, d_start.as<int64_t>());
+    int64_t *to = staged ? reinterpret_cast<int64_t *>(ctx->h_stage + 4) : d_start;
+    k_starts<<<hb, 256, 0, s>>>(rlen, rev_end, n_hits, to, ctx->error.as<int>(), ctx->h_stage);
     ++ctx->launches;
     SCU(cudaGetLastError());
-    int herr = 0;
-    SCU(cudaMemcpyAsync(start, d_start.p, (size_t)n_hits * 8, cudaMemcpyDeviceToHost, s));
-    SCU(cudaMemcpyAsync(&herr, ctx->error.p, 4, cudaMemcpyDeviceToHost, s));
+    if (!staged) SCU(cudaMemcpyAsync(start, d_start, (size_t)n_hits * 8, cudaMemcpyDeviceToHost, s));
     SCU(cudaStreamSynchronize(s));
+    if (staged) memcpy(start, to, (size_t)n_hits * 8);
+    const uint32_t herr = ctx->h_stage[0];
     if (herr & 2) rc = fail(ctx, ISH_ETIMEDOUT, "wavefront kernel exceeded its step budget (internal error)");
     else if (herr) rc = fail(ctx, ISH_EINVAL, "bad hit index or record code");
 #undef SCU

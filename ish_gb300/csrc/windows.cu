@@ -163,7 +163,7 @@ uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int 
 int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint64_t W, uint64_t O, WindowView &V,
                       cudaStream_t s) {
   if (V.nw && V.W == W && V.O == O && V.entries == nonempty) return ISH_OK;
-  V.release();
+  V.nw = 0;  // (its buffers may be those of an earlier view)
   std::vector<uint32_t> len(nonempty);
   std::vector<uint64_t> off(nonempty);
   CU(cudaStreamSynchronize(s));
@@ -218,11 +218,12 @@ int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint
   CU(V.slot.ensure((size_t)nw * 4));
   CU(V.start.ensure((size_t)nw * 4));
   CU(V.cs.ensure((size_t)(nonempty + 1) * 4));
-  CU(cudaMemcpy(V.off.p, voff.data(), (size_t)nw * 8, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(V.len.p, vlen.data(), (size_t)nw * 4, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(V.slot.p, vslot.data(), (size_t)nw * 4, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(V.start.p, wstart.data(), (size_t)nw * 4, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(V.cs.p, cs.data(), (size_t)(nonempty + 1) * 4, cudaMemcpyHostToDevice));
+  // (pageable sources: each call returns once its bytes are staged)
+  CU(cudaMemcpyAsync(V.off.p, voff.data(), (size_t)nw * 8, cudaMemcpyHostToDevice, s));
+  CU(cudaMemcpyAsync(V.len.p, vlen.data(), (size_t)nw * 4, cudaMemcpyHostToDevice, s));
+  CU(cudaMemcpyAsync(V.slot.p, vslot.data(), (size_t)nw * 4, cudaMemcpyHostToDevice, s));
+  CU(cudaMemcpyAsync(V.start.p, wstart.data(), (size_t)nw * 4, cudaMemcpyHostToDevice, s));
+  CU(cudaMemcpyAsync(V.cs.p, cs.data(), (size_t)(nonempty + 1) * 4, cudaMemcpyHostToDevice, s));
   V.W = W;
   V.O = O;
   V.entries = nonempty;
