@@ -449,22 +449,35 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
                 (unsigned long long)(first_stop >> 1));
   if (keep > 0xffffffffull) return fail(ctx, ISH_EINVAL, "too many records (%llu)", (unsigned long long)keep);
   const uint32_t nr = (uint32_t)keep;
-  if (bounds_out) {
-    if (nr > bounds_cap) return fail(ctx, ISH_EOVERFLOW, "%u records, bounds capacity %llu", nr,
-                                     (unsigned long long)bounds_cap);
-    if (nr) CU(cudaMemcpyAsync(bounds_out, fx.bounds.p, (size_t)nr * 32, cudaMemcpyDeviceToHost, s));
-  }
+  if (bounds_out && nr > bounds_cap)
+    return fail(ctx, ISH_EOVERFLOW, "%u records, bounds capacity %llu", nr, (unsigned long long)bounds_cap);
   rs.total = used;
   *n_out = nr;
-  if (nr == 0) {
+  if (nr == 0) return ISH_OK;
+  // The records are packed while the bounds, final since the wait above, are
+  // copied to the caller's array: filling pageable memory takes the host longer
+  // than the packing takes the device.
+  auto pack = [&](uint64_t raw_bytes, const uint64_t *end) -> int {
+    int prc = pack_set(ctx, nr, raw_bytes, end, enc, rs, nullptr, true);
+    if (prc) return prc;
+    rs.pending = false;
+    cudaError_t be = cudaSuccess;
+    if (bounds_out) {
+      be = cudaMemcpyAsync(bounds_out, fx.bounds.p, (size_t)nr * 32, cudaMemcpyDeviceToHost, ctx->copy_stream);
+      const cudaError_t se = cudaStreamSynchronize(ctx->copy_stream);
+      if (be == cudaSuccess) be = se;
+    }
     CU(cudaStreamSynchronize(s));
+    CU(be);
+    set_summary(rs, ctx->h_summary);
+    load_phase_times(ctx);
     return ISH_OK;
-  }
+  };
   if (one_line) {
     // every sequence is one line (FASTQ, unwrapped FASTA): packed from the text
     // where it lies
     std::swap(ctx->off_in, fx.seq_start);
-    return pack_set(ctx, nr, bytes, fx.seq_end.as<uint64_t>(), enc, rs);
+    return pack(bytes, fx.seq_end.as<uint64_t>());
   }
   // ---- the kept records' sequences, contiguous, then the common packing ----
   CU(fx.seq.ensure(seq_bytes + 32));
@@ -475,7 +488,7 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   CU(cudaGetLastError());
   std::swap(ctx->raw, fx.seq);
   std::swap(ctx->off_in, fx.rec_off);
-  return pack_set(ctx, nr, used, nullptr, enc, rs);
+  return pack(used, nullptr);
 }
 
 }  // namespace host
