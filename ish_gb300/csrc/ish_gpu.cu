@@ -568,7 +568,7 @@ int pack_set(ish_ctx *ctx, uint32_t n, uint64_t raw_bytes, const uint64_t *end, 
   ctx->raw_overlapped = raw_pending;
   if (raw_pending) CU(cudaStreamWaitEvent(s, ctx->raw_ev, 0));  // the records' bytes are on the device
   const uint32_t pb = pack_blocks(ctx, n, rs.total);
-  k_pack<<<pb, 256, 0, s>>>(ctx->raw.as<uint8_t>(), raw_bytes, ctx->off_in.as<uint64_t>(), end,
+  pack_fn(false)<<<pb, 256, 0, s>>>(ctx->raw.as<uint8_t>(), raw_bytes, ctx->off_in.as<uint64_t>(), end,
                             ctx->poff_tmp.as<uint64_t>(), n, rs.len_s.as<uint32_t>(), rs.orig_s.as<uint32_t>(),
                             max_bucket + 1, enc, rs.codes.as<uint8_t>(), summary, gw, 0);
   ++ctx->launches;
@@ -679,7 +679,7 @@ static int load_small(ish_ctx *ctx, const uint8_t *records, const uint64_t *offs
                                      rs.len_s.as<uint32_t>(), rs.off_s.as<uint64_t>(), rs.orig_s.as<uint32_t>(),
                                      long_counter, max_code);
   ++ctx->launches;
-  k_pack<<<pack_blocks(ctx, n, bytes), 256, 0, s>>>(
+  pack_fn(limit != 0)<<<pack_blocks(ctx, n, bytes), 256, 0, s>>>(
       ctx->raw.as<uint8_t>(), bytes, ctx->off_in.as<uint64_t>(), nullptr, ctx->poff_tmp.as<uint64_t>(), n,
       rs.len_s.as<uint32_t>(), rs.orig_s.as<uint32_t>(), long_counter, enc, rs.codes.as<uint8_t>(), max_code,
       pack_group(n, bytes), limit);

@@ -25,10 +25,11 @@ __global__ void k_scatter(const uint32_t *len, const uint64_t *poff, uint32_t n,
 constexpr uint32_t SORT_SMALL = 4096;    // records that k_sort_small takes
 __global__ void k_sort_small(uint64_t *off, uint32_t n, uint64_t base, uint64_t *poff, uint32_t *len_s,
                              uint64_t *off_s, uint32_t *orig_s, uint32_t *long_counter, uint32_t *max_code);
-__global__ void k_pack(const uint8_t *src, uint64_t src_bytes, const uint64_t *off, const uint64_t *end,
+typedef void (*PackFn)(const uint8_t *src, uint64_t src_bytes, const uint64_t *off, const uint64_t *end,
                        const uint64_t *poff, uint32_t n, const uint32_t *len_s, const uint32_t *orig_s,
                        uint32_t *long_counter, const uint8_t *enc, uint8_t *dst, uint32_t *max_code, uint32_t gw,
                        uint32_t limit);
+PackFn pack_fn(bool limited);
 __global__ void k_count_newlines(const uint8_t *text, uint64_t bytes, uint32_t *block_counts);
 // k_write_newlines<headers>: with headers, also the first '>' or '@' of every
 // line (hc, preset to all ones)
