@@ -19,8 +19,8 @@ seconds / 1e9 (ish's own definition, benchmarking/ish_bench_aligner.mojo:740-750
             left untouched by the CPU for 0.1-1 s was measured to upload at
             30-110 GB/s instead of 211 GB/s on some GB300 hosts.
   roofline  integer cell-update roofline: measured DPX add-max throughput x 2
-            cells per instruction / DPX instructions per cell pair (4 for
-            semi-global, 5 for local; 4.5 cell-weighted over the step).
+            cells per instruction / DPX instructions per cell pair (3 for
+            semi-global, 4 for local; 3.5 cell-weighted over the step).
   cpu_baseline / --impl reference: the CPU oracle (a restatement of ish's
             striped CPU matchers) on all host cores, on a bounded sample.
   parity    the timed step's scores, ends and hit flags compared with the
@@ -43,10 +43,11 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 # DPX add-max instructions per cell pair of the wavefront kernel (wave.cuh).
-# Local: T = max(Hdiag + P, E), u = max(T - open, 0), E = max(E - ext, u),
-# H = max(Fs - open, T), Fs = max(Fs - ext, T).  Semi-global holds its rows in
-# frames rising by ext per row, which folds u into the E update: four.
-INSTR_SG, INSTR_SW = 4, 5
+# Local: T = max(Hdiag + P, floor), H = max(T, E, F), E = max(E - ext, u),
+# F = max(F - ext, u); u = H - open is a plain add.  Semi-global holds its values
+# in frames rising by ext per row and column, which leaves H = max(T, E, F) and
+# two add-max with the same constant; T = Hdiag + P is a plain add: three.
+INSTR_SG, INSTR_SW = 3, 4
 
 
 def parse():
