@@ -1027,8 +1027,8 @@ __global__ void k_dpx_peak(uint32_t *out, int iters, uint32_t b, uint32_t c) {
 }
 
 // Local-alignment cell updates on packed lanes, for the lane-width choice of
-// the wavefront kernel.  U8 = false: two 16-bit lanes per word and the
-// wavefront kernel's five DPX add-max per word.  U8 = true: four 8-bit lanes
+// the wavefront kernel.  U8 = false: two 16-bit lanes per word and five DPX
+// add-max per word (the wavefront kernel needs four).  U8 = true: four 8-bit lanes
 // per word with a biased unsigned byte profile, as the reference's u8 pass
 // keeps it (local_aln/striped.mojo:78-139), through the saturating SIMD byte
 // intrinsics (add, subtract, max: ten per word).  Sixteen words of columns
