@@ -27,10 +27,11 @@ __global__ void k_invert(const uint32_t *orig_s, uint32_t n, uint32_t *inv) {
 }
 
 // Prefix length and 16-byte slot of every hit (the slot keeps at least one
-// zero byte past the prefix and is never empty).
+// zero byte past the prefix and is never empty).  No prefix is longer than
+// `most`, for which the host has made room.
 __global__ void k_rev_lengths(const uint32_t *hits, const int32_t *tend, uint32_t nh, const uint32_t *inv,
                               const uint32_t *len_s, uint32_t n, uint32_t *rlen, uint64_t *slot, uint32_t *orig,
-                              int32_t *rev_end, int *error) {
+                              int32_t *rev_end, int *error, uint64_t most) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nh; i += gridDim.x * blockDim.x) {
     const uint32_t h = hits[i];
     uint32_t r = 0;
@@ -39,6 +40,10 @@ __global__ void k_rev_lengths(const uint32_t *hits, const int32_t *tend, uint32_
       int64_t e = (int64_t)tend[i] + 1;
       e = e < 0 ? 0 : e;
       r = (uint32_t)(e < T ? e : T);
+      if (r > most) {
+        r = 0;
+        atomicOr(error, 4);
+      }
     } else {
       atomicOr(error, 4);
     }
@@ -120,12 +125,14 @@ extern "C" int ish_gpu_match_starts(ish_ctx *ctx, int32_t query_id, int32_t set_
   RecordSet &rs = *si_set;
   const uint32_t n = rs.n;
   // Bounds of the reversed prefixes' rows and bytes, from the ends alone (a row
-  // count is also at most its record's, which the device knows).
+  // count is also at most its record's, which the device knows; the host knows
+  // the longest record's, or, where the last length bucket holds some, the set's).
+  const uint64_t most = top_bucket(rs) == NBUCKETS - 1 ? std::min<uint64_t>(rs.total, 0xffffffffu) : rs.max_len;
   uint64_t bound = 0;
   uint32_t longest = 0;
   for (uint32_t i = 0; i < n_hits; ++i) {
     if (hit_idx[i] >= n) return fail(ctx, ISH_EINVAL, "hit index %u >= %u records", hit_idx[i], n);
-    const uint32_t r = (uint32_t)std::min<int64_t>(std::max<int64_t>((int64_t)target_end[i] + 1, 0), rs.max_len);
+    const uint32_t r = (uint32_t)std::min<int64_t>(std::max<int64_t>((int64_t)target_end[i] + 1, 0), (int64_t)most);
     longest = std::max(longest, r);
     bound += ((uint64_t)r + 16) & ~(uint64_t)15;
   }
@@ -202,7 +209,7 @@ extern "C" int ish_gpu_match_starts(ish_ctx *ctx, int32_t query_id, int32_t set_
     }
     const uint32_t hb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n_hits, 256), (uint32_t)ctx->num_sms * 8));
     k_rev_lengths<<<hb, 256, 0, s>>>(d_hits, d_tend, n_hits, rs.inv.as<uint32_t>(), rs.len_s.as<uint32_t>(), n, rlen,
-                                     slot, orig, rev_end, ctx->error.as<int>());
+                                     slot, orig, rev_end, ctx->error.as<int>(), most);
     ++ctx->launches;
     k_scan64_block<<<tiles, 1024, 0, s>>>(slot, poff, n_hits, bsum);
     ++ctx->launches;
