@@ -218,12 +218,12 @@ int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint
   CU(V.slot.ensure((size_t)nw * 4));
   CU(V.start.ensure((size_t)nw * 4));
   CU(V.cs.ensure((size_t)(nonempty + 1) * 4));
-  // (pageable sources: each call returns once its bytes are staged)
   CU(cudaMemcpyAsync(V.off.p, voff.data(), (size_t)nw * 8, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(V.len.p, vlen.data(), (size_t)nw * 4, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(V.slot.p, vslot.data(), (size_t)nw * 4, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(V.start.p, wstart.data(), (size_t)nw * 4, cudaMemcpyHostToDevice, s));
   CU(cudaMemcpyAsync(V.cs.p, cs.data(), (size_t)(nonempty + 1) * 4, cudaMemcpyHostToDevice, s));
+  CU(cudaStreamSynchronize(s));  // the arrays are temporaries
   V.W = W;
   V.O = O;
   V.entries = nonempty;
