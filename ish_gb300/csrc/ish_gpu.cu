@@ -715,7 +715,11 @@ int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, 
   if (bytes && !records) return fail(ctx, ISH_EINVAL, "records is NULL");
   rs.total = bytes;
   cudaStream_t s = stream ? stream : ctx->stream;
-  if (n <= SORT_SMALL) return load_small(ctx, records, offsets, n, rs, enc, s, defer, limit);
+  if (n <= SORT_SMALL) {
+    const int rc = load_small(ctx, records, offsets, n, rs, enc, s, defer, limit);
+    if (rc) cudaStreamSynchronize(s);  // the caller's buffers are free again on return
+    return rc;
+  }
   // The offsets go first on s; the records' bytes (+16 slack for the
   // realigning pack loads) follow on the copy stream once the offsets are in
   // (everything before this load on s, which includes the previous pack's
@@ -744,7 +748,10 @@ int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, 
   }
   if (base) CU(cudaEventSynchronize(ctx->off_ev));  // the rebased offsets are a temporary
   const int rc = pack_set(ctx, n, bytes, nullptr, enc, rs, s, defer, bytes != 0);
-  if (rc && bytes) cudaStreamSynchronize(ctx->copy_stream);
+  if (rc) {
+    cudaStreamSynchronize(ctx->copy_stream);
+    cudaStreamSynchronize(s);
+  }
   return rc;
 }
 

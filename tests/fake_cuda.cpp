@@ -33,6 +33,7 @@ struct Upload {
 std::vector<Upload> uploads;  // not waited for yet
 std::string report;
 bool refuse_func_attributes = false;
+int copies_to_go = -1;  // asynchronous copies that still succeed before one is refused (-1: all)
 dim3 grid_, block_;
 size_t shared_;
 cudaStream_t stream_;
@@ -139,6 +140,8 @@ extern "C" {
 
 __attribute__((visibility("default"))) const char *fake_report() { return report.c_str(); }
 __attribute__((visibility("default"))) void fake_refuse_func_attributes(int on) { refuse_func_attributes = on; }
+__attribute__((visibility("default"))) void fake_refuse_copy_after(int n) { copies_to_go = n; }
+__attribute__((visibility("default"))) int fake_unread_uploads() { return (int)uploads.size(); }
 
 void **__cudaRegisterFatBinary(void *) { return (void **)&perturb; }
 void __cudaRegisterFatBinaryEnd(void **) {}
@@ -189,6 +192,7 @@ cudaError_t cudaFreeHost(void *p) { return release(pinned, p); }
 
 cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t bytes, cudaMemcpyKind kind, cudaStream_t s) {
   std::lock_guard<std::recursive_mutex> lk(mu);
+  if (copies_to_go >= 0 && copies_to_go-- == 0) return cudaErrorInvalidValue;
   if (kind != cudaMemcpyDeviceToHost) touch("copy to the device", to, bytes);
   if (kind != cudaMemcpyHostToDevice) touch("copy from the device", from, bytes);
   if (kind == cudaMemcpyHostToDevice && !room(pinned, from))
