@@ -1139,11 +1139,13 @@ int run_scoring(ish_ctx *ctx, Query &q, RecordSet &rs) {
 }
 
 // max_code: the set's largest code where the host has not seen it yet (load_small
-// with a limit), checked against the query's alphabet; NULL else.
+// with a limit), checked against the query's alphabet before any output is
+// written: such a call's results are staged whether it wants the hits or not.
+// NULL else.
 int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32_t *tend, uint8_t *hit,
                   uint32_t *hit_idx, uint32_t *n_hits, const uint32_t *max_code = nullptr, int alphabet = 0) {
   cudaStream_t s = ctx->stream;
-  const bool compact = (hit_idx || n_hits) && n, staged = compact && n <= SORT_SMALL;
+  const bool compact = (hit_idx || n_hits || max_code) && n, staged = compact && n <= SORT_SMALL;
   CU(ctx->nhits.ensure(16));
   uint32_t *out3 = ctx->nhits.as<uint32_t>();  // hits, error flags, largest code
   if (compact) {
@@ -1180,8 +1182,8 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
   }
   CU(cudaEventRecord(ctx->ev1, s));
   // Results of a small call were written to pinned memory by the compaction;
-  // those of a larger one are copied: hit count, error flags and largest code go
-  // into pinned staging too, so that every copy stays asynchronous until the one
+  // those of a larger one are copied: hit count and error flags go into pinned
+  // staging too, so that every copy stays asynchronous until the one
   // synchronisation, and the first hit indices travel with the count (hit_idx
   // holds n entries, so the prefix fits whatever the count).
   uint32_t *hs = staged ? ctx->h_stage : reinterpret_cast<uint32_t *>(ctx->h_small);
@@ -1196,7 +1198,6 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
     if (compact) CU(cudaMemcpyAsync(hs, out3, 12, cudaMemcpyDeviceToHost, s));
     if (!compact || ceil_div(n, HIT_TILE) > 1024)
       CU(cudaMemcpyAsync(hs + 1, ctx->error.p, 4, cudaMemcpyDeviceToHost, s));
-    if (max_code && !(compact && n <= COMPACT_ONE)) CU(cudaMemcpyAsync(hs + 2, max_code, 4, cudaMemcpyDeviceToHost, s));
     if (hit_idx && compact) CU(cudaMemcpyAsync(hit_idx, ctx->hit_idx.p, (size_t)prefix * 4, cudaMemcpyDeviceToHost, s));
   }
   CU(cudaStreamSynchronize(s));
