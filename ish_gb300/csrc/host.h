@@ -263,8 +263,12 @@ struct ish_ctx {
 namespace ish {
 namespace host {
 
+// Formats the reason of a failure: into the context's error text, which belongs
+// to the thread that calls the library, or into thread_error on a thread of the
+// library's own that has set it.
 int fail(ish_ctx *c, int code, const char *fmt, ...);
 extern thread_local std::string g_open_error;
+extern thread_local std::string *thread_error;
 
 // Host wall time of a record-load call, kept for ish_gpu_last_load_ms.
 struct LoadTimer {

@@ -23,6 +23,7 @@ namespace ish {
 namespace host {
 
 thread_local std::string g_open_error;
+thread_local std::string *thread_error = nullptr;
 std::atomic<int64_t> g_alloc_fault{-1};
 
 int fail(ish_ctx *c, int code, const char *fmt, ...) {
@@ -31,7 +32,8 @@ int fail(ish_ctx *c, int code, const char *fmt, ...) {
   va_start(ap, fmt);
   vsnprintf(buf, sizeof buf, fmt, ap);
   va_end(ap);
-  if (c) c->err = buf;
+  if (thread_error) *thread_error = buf;
+  else if (c) c->err = buf;
   else g_open_error = buf;
   return code;
 }

@@ -212,7 +212,7 @@ int admit(Server &S, Request *r, char *msg, size_t) {
       // no layout: the lane-exact kernels score its chunks
       int rc = exact_prepare(S.ctx, r->q, S.max_chunk, S.exact);
       if (rc) {
-        snprintf(msg, 256, "exact kernel resources: %s", ish_gpu_last_error(S.ctx));
+        snprintf(msg, 256, "exact kernel resources: %s", thread_error->c_str());
         return rc;
       }
       r->exact = true;
@@ -265,7 +265,7 @@ int admit(Server &S, Request *r, char *msg, size_t) {
         const uint64_t Wv = std::max<uint64_t>(W, 8 * Ov);
         int rc = build_window_view(S.ctx, rs, nonempty, (Wv + 15) & ~15ull, Ov, v->V, S.s);
         if (rc) {
-          snprintf(msg, 256, "window view: %s", ish_gpu_last_error(S.ctx));
+          snprintf(msg, 256, "window view: %s", thread_error->c_str());
           return rc;
         }
         S.view = v;
@@ -373,7 +373,7 @@ int step(Server &S, char *msg) {
       }
       BatchLaunch launch;
       if (int rc = batch_launch(S.ctx, fn, C.K, C.mode, lean, C.prof_area, &launch)) {
-        snprintf(msg, 256, "%s", ish_gpu_last_error(S.ctx));
+        snprintf(msg, 256, "%s", thread_error->c_str());
         return rc;
       }
       BatchParams b{};
@@ -419,7 +419,7 @@ int step(Server &S, char *msg) {
       int rc = merge_windows(S.ctx, rs, rs.n - rs.n_empty, r->view->V, r->q, r->wscore.as<const int32_t>(),
                              r->wqend.as<const int32_t>(), r->wtend.as<const int32_t>(), out, s, nullptr);
       if (rc) {
-        snprintf(msg, 256, "window fold: %s", ish_gpu_last_error(S.ctx));
+        snprintf(msg, 256, "window fold: %s", thread_error->c_str());
         return rc;
       }
     }
@@ -499,6 +499,8 @@ void fail_all(Server &S, int rc, const char *msg) {
 
 void scheduler(Server *Sp) {
   Server &S = *Sp;
+  std::string why;  // of failures on this thread
+  thread_error = &why;
   cudaSetDevice(S.ctx->device);
   char msg[256];
   while (true) {

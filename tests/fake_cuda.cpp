@@ -18,6 +18,7 @@
 #include <mutex>
 #include <numeric>
 #include <string>
+#include <thread>
 #include <vector>
 
 namespace {
@@ -32,7 +33,8 @@ struct Upload {
 };
 std::vector<Upload> uploads;  // not waited for yet
 std::string report;
-bool refuse_func_attributes = false;
+bool refuse_func_attributes = false, refuse_other_threads = false;
+std::thread::id caller;  // where refuse_other_threads was set
 int copies_to_go = -1;  // asynchronous copies that still succeed before one is refused (-1: all)
 dim3 grid_, block_;
 size_t shared_;
@@ -121,6 +123,7 @@ void launch(const std::string &name, void **a) {
 
 cudaError_t alloc(std::map<const char *, size_t> &m, void **p, size_t bytes) {
   std::lock_guard<std::recursive_mutex> lk(mu);
+  if (refuse_other_threads && std::this_thread::get_id() != caller) return cudaErrorMemoryAllocation;
   *p = calloc(1, bytes);
   m[(const char *)*p] = bytes;
   return cudaSuccess;
@@ -146,6 +149,10 @@ extern "C" {
 
 __attribute__((visibility("default"))) const char *fake_report() { return report.c_str(); }
 __attribute__((visibility("default"))) void fake_refuse_func_attributes(int on) { refuse_func_attributes = on; }
+__attribute__((visibility("default"))) void fake_refuse_memory_to_other_threads(int on) {
+  refuse_other_threads = on;
+  caller = std::this_thread::get_id();
+}
 __attribute__((visibility("default"))) void fake_refuse_copy_after(int n) { copies_to_go = n; }
 __attribute__((visibility("default"))) int fake_unread_uploads() { return (int)uploads.size(); }
 
