@@ -97,7 +97,8 @@ extern "C" {
  * ISH_ETIMEDOUT -- the device-side bound every wavefront launch carries, made
  * to run out.  ISH_OPT_FAULT_ALLOC: n >= 0 makes the (n+1)-th device allocation
  * the library attempts from now on fail as if device memory were exhausted
- * (ISH_ENOMEM); it applies to every context of the process and disarms after
+ * (ISH_ENOMEM, where nothing kept between calls can be given back instead); it
+ * applies to every context of the process and disarms after
  * firing; -1 disarms it.  Neither changes results when left at its default. */
 #define ISH_OPT_STEP_BUDGET 11
 #define ISH_OPT_FAULT_ALLOC 12

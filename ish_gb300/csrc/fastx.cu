@@ -359,7 +359,7 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   if (!text) return fail(ctx, ISH_EINVAL, "text is NULL");
   cudaStream_t s = ctx->stream;
   FastxScratch &fx = ctx->fastx;
-  CU(ctx->raw.ensure(bytes + 32));
+  CU(grow(ctx, ctx->raw, bytes + 32));
   CU(cudaEventRecord(ctx->load_ev[0], s));
   CU(cudaMemcpyAsync(ctx->raw.p, text, bytes, cudaMemcpyHostToDevice, s));
   const uint8_t *dtext = ctx->raw.as<uint8_t>();
@@ -367,8 +367,8 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   const uint64_t tiles64 = (bytes + LINE_TILE - 1) / LINE_TILE;
   if (tiles64 > 0x7fffffffull) return fail(ctx, ISH_EINVAL, "text too large");
   const uint32_t btiles = (uint32_t)tiles64;
-  CU(ctx->block_counts.ensure((size_t)btiles * 4 + 8));
-  CU(ctx->nhits.ensure(16));
+  CU(grow(ctx, ctx->block_counts, (size_t)btiles * 4 + 8));
+  CU(grow(ctx, ctx->nhits, 16));
   k_count_newlines<<<btiles, 1024, 0, s>>>(dtext, bytes, ctx->block_counts.as<uint32_t>());
   ++ctx->launches;
   k_scan_counts<<<1, 1024, 0, s>>>(ctx->block_counts.as<uint32_t>(), btiles, ctx->nhits.as<uint32_t>());
@@ -381,17 +381,17 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   if (lines64 >= 0xfffff000ull) return fail(ctx, ISH_EINVAL, "too many lines (%llu)", (unsigned long long)lines64);
   const uint32_t n = (uint32_t)lines64;
   const uint32_t ltiles = ceil_div(n, FX_TILE);
-  CU(ctx->nl_pos.ensure((size_t)n_nl * 8 + 8));
-  CU(fx.hc.ensure((size_t)n * 8 + 8));
-  CU(fx.len.ensure((size_t)n * 8 + 8));
-  CU(fx.src.ensure((size_t)n * 8 + 8));
-  CU(fx.hdr.ensure((size_t)n * 8 + 8));
-  CU(fx.pos.ensure((size_t)n * 8 + 8));
-  CU(fx.rec.ensure((size_t)n * 8 + 8));
-  CU(fx.role.ensure((size_t)n + 16));
-  CU(fx.tiles.ensure((size_t)ltiles * 5 + 16));
-  CU(fx.scan.ensure(scan_u64_scratch(n)));
-  CU(fx.totals.ensure(64));
+  CU(grow(ctx, ctx->nl_pos, (size_t)n_nl * 8 + 8));
+  CU(grow(ctx, fx.hc, (size_t)n * 8 + 8));
+  CU(grow(ctx, fx.len, (size_t)n * 8 + 8));
+  CU(grow(ctx, fx.src, (size_t)n * 8 + 8));
+  CU(grow(ctx, fx.hdr, (size_t)n * 8 + 8));
+  CU(grow(ctx, fx.pos, (size_t)n * 8 + 8));
+  CU(grow(ctx, fx.rec, (size_t)n * 8 + 8));
+  CU(grow(ctx, fx.role, (size_t)n + 16));
+  CU(grow(ctx, fx.tiles, (size_t)ltiles * 5 + 16));
+  CU(grow(ctx, fx.scan, scan_u64_scratch(n)));
+  CU(grow(ctx, fx.totals, 64));
   CU(cudaMemsetAsync(fx.hc.p, 0xff, (size_t)n * 8 + 8, s));
   write_newlines_fn(true)<<<btiles, 1024, 0, s>>>(dtext, bytes, ctx->block_counts.as<uint32_t>(),
                                                   ctx->nl_pos.as<uint64_t>(), fx.hc.as<unsigned long long>());
@@ -414,11 +414,11 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   if (!rc) rc = scan_u64(ctx, fx.hdr.as<uint64_t>(), fx.rec.as<uint64_t>(), n, fx.scan);
   if (rc) return rc;
   // every line could be a header: size the record arrays for n + 1
-  CU(fx.rec_off.ensure((size_t)(n + 2) * 8));
-  CU(fx.bounds.ensure((size_t)(n + 1) * 32));
-  CU(fx.flags.ensure((size_t)(n + 1) * 4));
-  CU(fx.seq_start.ensure((size_t)(n + 1) * 8));
-  CU(fx.seq_end.ensure((size_t)(n + 1) * 8));
+  CU(grow(ctx, fx.rec_off, (size_t)(n + 2) * 8));
+  CU(grow(ctx, fx.bounds, (size_t)(n + 1) * 32));
+  CU(grow(ctx, fx.flags, (size_t)(n + 1) * 4));
+  CU(grow(ctx, fx.seq_start, (size_t)(n + 1) * 8));
+  CU(grow(ctx, fx.seq_end, (size_t)(n + 1) * 8));
   k_fx_totals<<<1, 1, 0, s>>>(n, fx.len.as<uint64_t>(), fx.pos.as<uint64_t>(), fx.hdr.as<uint64_t>(),
                               fx.rec.as<uint64_t>(), fx.rec_off.as<uint64_t>(), fx.totals.as<uint64_t>());
   ++ctx->launches;
@@ -480,7 +480,7 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
     return pack(bytes, fx.seq_end.as<uint64_t>());
   }
   // ---- the kept records' sequences, contiguous, then the common packing ----
-  CU(fx.seq.ensure(seq_bytes + 32));
+  CU(grow(ctx, fx.seq, seq_bytes + 32));
   const uint32_t gw = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div((uint64_t)n * 32, 256), (uint32_t)ctx->num_sms * 32));
   k_fx_gather<<<gw, 256, 0, s>>>(dtext, n, fx.role.as<uint8_t>(), fx.len.as<uint64_t>(), fx.src.as<uint64_t>(),
                                  fx.pos.as<uint64_t>(), fx.seq.as<uint8_t>());

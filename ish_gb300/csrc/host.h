@@ -293,6 +293,10 @@ struct LoadTimer {
     }                                                                                              \
   } while (0)
 
+// DevBuf::ensure for what loads and scoring allocate: when memory is short, what
+// start finding keeps between calls is given back first.
+cudaError_t grow(ish_ctx *ctx, DevBuf &b, size_t bytes);
+
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 int frame_rows(int ext);

@@ -61,8 +61,8 @@ void release_set(RecordSet &rs) {
 
 // Freed sets keep their device buffers for the next load: at most two sets,
 // each with packed codes under a sixteenth of device memory (at least 1 GiB),
-// so the cache stays small next to HBM; an allocation that fails gives the
-// cached buffers back first (pack_set).
+// so the cache stays small next to HBM; an allocation of codes that fails gives
+// the cached buffers back first (ensure_codes).
 static constexpr size_t kSpareSets = 2;
 static size_t spare_codes_max(const ish_ctx *ctx) { return std::max<size_t>(size_t(1) << 30, ctx->mem_total / 16); }
 
@@ -107,6 +107,32 @@ void take_spare_set(ish_ctx *ctx, RecordSet &rs, size_t codes_bytes) {
   rs.inv = sp.inv;
   rs.windows = sp.windows;
   ctx->spare_sets.erase(ctx->spare_sets.begin() + pick);
+}
+
+// Gives back start finding's buffers, and the window views and inverse orders of
+// freed sets; false where there were none.
+static bool give_back_starts(ish_ctx *ctx) {
+  WindowView &v = ctx->starts_windows;
+  size_t held = ctx->starts_ws.cap + ctx->starts_codes.cap + v.off.cap;
+  for (const RecordSet &sp : ctx->spare_sets) held += sp.inv.cap;
+  if (!held) return false;
+  ctx->starts_ws.release();
+  ctx->starts_codes.release();
+  v.release();
+  for (RecordSet &sp : ctx->spare_sets) {
+    sp.inv.release();
+    sp.windows.release();
+  }
+  return true;
+}
+
+cudaError_t grow(ish_ctx *ctx, DevBuf &b, size_t bytes) {
+  cudaError_t e = b.ensure(bytes);
+  if (e == cudaErrorMemoryAllocation && give_back_starts(ctx)) {
+    (void)cudaGetLastError();
+    e = b.ensure(bytes);
+  }
+  return e;
 }
 
 void compute_rows(Query &q) {
@@ -530,15 +556,15 @@ int pack_set(ish_ctx *ctx, uint32_t n, uint64_t raw_bytes, const uint64_t *end, 
   rs.n = n;
   const uint32_t tiles = ceil_div(n, SCAN_TILE);
   if (tiles > SCAN_TILE) return fail(ctx, ISH_EINVAL, "too many records in one set (%u)", n);
-  CU(ctx->len_tmp.ensure((size_t)n * 4));
-  CU(ctx->poff_tmp.ensure((size_t)n * 8));
-  CU(ctx->scan_tmp.ensure((size_t)tiles * 8));
+  CU(grow(ctx, ctx->len_tmp, (size_t)n * 4));
+  CU(grow(ctx, ctx->poff_tmp, (size_t)n * 8));
+  CU(grow(ctx, ctx->scan_tmp, (size_t)tiles * 8));
   // counts [NBUCKETS], descending cursors [NBUCKETS], the largest bucket and
   // the pack's long-record counter
-  CU(ctx->hist.ensure((size_t)NBUCKETS * 4 * 2 + 16));
+  CU(grow(ctx, ctx->hist, (size_t)NBUCKETS * 4 * 2 + 16));
   uint32_t *counts = ctx->hist.as<uint32_t>(), *cursor = counts + NBUCKETS, *max_bucket = cursor + NBUCKETS;
   // what the host reads back: largest code, largest bucket, counts
-  CU(ctx->summary.ensure((size_t)(2 + NBUCKETS) * 4));
+  CU(grow(ctx, ctx->summary, (size_t)(2 + NBUCKETS) * 4));
   uint32_t *summary = ctx->summary.as<uint32_t>();
   CU(cudaEventRecord(ctx->load_ev[1], s));
   if (ctx->pack_dirty) {  // first load, or the last one stopped before k_scatter cleared the accumulators
@@ -556,9 +582,9 @@ int pack_set(ish_ctx *ctx, uint32_t n, uint64_t raw_bytes, const uint64_t *end, 
   ++ctx->launches;
   const uint64_t packed = rs.total + 16ull * n + 16;
   take_spare_set(ctx, rs, packed);
-  CU(rs.len_s.ensure((size_t)n * 4));
-  CU(rs.off_s.ensure((size_t)n * 8));
-  CU(rs.orig_s.ensure((size_t)n * 4));
+  CU(grow(ctx, rs.len_s, (size_t)n * 4));
+  CU(grow(ctx, rs.off_s, (size_t)n * 8));
+  CU(grow(ctx, rs.orig_s, (size_t)n * 4));
   k_scatter<<<ceil_div(n, 1024), 1024, 0, s>>>(ctx->len_tmp.as<uint32_t>(), ctx->poff_tmp.as<uint64_t>(), n, cursor,
                                                rs.len_s.as<uint32_t>(), rs.off_s.as<uint64_t>(),
                                                rs.orig_s.as<uint32_t>(), counts, max_bucket, summary);
@@ -625,10 +651,10 @@ static uint32_t length_bucket(uint64_t len) {
   return (uint32_t)std::min<uint64_t>(32768 + ((len - 32768) >> 5), NBUCKETS - 1);
 }
 
-// Allocates the codes of a set, giving the cached buffers of freed sets back
-// first when memory is short.
+// Allocates the codes of a set, giving the cached buffers of freed sets back too
+// when memory is short.
 static cudaError_t ensure_codes(ish_ctx *ctx, RecordSet &rs, size_t bytes) {
-  cudaError_t e = rs.codes.ensure(bytes);
+  cudaError_t e = grow(ctx, rs.codes, bytes);
   if (e == cudaErrorMemoryAllocation && !ctx->spare_sets.empty()) {
     (void)cudaGetLastError();
     for (RecordSet &sp : ctx->spare_sets) release_set(sp);
@@ -660,14 +686,14 @@ static int load_small(ish_ctx *ctx, const uint8_t *records, const uint64_t *offs
   rs.max_code = 0;
   const uint64_t packed = bytes + 16ull * n + 16;
   take_spare_set(ctx, rs, packed);
-  CU(ctx->raw.ensure(bytes + 32));
-  CU(ctx->off_in.ensure((size_t)(n + 1) * 8));
-  CU(ctx->poff_tmp.ensure((size_t)n * 8));
-  CU(ctx->hist.ensure((size_t)NBUCKETS * 4 * 2 + 16));
-  CU(ctx->summary.ensure((size_t)(2 + NBUCKETS) * 4));
-  CU(rs.len_s.ensure((size_t)n * 4));
-  CU(rs.off_s.ensure((size_t)n * 8));
-  CU(rs.orig_s.ensure((size_t)n * 4));
+  CU(grow(ctx, ctx->raw, bytes + 32));
+  CU(grow(ctx, ctx->off_in, (size_t)(n + 1) * 8));
+  CU(grow(ctx, ctx->poff_tmp, (size_t)n * 8));
+  CU(grow(ctx, ctx->hist, (size_t)NBUCKETS * 4 * 2 + 16));
+  CU(grow(ctx, ctx->summary, (size_t)(2 + NBUCKETS) * 4));
+  CU(grow(ctx, rs.len_s, (size_t)n * 4));
+  CU(grow(ctx, rs.off_s, (size_t)n * 8));
+  CU(grow(ctx, rs.orig_s, (size_t)n * 4));
   CU(ensure_codes(ctx, rs, packed));
   uint32_t *long_counter = ctx->hist.as<uint32_t>() + 2 * NBUCKETS + 1, *max_code = ctx->summary.as<uint32_t>();
   CU(cudaEventRecord(ctx->load_ev[0], s));
@@ -727,8 +753,8 @@ int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, 
   // (everything before this load on s, which includes the previous pack's
   // reads of the same buffer, is before that point too), while s computes
   // lengths, packed offsets and sorted positions.
-  CU(ctx->raw.ensure(bytes + 32));
-  CU(ctx->off_in.ensure((size_t)(n + 1) * 8));
+  CU(grow(ctx, ctx->raw, bytes + 32));
+  CU(grow(ctx, ctx->off_in, (size_t)(n + 1) * 8));
   CU(cudaEventRecord(ctx->load_ev[0], s));
   std::vector<uint64_t> rebased;
   if (base) {
@@ -804,14 +830,14 @@ int load_lines(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   if (bytes == 0) return ISH_OK;
   if (!text) return fail(ctx, ISH_EINVAL, "text is NULL");
   cudaStream_t s = ctx->stream;
-  CU(ctx->raw.ensure(bytes + 32));
+  CU(grow(ctx, ctx->raw, bytes + 32));
   CU(cudaEventRecord(ctx->load_ev[0], s));
   CU(cudaMemcpyAsync(ctx->raw.p, text, bytes, cudaMemcpyHostToDevice, s));
   const uint64_t tiles64 = (bytes + LINE_TILE - 1) / LINE_TILE;
   if (tiles64 > 0x7fffffffull) return fail(ctx, ISH_EINVAL, "text too large");
   const uint32_t tiles = (uint32_t)tiles64;
-  CU(ctx->block_counts.ensure((size_t)tiles * 4 + 8));
-  CU(ctx->nhits.ensure(16));
+  CU(grow(ctx, ctx->block_counts, (size_t)tiles * 4 + 8));
+  CU(grow(ctx, ctx->nhits, 16));
   k_count_newlines<<<tiles, 1024, 0, s>>>(ctx->raw.as<uint8_t>(), bytes, ctx->block_counts.as<uint32_t>());
   ++ctx->launches;
   k_scan_counts<<<1, 1024, 0, s>>>(ctx->block_counts.as<uint32_t>(), tiles, ctx->nhits.as<uint32_t>());
@@ -824,9 +850,9 @@ int load_lines(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
   const uint64_t lines = (uint64_t)n_nl + (last != '\n' ? 1 : 0);
   if (lines >= 0xffffffffull) return fail(ctx, ISH_EINVAL, "too many lines (%llu)", (unsigned long long)lines);
   const uint32_t n = (uint32_t)lines;
-  CU(ctx->nl_pos.ensure((size_t)n_nl * 8 + 8));
-  CU(ctx->off_in.ensure((size_t)(n + 1) * 8));
-  CU(ctx->line_end.ensure((size_t)n * 8 + 8));
+  CU(grow(ctx, ctx->nl_pos, (size_t)n_nl * 8 + 8));
+  CU(grow(ctx, ctx->off_in, (size_t)(n + 1) * 8));
+  CU(grow(ctx, ctx->line_end, (size_t)n * 8 + 8));
   write_newlines_fn(false)<<<tiles, 1024, 0, s>>>(ctx->raw.as<uint8_t>(), bytes, ctx->block_counts.as<uint32_t>(),
                                                   ctx->nl_pos.as<uint64_t>(), nullptr);
   ++ctx->launches;
@@ -862,12 +888,12 @@ uint32_t count_longer(const RecordSet &rs, uint64_t len) {
 }
 
 int ensure_outputs(ish_ctx *ctx, uint32_t n) {
-  CU(ctx->out_score.ensure((size_t)n * 4 + 4));
-  CU(ctx->out_qend.ensure((size_t)n * 4 + 4));
-  CU(ctx->out_tend.ensure((size_t)n * 4 + 4));
-  CU(ctx->out_hit.ensure((size_t)n + 16));
-  CU(ctx->counter.ensure(64));
-  CU(ctx->error.ensure(64));
+  CU(grow(ctx, ctx->out_score, (size_t)n * 4 + 4));
+  CU(grow(ctx, ctx->out_qend, (size_t)n * 4 + 4));
+  CU(grow(ctx, ctx->out_tend, (size_t)n * 4 + 4));
+  CU(grow(ctx, ctx->out_hit, (size_t)n + 16));
+  CU(grow(ctx, ctx->counter, 64));
+  CU(grow(ctx, ctx->error, 64));
   return ISH_OK;
 }
 
@@ -1148,11 +1174,11 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
                   uint32_t *hit_idx, uint32_t *n_hits, const uint32_t *max_code = nullptr, int alphabet = 0) {
   cudaStream_t s = ctx->stream;
   const bool compact = (hit_idx || n_hits || max_code) && n, staged = compact && n <= SORT_SMALL;
-  CU(ctx->nhits.ensure(16));
+  CU(grow(ctx, ctx->nhits, 16));
   uint32_t *out3 = ctx->nhits.as<uint32_t>();  // hits, error flags, largest code
   if (compact) {
     const uint32_t nb = ceil_div(n, HIT_TILE);
-    CU(ctx->hit_idx.ensure((size_t)n * 4 + 4));
+    CU(grow(ctx, ctx->hit_idx, (size_t)n * 4 + 4));
     const uint8_t *flags = ctx->out_hit.as<uint8_t>();
     if (n <= COMPACT_ONE) {
       StageOut stage;
@@ -1167,7 +1193,7 @@ int fetch_outputs(ish_ctx *ctx, uint32_t n, int32_t *score, int32_t *qend, int32
                                        stage);
       ++ctx->launches;
     } else {
-      CU(ctx->block_counts.ensure((size_t)nb * 4 + 8));
+      CU(grow(ctx, ctx->block_counts, (size_t)nb * 4 + 8));
       uint32_t *counts = ctx->block_counts.as<uint32_t>();
       k_count_hits<<<nb, 1024, 0, s>>>(flags, n, counts);
       ++ctx->launches;

@@ -98,6 +98,8 @@ void launch(const std::string &name, void **a) {
       *arg<uint32_t *>(a, 11) = std::max<uint32_t>(*arg<uint32_t *>(a, 11), arg<uint8_t *>(a, 0)[i]);
   } else if (is("k_compact_one")) {  // the head of its results alone
     uint32_t *out = *(uint32_t **)a[6] ? *(uint32_t **)a[6] : arg<uint32_t *>(a, 5);
+    out[0] = 0;
+    out[1] = *arg<uint32_t *>(a, 3);
     out[2] = arg<uint32_t *>(a, 4) ? *arg<uint32_t *>(a, 4) : 0;
   } else if (is("k_invert")) {
     for (uint32_t e = 0; e < arg<uint32_t>(a, 1); ++e) arg<uint32_t *>(a, 2)[arg<uint32_t *>(a, 0)[e]] = e;
