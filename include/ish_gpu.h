@@ -196,7 +196,8 @@ ISH_API int ish_gpu_records_load_lines(ish_ctx *ctx, const uint8_t *text, uint64
  *     name [bounds[4i], bounds[4i+1]) (the header line after its '>'/'@',
  *     as the reader keeps it), quality [bounds[4i+2], bounds[4i+3]) (both 0
  *     for a FASTA record).  If more than bounds_cap records are read the call
- *     fails with ISH_EOVERFLOW and loads nothing.
+ *     fails with ISH_EOVERFLOW, loads nothing and sets *n_records to the number
+ *     of records there are.
  * A FASTQ quality that continues on the next line (legal for kseq, which
  * reads quality lines until the quality is as long as the sequence) is not
  * split on the device: ISH_EINVAL. */

@@ -449,10 +449,10 @@ int load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes, RecordSet &rs,
                 (unsigned long long)(first_stop >> 1));
   if (keep > 0xffffffffull) return fail(ctx, ISH_EINVAL, "too many records (%llu)", (unsigned long long)keep);
   const uint32_t nr = (uint32_t)keep;
+  *n_out = nr;
   if (bounds_out && nr > bounds_cap)
     return fail(ctx, ISH_EOVERFLOW, "%u records, bounds capacity %llu", nr, (unsigned long long)bounds_cap);
   rs.total = used;
-  *n_out = nr;
   if (nr == 0) return ISH_OK;
   // The records are packed while the bounds, final since the wait above, are
   // copied to the caller's array: filling pageable memory takes the host longer
@@ -513,6 +513,7 @@ int ish_gpu_records_load_fastx(ish_ctx *ctx, const uint8_t *text, uint64_t bytes
   if (rc) {
     cudaStreamSynchronize(ctx->stream);
     release_set(rs);
+    if (rc == ISH_EOVERFLOW && n_records) *n_records = n;
     return rc;
   }
   const int32_t id = ctx->next_set++;

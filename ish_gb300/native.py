@@ -293,18 +293,17 @@ class Context:
         n = C.c_uint32()
         # every record needs a header line: at most one record per newline + 1.
         # Counting them took longer than the whole load, so the room is
-        # estimated from a sample, and counted where the text overflows it
-        # (a failed call loads nothing).
+        # estimated from a sample; where the text overflows it, the failed call
+        # (which loads nothing) has counted the records on the device.
         room = _line_room(buf) if bounds else 0
         while True:
             bnd = np.empty((room, 4), np.uint64) if bounds else None
             rc = self._L.ish_gpu_records_load_fastx(
                 self._h, _p(buf, C.c_uint8) if len(buf) else None, len(buf), matrix_kind, C.byref(sid), C.byref(n),
                 _p(bnd, C.c_uint64) if bounds else None, room)
-            most = int(np.count_nonzero(buf == 10)) + 1 if rc == EOVERFLOW else 0
-            if rc != EOVERFLOW or room >= most:
+            if rc != EOVERFLOW or n.value <= room:
                 break
-            room = most
+            room = n.value
         self._check(rc)
         return sid.value, n.value, (bnd[:n.value] if bounds else None)
 
