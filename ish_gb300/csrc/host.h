@@ -326,7 +326,7 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
 uint64_t tune_key(int mode, int alphabet, int Q);
 int layout_stride(int layout, int K);
 size_t layout_bytes(int layout, int alphabet, int G, int K);
-int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode);
+int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode, int ends);
 int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayout **out);
 int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, uint32_t n, RecordSet &rs,
                  const uint8_t *enc, cudaStream_t s = nullptr, bool defer = false, uint32_t limit = 0);

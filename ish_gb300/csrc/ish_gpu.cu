@@ -343,13 +343,22 @@ static int wave_fit_threads(size_t prof_area, int K, int mode, int lean) {
 // 100,000 proteins 7,440 with the 160 KB 32-bit profile, 6,600 with 16-bit words;
 // 1,900 residues, local, where 96 of 256 threads fit beside the 32-bit profile,
 // 3,165 against 4,670 with 16-bit words.
-int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode) {
+// With a free query end every thread copies its row to local memory where a
+// record ends, and wide groups on short records do little else: the copies have
+// to stay in the L1 that the profile leaves of 256 KB.  160,000 reads of 150 nt,
+// 32 threads, pair / 32-bit profile: 44 columns (208 KB with the copies) 7.2 /
+// 7.9 ms, 48 (240) 10.4 / 8.6, 60 (253) 14.6 / 13.1, 64 (281) 31.4 / 14.0.
+// 120,000 proteins, 32-bit / 16-bit: 56 (241) 16.4 / 17.0, 60 (245) 17.6 / 17.6,
+// 62 (271) 28.9 / 18.1.
+int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode, int ends) {
   const int lean = wave_lean(ctx, K, mode), all = wave_sm_threads(K, lean);
-  auto fit = [&](int layout) {
-    return wave_fit_threads(((layout_bytes(layout, rows, G, K) + 15) & ~(size_t)15) + 256, K, mode, lean);
+  const size_t copies = mode == SG && (ends & ISH_FREE_QUERY_END) ? (size_t)all * K * 4 : 0;
+  auto fit = [&](int layout, size_t most) {
+    const size_t prof = ((layout_bytes(layout, rows, G, K) + 15) & ~(size_t)15) + 256;
+    return copies && prof + copies > most * 1024 ? 0 : wave_fit_threads(prof, K, mode, lean);
   };
-  if (fit(PROF_PAIR) == all) return PROF_PAIR;
-  if (4 * fit(PROF_S32) >= 3 * all) return PROF_S32;
+  if (fit(PROF_PAIR, 224) == all) return PROF_PAIR;
+  if (4 * fit(PROF_S32, 246) >= 3 * all) return PROF_S32;
   return PROF_S16;
 }
 
@@ -364,11 +373,11 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
   if (!ctx->force_G && !ctx->force_K && ctx->force_layout < 0 && it != ctx->tuned.end()) {
     *G = it->second.G;
     *K = it->second.K;
-    *layout = it->second.layout >= 0 ? it->second.layout : choose_layout(ctx, q.rows, *G, *K, mode);
+    *layout = it->second.layout >= 0 ? it->second.layout : choose_layout(ctx, q.rows, *G, *K, mode, q.ends);
     return;
   }
   auto layout_of = [&](int g, int k) {
-    return ctx->force_layout >= 0 ? ctx->force_layout : (g ? choose_layout(ctx, q.rows, g, k, mode) : (int)PROF_S16);
+    return ctx->force_layout >= 0 ? ctx->force_layout : (g ? choose_layout(ctx, q.rows, g, k, mode, q.ends) : (int)PROF_S16);
   };
   choose_shape(ctx, mode, q.Q, nullptr, 1, G, K);
   *layout = layout_of(*G, *K);

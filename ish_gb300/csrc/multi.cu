@@ -531,7 +531,7 @@ int ish_gpu_autotune(ish_ctx *ctx, int32_t set_id, const int32_t *query_ids, uin
         // the layout rule's pick, and the 16/32-bit alternative to it (the
         // 32-bit profile saves an ALU instruction per column but can cost
         // occupancy)
-        const int pick = choose_layout(ctx, q.rows, g, k, mode);
+        const int pick = choose_layout(ctx, q.rows, g, k, mode, q.ends);
         cands.push_back({g, k, pick, m});
         const int other = pick == PROF_S32 ? PROF_S16 : (pick == PROF_S16 ? PROF_S32 : -1);
         if (other >= 0 && wave_fits(q, g, k, other)) cands.push_back({g, k, other, m});

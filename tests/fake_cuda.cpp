@@ -32,7 +32,7 @@ struct Upload {
   std::string bytes;  // the source when the copy was asked for
 };
 std::vector<Upload> uploads;  // not waited for yet
-std::string report;
+std::string report, wave;  // wave: the last wavefront kernel launched
 bool refuse_func_attributes = false, refuse_other_threads = false;
 std::thread::id caller;  // where refuse_other_threads was set
 int copies_to_go = -1;  // asynchronous copies that still succeed before one is refused (-1: all)
@@ -79,6 +79,7 @@ uint64_t bucket(uint64_t len) { return len < 32768 ? len : std::min<uint64_t>(32
 
 void launch(const std::string &name, void **a) {
   auto is = [&](const char *k) { return name.find(k) != std::string::npos; };
+  if (is("wave_kernel") || is("batch_kernel")) wave = name;
   if (is("k_sort_small")) {
     const uint64_t *off = arg<uint64_t *>(a, 0);
     const uint32_t n = arg<uint32_t>(a, 1);
@@ -150,6 +151,7 @@ cudaError_t handle(T *p) {
 extern "C" {
 
 __attribute__((visibility("default"))) const char *fake_report() { return report.c_str(); }
+__attribute__((visibility("default"))) const char *fake_last_wave() { return wave.c_str(); }
 __attribute__((visibility("default"))) void fake_refuse_func_attributes(int on) { refuse_func_attributes = on; }
 __attribute__((visibility("default"))) void fake_refuse_memory_to_other_threads(int on) {
   refuse_other_threads = on;

@@ -13,14 +13,18 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 
 PRELUDE = """
 import ctypes as C
+import re
 import sys
 import numpy as np
 sys.path[:0] = [{root!r}, {here!r}]
 from ish_gb300 import build, native
 build.LIB = {lib!r}
 fake = C.CDLL({lib!r})
-fake.fake_report.restype = C.c_char_p
+fake.fake_report.restype = fake.fake_last_wave.restype = C.c_char_p
 ctx = native.Context(0)
+def last_wave():
+    "(columns per thread, mode, layout, lean build) of the last wavefront kernel"
+    return tuple(map(int, re.search(rb"_kernelILi(\\d+)ELi(\\d)ELi(\\d)ELi(\\d)E", fake.fake_last_wave()).groups()))
 """
 
 
