@@ -336,8 +336,12 @@ static int wave_fit_threads(size_t prof_area, int K, int mode, int lean) {
 
 // The pair layout (no per-column work to assemble a record pair's word, half
 // the shared-memory loads of the 32-bit one) while all of an SM's threads fit
-// beside it; else 32-bit single-code words under the same rule; else 16-bit
-// words, whose PRMT per column costs what up to a quarter of the warps do.
+// beside it; else 32-bit single-code words: for semi-global while three quarters
+// of them do, for local alignment while all do; else 16-bit words, whose PRMT per
+// column costs semi-global what up to a quarter of the warps do and local
+// alignment next to nothing (32 threads on 120,000 proteins, 32-bit / 16-bit: 52
+// columns 16.4 / 16.8 ms with all threads beside both, 56 columns 22.4 / 18.0
+// with three quarters beside the first).
 // Measured: 1,000 nt x 200,000 reads, semi-global, 7,820 GCUPS with the 115 KB
 // pair profile, 6,920 with 32-bit words, 5,930 with 16-bit ones; 1,501 residues x
 // 100,000 proteins 7,440 with the 160 KB 32-bit profile, 6,600 with 16-bit words;
@@ -358,7 +362,7 @@ int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode, int ends
     return copies && prof + copies > most * 1024 ? 0 : wave_fit_threads(prof, K, mode, lean);
   };
   if (fit(PROF_PAIR, 224) == all) return PROF_PAIR;
-  if (4 * fit(PROF_S32, 246) >= 3 * all) return PROF_S32;
+  if (4 * fit(PROF_S32, 246) >= (mode == SG ? 3 : 4) * all) return PROF_S32;
   return PROF_S16;
 }
 
