@@ -302,6 +302,10 @@ inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1)
 int frame_rows(int ext);
 int wave_lean(const ish_ctx *ctx, int K, int mode);
 double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps);
+// Build of the wavefront kernel for a shape and a set (scored by `share` queries
+// at once), and the modelled clocks with it.
+int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share);
+double shape_time(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share);
 uint64_t window_overlap(const Query &q);
 int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, OutDev out, cudaStream_t s, bool *done);
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode);
@@ -326,6 +330,7 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
 uint64_t tune_key(int mode, int alphabet, int Q);
 int layout_stride(int layout, int K);
 size_t layout_bytes(int layout, int alphabet, int G, int K);
+int profile_slots(int layout, int alphabet, int G, int K);
 int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode, int ends);
 int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayout **out);
 int load_records(ish_ctx *ctx, const uint8_t *records, const uint64_t *offsets, uint32_t n, RecordSet &rs,

@@ -218,41 +218,85 @@ int neg_limit_of(int open, int mmin) {
 // Scheduler clocks of one warp-row (one row of 32 / G record pairs) with the
 // warps of a full SM taking turns, and of one row of a warp that has its
 // scheduler to itself (the chain of its columns, shuffles and loads).  Straight
-// lines through measurements at G = 8, proteins, K = 4..64 (semi-global 87 at K =
-// 4, 180 at 16, 326 at 32, 384 at 38, 631 at 60; local 184, 258, 468, 561, 941;
-// alone 451 / 752 at K = 32, 619 / 1,074 at 48), with what the builds with fewer
-// warps add, and wide groups (32 threads 9 % at K = 16..32 on proteins: most
+// lines through measurements at G = 8 and 16, proteins, K = 4..64 (semi-global 87
+// at K = 4, 180 at 16, 326 at 32, 384 at 38, 631 at 60; local 184, 258, 468, 561,
+// 1,032; alone 451 / 752 at K = 32, 619 / 1,074 at 48), with what the builds with
+// fewer warps add, and wide groups (32 threads 9 % at K = 16..32 on proteins: most
 // steps of a warp start a pair in one of its threads).
-static double warp_row_clocks(int mode, int K, int G) {
-  const double wide = 1.0 + 0.1 * (G / 32.0) * (G / 32.0);
-  if (mode == SG) return (50 + 8.6 * K) * (K > 48 ? 1.1 : 1.0) * wide;
-  return (50 + 13.3 * K) * (K > 40 ? 1.08 : 1.0) * wide;
+// `lean` is the build; where the other one is the usual choice (wave_lean), it
+// costs what 120,000 proteins at G = 16 and 32 showed (semi-global 2-7 % up to K =
+// 32, 7-12 % above; local 10 % at K = 34..38, level at 40; the default build of
+// K = 42..48 5 % to 1.6x).
+static double warp_row_clocks(const ish_ctx *ctx, int mode, int K, int G, int lean) {
+  double c = 1.0 + 0.1 * (G / 32.0) * (G / 32.0);
+  if (mode == SG) c *= (50 + 8.6 * K) * (K > 48 ? 1.1 : 1.0);
+  else c *= (50 + 13.3 * K) * (K > 48 ? 1.11 + 0.02 * std::max(0, K - 56) : K > 40 ? 1.08 : 1.0);
+  if (lean == wave_lean(ctx, K, mode)) return c;
+  if (!lean) return c * (K <= 32 ? 1.04 : G < 32 ? 1.08 : 1.3);
+  return c * (mode == SG ? (K <= 32 ? 1.05 : 1.1) : K <= 26 ? 1.02 : K < 40 ? 1.1 : 1.0);
 }
 static double lone_row_clocks(int mode, int K) { return mode == SG ? 150 + 9.5 * K : 200 + 17.5 * K; }
 
 // Warps per scheduler of a full SM, by the kernels' launch bounds.
-static double full_warps(int K) { return K <= 32 ? 4 : K <= 48 ? 3 : 2; }
+static double full_warps(int K, int lean) { return wave_sm_threads(K, lean) / 128; }
 
 // Clocks in which each of `warps` warps on the device advances by one row: from
 // one warp per scheduler to a full SM about linear (K = 32: 451 alone, 740 with
 // two, 1,300 with four).
+static double build_row_clocks(const ish_ctx *ctx, int mode, int K, int lean, double warps, double full_row) {
+  const double w = std::max(1.0, warps / (4.0 * ctx->num_sms)), cap = full_warps(K, lean), lone = lone_row_clocks(mode, K);
+  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * full_row - lone);
+}
 double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps) {
-  const double w = std::max(1.0, warps / (4.0 * ctx->num_sms)), cap = full_warps(K), lone = lone_row_clocks(mode, K);
-  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * warp_row_clocks(mode, K, G) - lone);
+  const int lean = wave_lean(ctx, K, mode);
+  return build_row_clocks(ctx, mode, K, lean, warps, warp_row_clocks(ctx, mode, K, G, lean));
 }
 
-// Modelled time of one query against `set` (null: many records of any length)
-// with G threads x K columns: every warp's share of the rows at the rate of the
-// warps in flight, or the longest pair alone, whichever takes longer.  `share`
-// queries run at once.
-static double shape_clocks(const ish_ctx *ctx, int mode, int G, int K, const RecordSet *set, double share) {
-  if (!set) return G * warp_row_clocks(mode, K, G);
-  const double pairs = std::max(1.0, (set->n - set->n_empty) / 2.0) * share, rows = set->total / 2.0 * share;
-  const double full = 4.0 * ctx->num_sms * full_warps(K);
-  const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), full));
-  const double all = rows * G / 32 / warps * row_clocks(ctx, mode, K, G, warps);
-  const double last = ((double)set->max_len + 4 * G) * row_clocks(ctx, mode, K, G, 1);
-  return std::max(all, last) + 0.1 * all;
+// Modelled time of one query against `set` (null: many records) with G threads x
+// K columns: every group's share of the rows at the rate of the warps in flight,
+// then what the longest pair has left, alone (it ran at the same rate as the
+// others until then).  `share` queries run at once; `rows` is the profile's.
+// Groups narrower than a quarter-warp also pay for the pairs that the other
+// groups of their warp begin and end (160,000 reads of 150: 32 groups per warp
+// 115 clocks a row more than four, 16 groups 45, eight 11; local half as much
+// again), and, with too large a profile to repeat their slices (profile_slots),
+// for bank conflicts (proteins, four threads: 849 -> 1,261 clocks at K = 52 -> 54,
+// local 1,260 -> 1,564).  Of 590 measured times (3,000 to 200,000 proteins, 40 to
+// 2,047 residues, every shape and build without windows) the model is off by 6 %
+// (standard deviation; 13 % with the longest pair taken to run alone from the
+// start), and the shape it takes is 0.3 % slower than the best, at most 8 %.
+static double shape_clocks(const ish_ctx *ctx, const Query &q, int G, int K, int layout, int lean, const RecordSet *set,
+                           double share) {
+  const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
+  const double n = set ? std::max(1.0, (double)set->n - set->n_empty) : 0, length = set ? std::max(1.0, set->total / n) : 350;
+  double row = warp_row_clocks(ctx, mode, K, G, lean);
+  if (G < 8) {
+    row += (mode == SG ? 500 : 750) * (32 / G - 4) / length;
+    if (profile_slots(layout, q.rows, G, K) < 8) row *= mode == SG ? 1.55 : 1.2;
+  }
+  if (!set) return G * row;
+  const double pairs = std::max(1.0, n / 2) * share, rows = set->total / 2.0 * share;
+  const double full = 4.0 * ctx->num_sms * full_warps(K, lean);
+  const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), full)), each = rows * G / 32 / warps;
+  return each * build_row_clocks(ctx, mode, K, lean, warps, row) +
+         std::max(0.0, (double)set->max_len + 4 * G - each) * lone_row_clocks(mode, K);
+}
+
+// The build for a shape and a set.  Where all pairs are in flight at once in the
+// build with fewer warps, the other one has no more of them, and fewer registers
+// (3,000 proteins: 2 % behind to 23 % ahead at K = 25..46); else the one with the
+// smaller modelled time: with fewer warps the longest pairs run faster (15,000
+// proteins, 32 threads x 32 columns: 1,376 us with 512 threads per SM, 1,222 with
+// 384).
+int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share) {
+  const int usual = wave_lean(ctx, K, q.algo == ISH_ALGO_LOCAL ? SW : SG);
+  if (!set || !wave_has_lean(K) || ctx->force_lean >= 0) return usual;
+  if ((set->n - set->n_empty) / 2.0 * share * G / 32 <= 4.0 * ctx->num_sms * full_warps(K, 1)) return 1;
+  return shape_clocks(ctx, q, G, K, layout, !usual, set, share) < 0.97 * shape_clocks(ctx, q, G, K, layout, usual, set, share)
+             ? !usual : usual;
+}
+double shape_time(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share) {
+  return shape_clocks(ctx, q, G, K, layout, lean_for(ctx, q, G, K, layout, set, share), set, share);
 }
 
 // Columns per thread (K) and threads per group (G) with the smallest modelled
@@ -260,15 +304,20 @@ static double shape_clocks(const ish_ctx *ctx, int mode, int G, int K, const Rec
 // K up to 64.
 int wave_k_available(int k) { return (k >= 1 && k <= 32) || (k > 32 && k <= WAVE_KMAX && !(k & 1)); }
 
-static void choose_shape(const ish_ctx *ctx, int mode, int Q, const RecordSet *set, double share, int *G, int *K) {
+static int shape_layout(const ish_ctx *ctx, const Query &q, int G, int K) {
+  if (ctx->force_layout >= 0) return ctx->force_layout;
+  return G ? choose_layout(ctx, q.rows, G, K, q.algo == ISH_ALGO_LOCAL ? SW : SG, q.ends) : (int)PROF_S16;
+}
+
+static void choose_shape(const ish_ctx *ctx, const Query &q, const RecordSet *set, double share, int *G, int *K) {
   double bestc = 1e30;
   int bg = 0, bk = 0;
   for (int g = 1; g <= 32; g <<= 1) {
     if (ctx->force_G && g != ctx->force_G) continue;
-    int k = ctx->force_K ? ctx->force_K : (Q + 1 + g - 1) / g;
+    int k = ctx->force_K ? ctx->force_K : (q.Q + 1 + g - 1) / g;
     if (!ctx->force_K && k > 32) k = (k + 1) & ~1;
-    if (!wave_k_available(k) || g * k < Q + 1) continue;
-    const double c = shape_clocks(ctx, mode, g, k, set, share);
+    if (!wave_k_available(k) || g * k < q.Q + 1) continue;
+    const double c = shape_time(ctx, q, g, k, shape_layout(ctx, q, g, k), set, share);
     if (c < bestc) {
       bestc = c;
       bg = g;
@@ -377,24 +426,22 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
   if (!ctx->force_G && !ctx->force_K && ctx->force_layout < 0 && it != ctx->tuned.end()) {
     *G = it->second.G;
     *K = it->second.K;
-    *layout = it->second.layout >= 0 ? it->second.layout : choose_layout(ctx, q.rows, *G, *K, mode, q.ends);
+    *layout = it->second.layout >= 0 ? it->second.layout : shape_layout(ctx, q, *G, *K);
     return;
   }
-  auto layout_of = [&](int g, int k) {
-    return ctx->force_layout >= 0 ? ctx->force_layout : (g ? choose_layout(ctx, q.rows, g, k, mode, q.ends) : (int)PROF_S16);
-  };
-  choose_shape(ctx, mode, q.Q, nullptr, 1, G, K);
-  *layout = layout_of(*G, *K);
+  choose_shape(ctx, q, nullptr, 1, G, K);
+  *layout = shape_layout(ctx, q, *G, *K);
   if (!set || !*G) return;
   int g = 0, k = 0;
-  choose_shape(ctx, mode, q.Q, set, share, &g, &k);
-  // (within a tenth the model does not tell shapes apart)
-  if (!g || shape_clocks(ctx, mode, g, k, set, share) > 0.9 * shape_clocks(ctx, mode, *G, *K, set, share)) return;
+  choose_shape(ctx, q, set, share, &g, &k);
+  const int l = shape_layout(ctx, q, g, k);
+  // (closer than that the model does not tell shapes apart)
+  if (!g || shape_time(ctx, q, g, k, l, set, share) > 0.97 * shape_time(ctx, q, *G, *K, *layout, set, share)) return;
   const Regime r = regime(q, g * k);
-  if (!r.fast || set->max_len > r.max_safe_len || !wave_fits(q, g, k, layout_of(g, k))) return;
+  if (!r.fast || set->max_len > r.max_safe_len || !wave_fits(q, g, k, l)) return;
   *G = g;
   *K = k;
-  *layout = layout_of(g, k);
+  *layout = l;
 }
 
 int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayout **out) {
@@ -976,7 +1023,7 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
   int rc = build_wave_layout(ctx, q, G, K, layout, &L);
   if (rc) return rc;
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
-  const int lean = wave_lean(ctx, K, mode);
+  const int lean = lean_for(ctx, q, G, K, L->layout, &rs, 1);
   WaveFn fn = wave_fn(K, mode, L->layout, lean);
   if (!fn) return fail(ctx, ISH_EOVERFLOW, "no wavefront kernel for K=%d", K);
   {

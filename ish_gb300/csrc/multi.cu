@@ -209,7 +209,8 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
 
   // ---- per class: kernel, occupancy, parameters, tiles ----
   for (MultiClass &c : P.classes) {
-    const int lean = wave_lean(ctx, c.K, c.mode);
+    const Member &m0 = *std::find_if(members.begin(), members.end(), [&](const Member &x) { return x.pos == c.members[0]; });
+    const int lean = lean_for(ctx, ctx->queries.at(qids[m0.pos]), m0.G, c.K, c.layout, windowed[m0.pos] ? &view : &rs, nq);
     c.fn = batch_fn(c.K, c.mode, c.layout, lean);
     if (!c.fn) return fail(ctx, ISH_EOVERFLOW, "no batch kernel for K=%d", c.K);
     BatchLaunch launch;

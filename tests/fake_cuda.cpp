@@ -77,23 +77,45 @@ T arg(void **a, int i) {
 
 uint64_t bucket(uint64_t len) { return len < 32768 ? len : std::min<uint64_t>(32768 + ((len - 32768) >> 5), 65535); }
 
+// The longest first, equal lengths in record order.
+void sort_records(const uint32_t *len, const uint64_t *pos, uint32_t n, uint32_t *len_s, uint64_t *off_s, uint32_t *orig_s) {
+  std::iota(orig_s, orig_s + n, 0u);
+  std::stable_sort(orig_s, orig_s + n, [&](uint32_t x, uint32_t y) { return bucket(len[x]) > bucket(len[y]); });
+  for (uint32_t e = 0; e < n; ++e) {
+    len_s[e] = len[orig_s[e]];
+    off_s[e] = pos[orig_s[e]];
+  }
+}
+
 void launch(const std::string &name, void **a) {
   auto is = [&](const char *k) { return name.find(k) != std::string::npos; };
   if (is("wave_kernel") || is("batch_kernel")) wave = name;
   if (is("k_sort_small")) {
     const uint64_t *off = arg<uint64_t *>(a, 0);
     const uint32_t n = arg<uint32_t>(a, 1);
+    std::vector<uint32_t> len(n);
     std::vector<uint64_t> pos(n);
-    std::vector<uint32_t> order(n);
-    std::iota(order.begin(), order.end(), 0u);
-    for (uint32_t i = 1; i < n; ++i) pos[i] = pos[i - 1] + ((off[i] - off[i - 1] + 15) & ~15ull);
-    std::stable_sort(order.begin(), order.end(),
-                     [&](uint32_t x, uint32_t y) { return bucket(off[x + 1] - off[x]) > bucket(off[y + 1] - off[y]); });
-    for (uint32_t e = 0; e < n; ++e) {
-      arg<uint32_t *>(a, 4)[e] = (uint32_t)(off[order[e] + 1] - off[order[e]]);
-      arg<uint64_t *>(a, 5)[e] = pos[order[e]];
-      arg<uint32_t *>(a, 6)[e] = order[e];
+    for (uint32_t i = 0; i < n; ++i) len[i] = (uint32_t)(off[i + 1] - off[i]);
+    for (uint32_t i = 1; i < n; ++i) pos[i] = pos[i - 1] + ((len[i - 1] + 15) & ~15ull);
+    sort_records(len.data(), pos.data(), n, arg<uint32_t *>(a, 4), arg<uint64_t *>(a, 5), arg<uint32_t *>(a, 6));
+  } else if (is("k_lengths")) {
+    const uint64_t *off = arg<uint64_t *>(a, 0), *end = arg<uint64_t *>(a, 1);
+    for (uint32_t i = 0; i < arg<uint32_t>(a, 2); ++i)
+      arg<uint32_t *>(a, 3)[i] = (uint32_t)((end ? end[i] : off[i + 1]) - off[i]);
+    arg<uint32_t *>(a, 7)[0] = 0;
+  } else if (is("k_scan_slots")) {
+    uint64_t sum = 0;
+    for (uint32_t i = 0; i < arg<uint32_t>(a, 1); ++i) {
+      arg<uint64_t *>(a, 3)[i] = sum;
+      sum += (arg<uint32_t *>(a, 0)[i] + 15) & ~15ull;
     }
+  } else if (is("k_scatter")) {
+    const uint32_t n = arg<uint32_t>(a, 2);
+    uint32_t *len_s = arg<uint32_t *>(a, 4), *summary = arg<uint32_t *>(a, 9);
+    sort_records(arg<uint32_t *>(a, 0), arg<uint64_t *>(a, 1), n, len_s, arg<uint64_t *>(a, 5), arg<uint32_t *>(a, 6));
+    std::fill(summary + 2, summary + 2 + 65536, 0u);
+    for (uint32_t e = 0; e < n; ++e) ++summary[2 + bucket(len_s[e])];
+    summary[1] = (uint32_t)bucket(len_s[0]);
   } else if (is("k_pack")) {  // the largest code alone
     for (uint64_t i = 0; i < arg<uint64_t>(a, 1); ++i)
       *arg<uint32_t *>(a, 11) = std::max<uint32_t>(*arg<uint32_t *>(a, 11), arg<uint8_t *>(a, 0)[i]);
