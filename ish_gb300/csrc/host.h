@@ -112,7 +112,8 @@ struct WindowView {
   uint64_t W = 0, O = 0;      // window stride and overlap (rows)
   uint32_t entries = 0;       // sorted entries covered
   uint32_t nw = 0;            // windows (slots)
-  uint32_t n_first = 0;       // view entries [0, n_first) start at record row 0, the rest later
+  bool split = false;         // the windows at record row 0 first (else longest first)
+  uint32_t n_first = 0;       // with split, view entries [0, n_first) start at record row 0, the rest later
   uint64_t total = 0;         // rows over all windows
   uint32_t max_len = 0;
   DevBuf off, len, slot;      // per view entry (longest first): code offset, rows, slot
@@ -309,8 +310,8 @@ double shape_time(const ish_ctx *ctx, const Query &q, int G, int K, int layout, 
 uint64_t window_overlap(const Query &q);
 int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, OutDev out, cudaStream_t s, bool *done);
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode);
-int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint64_t W, uint64_t O, WindowView &V,
-                      cudaStream_t s);
+int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint64_t W, uint64_t O, bool split,
+                      WindowView &V, cudaStream_t s);
 RecordSet window_set(const RecordSet &rs, const WindowView &V);
 int merge_windows(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, const WindowView &V, const Query &q,
                   const int32_t *ws, const int32_t *wq, const int32_t *wt, OutDev out, cudaStream_t s,

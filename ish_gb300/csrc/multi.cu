@@ -172,7 +172,7 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
     }
     if (W) {
       W = std::max(W, 8 * O);  // the queries of the launch fill each other's tails: few repeated rows
-      int rc = build_window_view(ctx, rs, nonempty, W, O, P.view, ctx->stream);
+      int rc = build_window_view(ctx, rs, nonempty, W, O, false, P.view, ctx->stream);
       if (rc) return rc;
       for (const Member &m : members) {
         const Query &q = ctx->queries.at(qids[m.pos]);

@@ -263,7 +263,7 @@ int admit(Server &S, Request *r, char *msg, size_t) {
         auto v = std::make_shared<SharedView>();
         const uint64_t Ov = S.view ? std::max<uint64_t>(O, S.view->V.O) : O;
         const uint64_t Wv = std::max<uint64_t>(W, 8 * Ov);
-        int rc = build_window_view(S.ctx, rs, nonempty, (Wv + 15) & ~15ull, Ov, v->V, S.s);
+        int rc = build_window_view(S.ctx, rs, nonempty, (Wv + 15) & ~15ull, Ov, false, v->V, S.s);
         if (rc) {
           snprintf(msg, 256, "window view: %s", thread_error->c_str());
           return rc;

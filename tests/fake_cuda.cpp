@@ -32,7 +32,8 @@ struct Upload {
   std::string bytes;  // the source when the copy was asked for
 };
 std::vector<Upload> uploads;  // not waited for yet
-std::string report, wave;  // wave: the last wavefront kernel launched
+std::string report, wave;             // wave: the last wavefront kernel launched
+std::vector<std::string> contents;  // of the asynchronous uploads from pageable memory
 bool refuse_func_attributes = false, refuse_other_threads = false;
 std::thread::id caller;  // where refuse_other_threads was set
 int copies_to_go = -1;  // asynchronous copies that still succeed before one is refused (-1: all)
@@ -174,6 +175,12 @@ extern "C" {
 
 __attribute__((visibility("default"))) const char *fake_report() { return report.c_str(); }
 __attribute__((visibility("default"))) const char *fake_last_wave() { return wave.c_str(); }
+// Bytes of upload i from the last (0), to `to` if given.
+__attribute__((visibility("default"))) size_t fake_upload(size_t i, char *to) {
+  const std::string &c = contents[contents.size() - 1 - i];
+  if (to) memcpy(to, c.data(), c.size());
+  return c.size();
+}
 __attribute__((visibility("default"))) void fake_refuse_func_attributes(int on) { refuse_func_attributes = on; }
 __attribute__((visibility("default"))) void fake_refuse_memory_to_other_threads(int on) {
   refuse_other_threads = on;
@@ -235,7 +242,8 @@ cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t bytes, cudaMemcpy
   if (kind != cudaMemcpyDeviceToHost) touch("copy to the device", to, bytes);
   if (kind != cudaMemcpyHostToDevice) touch("copy from the device", from, bytes);
   if (kind == cudaMemcpyHostToDevice && !room(pinned, from))
-    uploads.push_back(Upload{s, (const char *)from, std::string((const char *)from, bytes)});
+    uploads.push_back(Upload{s, (const char *)from, std::string((const char *)from, bytes)}),
+        contents.push_back(uploads.back().bytes);
   memmove(to, from, bytes);
   return cudaSuccess;
 }
