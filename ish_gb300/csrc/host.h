@@ -114,6 +114,7 @@ struct WindowView {
   uint32_t nw = 0;            // windows (slots)
   bool split = false;         // the windows at record row 0 first (else longest first)
   uint32_t n_first = 0;       // with split, view entries [0, n_first) start at record row 0, the rest later
+  uint32_t multi = 0;         // entries up to the last one of several windows
   uint64_t total = 0;         // rows over all windows
   uint32_t max_len = 0;
   DevBuf off, len, slot;      // per view entry (longest first): code offset, rows, slot

@@ -45,25 +45,42 @@
 
 namespace ish {
 
-// One thread per sorted entry: fold the entry's window results (slots
-// [cs[e], cs[e+1]), window w starting at record row start[w]) into its outputs.
-__global__ void k_merge_windows(const uint32_t *orig_s, uint32_t n, const uint32_t *cs, const uint32_t *start,
-                                const int32_t *ws, const int32_t *wq, const int32_t *wt, int mode, OutDev out,
-                                Decision dec) {
-  for (uint32_t e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+// Folds the window results of sorted entries (entry e: slots [cs[e], cs[e+1]),
+// window w starting at record row start[w]) into their outputs: a warp for each
+// of the first `multi` entries, a thread for each of the others, which are one
+// window.  (With a thread for every entry, 60 records of 10 kb - 400 kb in 25,600
+// windows of a 20-nt query took about 500 us to fold, 52 so; scoring them 76.)
+__global__ void k_merge_windows(const uint32_t *orig_s, uint32_t n, uint32_t multi, const uint32_t *cs,
+                                const uint32_t *start, const int32_t *ws, const int32_t *wq, const int32_t *wt,
+                                int mode, OutDev out, Decision dec) {
+  const uint32_t lane = threadIdx.x & 31, items = multi + (n - multi + 31) / 32;
+  for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < items; i += (gridDim.x * blockDim.x) >> 5) {
+    const bool whole = i < multi;
+    const uint32_t e = whole ? i : multi + (i - multi) * 32 + lane;
+    if (e >= n) continue;
     const uint32_t a = cs[e], b = cs[e + 1];
-    int bs = ws[a], bq = wq[a];
-    long long bt = wt[a] >= 0 ? (long long)wt[a] + start[a] : -1;
-    for (uint32_t w = a + 1; w < b; ++w) {
-      const int sc = ws[w], tq = wq[w];
-      const long long tt = wt[w] >= 0 ? (long long)wt[w] + start[w] : -1;
-      // equal scores carry rows of the same kind (all -1 when nothing beat
-      // the initial best), so the row and column order the ties
-      if (sc > bs || (sc == bs && tt >= 0 && (tt < bt || (tt == bt && tq < bq)))) {
-        bs = sc;
-        bq = tq;
-        bt = tt;
+    bool any = false;
+    int bs = 0, bq = 0;
+    long long bt = -1;
+    // equal scores carry rows of the same kind (all -1 when nothing beat the
+    // initial best), so the row and column order the ties
+    auto take = [&](int sc, int tq, long long tt) {
+      if (any && !(sc > bs || (sc == bs && tt >= 0 && (tt < bt || (tt == bt && tq < bq))))) return;
+      any = true;
+      bs = sc;
+      bq = tq;
+      bt = tt;
+    };
+    for (uint32_t w = whole ? a + lane : a; w < b; w += whole ? 32 : 1)
+      take(ws[w], wq[w], wt[w] >= 0 ? (long long)wt[w] + start[w] : -1);
+    if (whole) {
+      for (int o = 16; o > 0; o >>= 1) {
+        const bool has = __shfl_down_sync(0xffffffffu, any, o);
+        const int sc = __shfl_down_sync(0xffffffffu, bs, o), tq = __shfl_down_sync(0xffffffffu, bq, o);
+        const long long tt = __shfl_down_sync(0xffffffffu, bt, o);
+        if (has) take(sc, tq, tt);
       }
+      if (lane) continue;
     }
     const uint32_t o = orig_s[e];
     if (out.score) out.score[o] = bs;
@@ -174,6 +191,7 @@ int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint
   // record row, a length and a code offset
   std::vector<uint32_t> cs(nonempty + 1), wstart, wlen;
   std::vector<uint64_t> woff;
+  V.multi = 0;
   for (uint32_t e = 0; e < nonempty; ++e) {
     cs[e] = (uint32_t)wstart.size();
     const uint64_t L = len[e];
@@ -183,6 +201,7 @@ int build_window_view(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, uint
       woff.push_back(off[e]);
       continue;
     }
+    V.multi = e + 1;
     // window k covers [k * W, (k + 1) * W + O): the cells it adds to the windows
     // before it lie O rows or more below its start
     for (uint64_t st = 0;; st += W) {
@@ -257,8 +276,9 @@ int merge_windows(ish_ctx *ctx, const RecordSet &rs, uint32_t nonempty, const Wi
                   const int32_t *ws, const int32_t *wq, const int32_t *wt, OutDev out, cudaStream_t s,
                   uint32_t *kernels) {
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
-  const uint32_t nb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(nonempty, 256), (uint32_t)ctx->num_sms * 8));
-  k_merge_windows<<<nb, 256, 0, s>>>(rs.orig_s.as<const uint32_t>(), nonempty, V.cs.as<const uint32_t>(),
+  const uint64_t warps = V.multi + ceil_div(nonempty - V.multi, 32);
+  const uint32_t nb = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(warps * 32, 256), (uint32_t)ctx->num_sms * 8));
+  k_merge_windows<<<nb, 256, 0, s>>>(rs.orig_s.as<const uint32_t>(), nonempty, V.multi, V.cs.as<const uint32_t>(),
                                      V.start.as<const uint32_t>(), ws, wq, wt, mode, out,
                                      Decision{q.max_score, q.thr});
   if (kernels)
