@@ -305,9 +305,8 @@ int frame_rows(int ext);
 int wave_lean(const ish_ctx *ctx, int K, int mode);
 double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps);
 // Build of the wavefront kernel for a shape and a set (scored by `share` queries
-// at once), and the modelled clocks with it.
+// at once).
 int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share);
-double shape_time(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share);
 uint64_t window_overlap(const Query &q);
 int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, OutDev out, cudaStream_t s, bool *done);
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode);

@@ -243,60 +243,91 @@ static double full_warps(int K, int lean) { return wave_sm_threads(K, lean) / 12
 // Clocks in which each of `warps` warps on the device advances by one row: from
 // one warp per scheduler to a full SM about linear (K = 32: 451 alone, 740 with
 // two, 1,300 with four).
-static double build_row_clocks(const ish_ctx *ctx, int mode, int K, int lean, double warps, double full_row) {
-  const double w = std::max(1.0, warps / (4.0 * ctx->num_sms)), cap = full_warps(K, lean), lone = lone_row_clocks(mode, K);
-  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * full_row - lone);
+static double build_row_clocks(const ish_ctx *ctx, int K, int lean, double warps, double full, double lone) {
+  const double w = std::max(1.0, warps / (4.0 * ctx->num_sms)), cap = full_warps(K, lean);
+  return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * full - lone);
 }
 double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps) {
   const int lean = wave_lean(ctx, K, mode);
-  return build_row_clocks(ctx, mode, K, lean, warps, warp_row_clocks(ctx, mode, K, G, lean));
+  return build_row_clocks(ctx, K, lean, warps, warp_row_clocks(ctx, mode, K, G, lean), lone_row_clocks(mode, K));
 }
 
 // Modelled time of one query against `set` (null: many records) with G threads x
-// K columns: every group's share of the rows at the rate of the warps in flight,
-// then what the longest pair has left, alone (it ran at the same rate as the
-// others until then).  `share` queries run at once; `rows` is the profile's.
-// Groups narrower than a quarter-warp also pay for the pairs that the other
-// groups of their warp begin and end (160,000 reads of 150: 32 groups per warp
-// 115 clocks a row more than four, 16 groups 45, eight 11; local half as much
-// again), and, with too large a profile to repeat their slices (profile_slots),
-// for bank conflicts (proteins, four threads: 849 -> 1,261 clocks at K = 52 -> 54,
-// local 1,260 -> 1,564).  Of 590 measured times (3,000 to 200,000 proteins, 40 to
-// 2,047 residues, every shape and build without windows) the model is off by 6 %
-// (standard deviation; 13 % with the longest pair taken to run alone from the
-// start), and the shape it takes is 0.3 % slower than the best, at most 8 %.
-static double shape_clocks(const ish_ctx *ctx, const Query &q, int G, int K, int layout, int lean, const RecordSet *set,
-                           double share) {
+// K columns and a build: every group's share of the rows at the rate of the warps
+// in flight, then what the longest pair has left, alone (it ran at the same rate
+// as the others until then), and the group's last thread, 4 rows behind each
+// before it.  `share` queries run at once.  Four costs come on top of a row:
+//   - in local alignment, the ends of records shorter than proteins (reads of 150
+//     against proteins: 28 to 40 clocks at K = 8, 49 to 65 at 24, 62 at 40, 102 at
+//     56);
+//   - in groups narrower than a quarter-warp, the pairs that the other groups of
+//     the warp begin and end (reads of 150: 32 groups per warp 115 clocks more than
+//     four, 16 groups 45, eight 11; local half as much again);
+//   - there, with too large a profile to repeat their slices (profile_slots), bank
+//     conflicts (proteins, four threads: 849 -> 1,261 clocks at K = 52 -> 54, local
+//     1,260 -> 1,564);
+//   - with a free query end, the steps taken row by row while a record's end goes
+//     through the group (reads of 150, K = 24: 40 clocks for eight threads, 77 for
+//     16, 162 for 32; proteins 29 for 16, 57 for 32).
+// Of 500 measured times (3,000 to 200,000 proteins, 20 to 2,047 residues, every
+// shape and build without windows) the model is off by 6 % (standard deviation; 13
+// % with the longest pair taken to run alone from the start), and the shape it
+// takes is 0.2 % slower than the best, at most 8 %.
+struct ShapeCost {
+  double each = 0, clocks = 0;  // rows of a group; modelled clocks
+};
+static ShapeCost shape_cost(const ish_ctx *ctx, const Query &q, int G, int K, int layout, int lean, const RecordSet *set,
+                            double share) {
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
   const double n = set ? std::max(1.0, (double)set->n - set->n_empty) : 0, length = set ? std::max(1.0, set->total / n) : 350;
-  double row = warp_row_clocks(ctx, mode, K, G, lean);
-  if (G < 8) {
-    row += (mode == SG ? 500 : 750) * (32 / G - 4) / length;
-    if (profile_slots(layout, q.rows, G, K) < 8) row *= mode == SG ? 1.55 : 1.2;
+  double more = mode == SW ? 260 * (40 + K) * std::max(0.0, 1 / length - 1 / 350.0) : 0.0, times = 1;
+  if (mode == SG && (q.ends & ISH_FREE_QUERY_END)) more = (150 + 28 * K) * std::min(0.25, G / length);
+  const double narrow = G < 8 ? (mode == SG ? 500 : 750) * (32 / G - 4) / length : 0.0;
+  if (G < 8 && profile_slots(layout, q.rows, G, K) < 8) times = mode == SG ? 1.55 : 1.2;
+  const double row = (warp_row_clocks(ctx, mode, K, G, lean) + more + narrow) * times;
+  ShapeCost c;
+  if (!set) {
+    c.clocks = G * row;
+    return c;
   }
-  if (!set) return G * row;
+  const double lone = (lone_row_clocks(mode, K) + more) * times;
   const double pairs = std::max(1.0, n / 2) * share, rows = set->total / 2.0 * share;
-  const double full = 4.0 * ctx->num_sms * full_warps(K, lean);
-  const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), full)), each = rows * G / 32 / warps;
-  return each * build_row_clocks(ctx, mode, K, lean, warps, row) +
-         std::max(0.0, (double)set->max_len + 4 * G - each) * lone_row_clocks(mode, K);
+  const double warps = std::max(1.0, std::min(std::ceil(pairs * G / 32), 4.0 * ctx->num_sms * full_warps(K, lean)));
+  c.each = rows * G / 32 / warps;
+  c.clocks = c.each * build_row_clocks(ctx, K, lean, warps, row, lone) +
+             (std::max(0.0, (double)set->max_len - c.each) + 4 * G) * lone;
+  return c;
 }
 
-// The build for a shape and a set.  Where all pairs are in flight at once in the
-// build with fewer warps, the other one has no more of them, and fewer registers
-// (3,000 proteins: 2 % behind to 23 % ahead at K = 25..46); else the one with the
-// smaller modelled time: with fewer warps the longest pairs run faster (15,000
-// proteins, 32 threads x 32 columns: 1,376 us with 512 threads per SM, 1,222 with
-// 384).
-int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share) {
+// The build for a shape and a set, and the modelled clocks with it.  Where all
+// pairs are in flight at once in the build with fewer warps, the other one has no
+// more of them, and fewer registers (3,000 proteins: 2 % behind to 23 % ahead at K
+// = 25..46).  Else, where the longest pair has much more than its share of the
+// rows, the one with the smaller modelled time: with fewer warps that pair runs
+// faster (15,000 proteins, 32 threads x 32 columns: 1,376 us with 512 threads per
+// SM, 1,222 with 384).
+static double shape_clocks(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share,
+                           int *build = nullptr) {
   const int usual = wave_lean(ctx, K, q.algo == ISH_ALGO_LOCAL ? SW : SG);
-  if (!set || !wave_has_lean(K) || ctx->force_lean >= 0) return usual;
-  if ((set->n - set->n_empty) / 2.0 * share * G / 32 <= 4.0 * ctx->num_sms * full_warps(K, 1)) return 1;
-  return shape_clocks(ctx, q, G, K, layout, !usual, set, share) < 0.97 * shape_clocks(ctx, q, G, K, layout, usual, set, share)
-             ? !usual : usual;
+  ShapeCost c = shape_cost(ctx, q, G, K, layout, usual, set, share);
+  int lean = usual;
+  if (set && wave_has_lean(K) && ctx->force_lean < 0) {
+    const bool all = (set->n - set->n_empty) / 2.0 * share * G / 32 <= 4.0 * ctx->num_sms * full_warps(K, 1);
+    if (all ? !usual : set->max_len > 1.5 * c.each) {
+      const ShapeCost o = shape_cost(ctx, q, G, K, layout, !usual, set, share);
+      if (all || o.clocks < 0.97 * c.clocks) {
+        c = o;
+        lean = !usual;
+      }
+    }
+  }
+  if (build) *build = lean;
+  return c.clocks;
 }
-double shape_time(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share) {
-  return shape_clocks(ctx, q, G, K, layout, lean_for(ctx, q, G, K, layout, set, share), set, share);
+int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share) {
+  int lean = 0;
+  shape_clocks(ctx, q, G, K, layout, set, share, &lean);
+  return lean;
 }
 
 // Columns per thread (K) and threads per group (G) with the smallest modelled
@@ -310,6 +341,10 @@ static int shape_layout(const ish_ctx *ctx, const Query &q, int G, int K) {
 }
 
 static void choose_shape(const ish_ctx *ctx, const Query &q, const RecordSet *set, double share, int *G, int *K) {
+  // Of shapes that the model does not tell apart a launch for several queries takes
+  // the widest group: near-equal queries then have the same columns, and one kernel
+  // (six of 26 to 31 nt against 1,000 lines 99 -> 77 us).
+  const double same = set && share > 1 ? 1.04 : 1.0;
   double bestc = 1e30;
   int bg = 0, bk = 0;
   for (int g = 1; g <= 32; g <<= 1) {
@@ -317,9 +352,9 @@ static void choose_shape(const ish_ctx *ctx, const Query &q, const RecordSet *se
     int k = ctx->force_K ? ctx->force_K : (q.Q + 1 + g - 1) / g;
     if (!ctx->force_K && k > 32) k = (k + 1) & ~1;
     if (!wave_k_available(k) || g * k < q.Q + 1) continue;
-    const double c = shape_time(ctx, q, g, k, shape_layout(ctx, q, g, k), set, share);
-    if (c < bestc) {
-      bestc = c;
+    const double c = shape_clocks(ctx, q, g, k, shape_layout(ctx, q, g, k), set, share);
+    if (c < bestc * same) {
+      bestc = std::min(c, bestc);
       bg = g;
       bk = k;
     }
@@ -378,9 +413,9 @@ static constexpr size_t WAVE_SMEM_MAX = 226 * 1024;
 // Threads of the largest block of this shape that fits beside the profile: all
 // the SM's registers allow, or fewer where their saved rows do not fit.
 static int wave_fit_threads(size_t prof_area, int K, int mode, int lean) {
-  int t = wave_sm_threads(K, lean);
-  while (t > 0 && wave_smem(prof_area, t, K, mode) > WAVE_SMEM_MAX) t -= 32;
-  return t;
+  if (prof_area > WAVE_SMEM_MAX) return 0;
+  const size_t warp = wave_smem(0, 32, K, mode);
+  return (int)std::min<size_t>(wave_sm_threads(K, lean), (WAVE_SMEM_MAX - prof_area) / warp * 32);
 }
 
 // The pair layout (no per-column work to assemble a record pair's word, half
@@ -436,7 +471,7 @@ void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const
   choose_shape(ctx, q, set, share, &g, &k);
   const int l = shape_layout(ctx, q, g, k);
   // (closer than that the model does not tell shapes apart)
-  if (!g || shape_time(ctx, q, g, k, l, set, share) > 0.97 * shape_time(ctx, q, *G, *K, *layout, set, share)) return;
+  if (!g || shape_clocks(ctx, q, g, k, l, set, share) > 0.97 * shape_clocks(ctx, q, *G, *K, *layout, set, share)) return;
   const Regime r = regime(q, g * k);
   if (!r.fast || set->max_len > r.max_safe_len || !wave_fits(q, g, k, l)) return;
   *G = g;
