@@ -283,7 +283,10 @@ static ShapeCost shape_cost(const ish_ctx *ctx, const Query &q, int G, int K, in
   double more = mode == SW ? 260 * (40 + K) * std::max(0.0, 1 / length - 1 / 350.0) : 0.0, times = 1;
   if (mode == SG && (q.ends & ISH_FREE_QUERY_END)) more = (150 + 28 * K) * std::min(0.25, G / length);
   const double narrow = G < 8 ? (mode == SG ? 500 : 750) * (32 / G - 4) / length : 0.0;
-  if (G < 8 && profile_slots(layout, q.rows, G, K) < 8) times = mode == SG ? 1.55 : 1.2;
+  if (G < 8 && profile_slots(layout, q.rows, G, K) < 8) {
+    if (layout == PROF_PAIR) times = mode == SG ? 1.1 : 1.0;
+    else times = mode == SG ? 1.55 : 1.2;
+  }
   const double row = (warp_row_clocks(ctx, mode, K, G, lean) + more + narrow) * times;
   ShapeCost c;
   if (!set) {
