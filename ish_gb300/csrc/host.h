@@ -302,7 +302,7 @@ cudaError_t grow(ish_ctx *ctx, DevBuf &b, size_t bytes);
 inline uint32_t ceil_div(uint64_t a, uint64_t b) { return (uint32_t)((a + b - 1) / b); }
 
 int frame_rows(int ext);
-int wave_lean(const ish_ctx *ctx, int K, int mode);
+int wave_lean(const ish_ctx *ctx, int K, int mode, int layout);
 double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps);
 // Build of the wavefront kernel for a shape and a set (scored by `share` queries
 // at once).

@@ -160,18 +160,21 @@ int matrix_alphabet_ok(uint32_t alphabet) { return alphabet >= 1 && alphabet <= 
 // gap_open > gap_extend and no lane value of the reference can saturate or
 // wrap.  Bounds are conservative.
 
-// Whether (K, mode) runs the lean kernel variant, as measured on GB300 (300,000
-// proteins, G = 8, Q = 8K - 2; see the kernels' launch bounds in kernels.cuh).
-// Semi-global rows need so few registers that the builds with more warps are
-// ahead or level everywhere: 256 x 2 against 128 x 3 within 1 % at K = 25..32
-// (nucleotide pairs up to 3 % ahead), 128 x 3 against 128 x 2 by 2-8 % at K =
-// 34..48.  Local alignment keeps a row maximum and more state: 128 x 3 is ahead
-// of 256 x 2 by 1-5 % at K = 27..32, and from K = 42 on 128 x 3 spills and 128 x
-// 2 is ahead by 13-47 %.
-int wave_lean(const ish_ctx *ctx, int K, int mode) {
+// Whether a shape usually runs the lean build (see the kernels' launch bounds in
+// kernels.cuh), from 200,000 proteins (G = 8 and 16; 16- and 32-bit profiles) and
+// 200,000 reads of 150 (G = 4 and 8; pair profile).  Semi-global rows need so few
+// registers that the builds with more warps are ahead or level: 0-6 % at K = 25..32
+// (K = 27 -3 %), 4-17 % at K = 34..48.  Local alignment keeps a row maximum and
+// more state, and its builds with more warps spill from K = 25 on but for 34 (24 to
+// 50 bytes read back at K = 25, 36 and 38, 60 to 240 elsewhere).  On proteins the
+// lean build is ahead by 0-7 % at K = 27..32 and, where it has 8 warps against 12,
+// 10 % behind at K = 34..38, level at 42 and 3-12 % ahead from 44 (32 threads: 1.6
+// times at 46).  Pair profiles, with half the loads in flight, keep the 12 warps 3
+// to 14 % ahead at all K from 34.  (lean_for weighs the set in.)
+int wave_lean(const ish_ctx *ctx, int K, int mode, int layout) {
   if (!wave_has_lean(K)) return 0;
   if (ctx->force_lean >= 0) return ctx->force_lean;
-  return mode == SW && ((K >= 27 && K <= 32) || K >= 42);
+  return mode == SW && ((K >= 27 && K <= 32) || (K >= 42 && layout != PROF_PAIR));
 }
 
 // Semi-global rows are held in frames that rise by ext per row and drop back
@@ -223,17 +226,15 @@ int neg_limit_of(int open, int mmin) {
 // 1,032; alone 451 / 752 at K = 32, 619 / 1,074 at 48), with what the builds with
 // fewer warps add, and wide groups (32 threads 9 % at K = 16..32 on proteins: most
 // steps of a warp start a pair in one of its threads).
-// `lean` is the build; where the other one is the usual choice (wave_lean), it
-// costs what 120,000 proteins at G = 16 and 32 showed (semi-global 2-7 % up to K =
-// 32, 7-12 % above; local 10 % at K = 34..38, level at 40; the default build of
-// K = 42..48 5 % to 1.6x).
-static double warp_row_clocks(const ish_ctx *ctx, int mode, int K, int G, int lean) {
+// `lean` is the build; where the other one is the usual choice, it costs what that
+// measured (see wave_lean).
+static double warp_row_clocks(const ish_ctx *ctx, int mode, int K, int G, int layout, int lean) {
   double c = 1.0 + 0.1 * (G / 32.0) * (G / 32.0);
   if (mode == SG) c *= (50 + 8.6 * K) * (K > 48 ? 1.1 : 1.0);
   else c *= (50 + 13.3 * K) * (K > 48 ? 1.11 + 0.02 * std::max(0, K - 56) : K > 40 ? 1.08 : 1.0);
-  if (lean == wave_lean(ctx, K, mode)) return c;
+  if (lean == wave_lean(ctx, K, mode, layout)) return c;
   if (!lean) return c * (K <= 32 ? 1.04 : G < 32 ? 1.08 : 1.3);
-  return c * (mode == SG ? (K <= 32 ? 1.05 : 1.1) : K <= 26 ? 1.02 : K < 40 ? 1.1 : 1.0);
+  return c * (mode == SG ? (K <= 32 ? 1.05 : 1.1) : K <= 26 ? 1.02 : K < 40 ? 1.1 : layout == PROF_PAIR ? 1.07 : 1.0);
 }
 static double lone_row_clocks(int mode, int K) { return mode == SG ? 150 + 9.5 * K : 200 + 17.5 * K; }
 
@@ -248,8 +249,8 @@ static double build_row_clocks(const ish_ctx *ctx, int K, int lean, double warps
   return lone + (w - 1) / (cap - 1) * std::max(0.0, cap * full - lone);
 }
 double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps) {
-  const int lean = wave_lean(ctx, K, mode);
-  return build_row_clocks(ctx, K, lean, warps, warp_row_clocks(ctx, mode, K, G, lean), lone_row_clocks(mode, K));
+  const int lean = wave_lean(ctx, K, mode, PROF_S32);
+  return build_row_clocks(ctx, K, lean, warps, warp_row_clocks(ctx, mode, K, G, PROF_S32, lean), lone_row_clocks(mode, K));
 }
 
 // Modelled time of one query against `set` (null: many records) with G threads x
@@ -287,7 +288,7 @@ static ShapeCost shape_cost(const ish_ctx *ctx, const Query &q, int G, int K, in
     if (layout == PROF_PAIR) times = mode == SG ? 1.1 : 1.0;
     else times = mode == SG ? 1.55 : 1.2;
   }
-  const double row = (warp_row_clocks(ctx, mode, K, G, lean) + more + narrow) * times;
+  const double row = (warp_row_clocks(ctx, mode, K, G, layout, lean) + more + narrow) * times;
   ShapeCost c;
   if (!set) {
     c.clocks = G * row;
@@ -311,7 +312,7 @@ static ShapeCost shape_cost(const ish_ctx *ctx, const Query &q, int G, int K, in
 // SM, 1,222 with 384).
 static double shape_clocks(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share,
                            int *build = nullptr) {
-  const int usual = wave_lean(ctx, K, q.algo == ISH_ALGO_LOCAL ? SW : SG);
+  const int usual = wave_lean(ctx, K, q.algo == ISH_ALGO_LOCAL ? SW : SG, layout);
   ShapeCost c = shape_cost(ctx, q, G, K, layout, usual, set, share);
   int lean = usual;
   if (set && wave_has_lean(K) && ctx->force_lean < 0) {
@@ -442,14 +443,14 @@ static int wave_fit_threads(size_t prof_area, int K, int mode, int lean) {
 // 120,000 proteins, 32-bit / 16-bit: 56 (241) 16.4 / 17.0, 60 (245) 17.6 / 17.6,
 // 62 (271) 28.9 / 18.1.
 int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode, int ends) {
-  const int lean = wave_lean(ctx, K, mode), all = wave_sm_threads(K, lean);
-  const size_t copies = mode == SG && (ends & ISH_FREE_QUERY_END) ? (size_t)all * K * 4 : 0;
+  auto threads = [&](int layout) { return wave_sm_threads(K, wave_lean(ctx, K, mode, layout)); };
   auto fit = [&](int layout, size_t most) {
     const size_t prof = ((layout_bytes(layout, rows, G, K) + 15) & ~(size_t)15) + 256;
-    return copies && prof + copies > most * 1024 ? 0 : wave_fit_threads(prof, K, mode, lean);
+    if (mode == SG && (ends & ISH_FREE_QUERY_END) && prof + (size_t)threads(layout) * K * 4 > most * 1024) return 0;
+    return wave_fit_threads(prof, K, mode, wave_lean(ctx, K, mode, layout));
   };
-  if (fit(PROF_PAIR, 224) == all) return PROF_PAIR;
-  if (4 * fit(PROF_S32, 246) >= (mode == SG ? 3 : 4) * all) return PROF_S32;
+  if (fit(PROF_PAIR, 224) == threads(PROF_PAIR)) return PROF_PAIR;
+  if (4 * fit(PROF_S32, 246) >= (mode == SG ? 3 : 4) * threads(PROF_S32)) return PROF_S32;
   return PROF_S16;
 }
 

@@ -93,28 +93,28 @@ __global__ void k_gather_hits(const uint32_t *idx, const uint32_t *count, const 
 #define WAVE_RPS_SW 4
 #endif
 
-// Wavefront kernels are instantiated for K = 2, 4, ..., WAVE_KMAX columns per
-// thread, both modes and both profile layouts.
+// Wavefront kernels are instantiated for K = 1..32 and even K up to WAVE_KMAX
+// columns per thread, both modes and the three profile layouts.
 constexpr int WAVE_KMAX = 64;
 // Threads an SM holds (the register budget): 512 up to K = 32 columns per
 // thread (128 registers), 384 up to K = 48 (168), 256 above.  Register-lean
 // builds trade warps for registers per thread: 384 threads for 25 <= K <= 32 and
 // 256 for 34 <= K <= 48.  Which build runs is chosen per (K, mode) from
-// measurements (wave_lean).  The launch bound is one block of all of them, so the
-// host may launch them as one block that shares one profile, or as smaller ones
-// (wave_launch, batch_launch).
+// measurements (wave_lean, lean_for).  The launch bound is one block of all of
+// them, so the host may launch them as one block that shares one profile
+// (launch_wave_range), or as smaller ones (batch_launch).
 constexpr int WAVE_LEAN_KMIN = 25, WAVE_LEAN_KMAX = 48;
 __host__ __device__ constexpr bool wave_has_lean(int K) { return K >= WAVE_LEAN_KMIN && K <= WAVE_LEAN_KMAX && K != 33; }
 __host__ __device__ constexpr int wave_sm_threads(int K, int lean) {
   return lean && wave_has_lean(K) ? (K <= 32 ? 384 : 256) : (K <= 32 ? 512 : K <= 48 ? 384 : 256);
 }
-// wave_kernel reads its parameters from a shared-memory copy for these
-// (K, mode, lean build) (see wave.cuh).  Measured on the protein search
-// (400k records, G = 8, Q = 8K - 2): semi-global at K = 9..32 +1 to +12 %;
-// local at K = 12..32 mostly +1.4 to +9.7 %; the 128 x 3 builds of K = 34..48
-// +5 to +10 % (semi-global), -1 to +10 % (local); K = 58..64 +1.5 to +6.6 %
-// and local K = 50 +3 % (K = 52..56: -2.6 to +0.2 %).  The register-lean
-// builds of K >= 34 keep the parameter bank.
+// wave_kernel reads its parameters from a shared-memory copy for these (K, mode,
+// lean build) (see wave.cuh).  Against the parameter bank, on 200,000 proteins (G =
+// 8 and 16) and 200,000 reads of 150 (G = 4 and 8): semi-global 0 to +4 % at K =
+// 10..48 with few exceptions (K = 26 with the 32-bit profile +32 %, K = 27 -4 %, K =
+// 36 with the pair profile -5 %), -1 to +4 % from K = 58 on, and level or behind on
+// reads at the K left out; local -5 to +2 % (K = 38 of the protein search +2 %, the
+// mean -1 %), where the copy stays as it was set for rows that needed it.
 #ifndef WAVE_PARAMS_SMEM
 #define WAVE_PARAMS_SMEM(K, MODE, LEAN)                                              \
   (((MODE) == 0 && (K) >= 9 && (K) <= 32) || ((MODE) == 1 && (K) >= 12 && (K) <= 32) || \

@@ -121,9 +121,11 @@ uint64_t window_overlap(const Query &q) {
 
 // Windows pay when the longest record exceeds ISH_WINDOW_QUARTERS / 4 of the
 // rows a group scores on average: its pair alone would then outlast the pass.
-// Measured on 10,000 records of 10 kb-1 Mb (1,000-nt query, 32-thread groups,
-// 589k rows per group on average, 1M rows in the longest record): no windows
-// at 2x (5,112-5,336 GCUPS), windows at 1.25x and 1x (6,794 / 6,803).
+// Measured with 4, 5 and 8 quarters on 1,000 to 200,000 proteins (20 to 1,000
+// residues) where they differ: 60,000, local, 340 residues 1,679 / 1,681 / 1,962 us
+// and 460 residues 2,106 / 2,107 / 2,182; 200,000, semi-global, 180 residues 1,777 /
+// 1,780 / 1,877, but 220 residues 2,206 / 2,176 / 2,176 and local 180 residues 2,686
+// / 2,640 / 2,643.
 #ifndef ISH_WINDOW_QUARTERS
 #define ISH_WINDOW_QUARTERS 5
 #endif
@@ -139,7 +141,7 @@ uint64_t window_overlap(const Query &q) {
 // stride of at least 8 x O, 10 records of 10 kb - 1 Mb made 32 windows for 1,000
 // nt (11.4 ms; 2.2 ms with this rule), 200 records 1,102 (11.7 ms; 8.4 ms).
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode) {
-  const int lean = wave_lean(ctx, K, mode);
+  const int lean = wave_lean(ctx, K, mode, PROF_S32);
   // groups in flight and the rows each would score on average (two records
   // per pair share their rows)
   const uint64_t groups = (uint64_t)ctx->num_sms * wave_sm_threads(K, lean) / G;
