@@ -307,6 +307,8 @@ double row_clocks(const ish_ctx *ctx, int mode, int K, int G, double warps);
 // Build of the wavefront kernel for a shape and a set (scored by `share` queries
 // at once).
 int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share);
+// Modelled clocks of a row of 32 record pairs with a shape, for many records.
+double shape_rate(const ish_ctx *ctx, const Query &q, int G, int K, int layout);
 uint64_t window_overlap(const Query &q);
 int launch_windows(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t nonempty, OutDev out, cudaStream_t s, bool *done);
 uint64_t window_stride(const ish_ctx *ctx, const RecordSet &rs, uint64_t O, int G, int K, int mode);

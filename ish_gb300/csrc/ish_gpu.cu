@@ -328,6 +328,9 @@ static double shape_clocks(const ish_ctx *ctx, const Query &q, int G, int K, int
   if (build) *build = lean;
   return c.clocks;
 }
+double shape_rate(const ish_ctx *ctx, const Query &q, int G, int K, int layout) {
+  return shape_clocks(ctx, q, G, K, layout, nullptr, 1);
+}
 int lean_for(const ish_ctx *ctx, const Query &q, int G, int K, int layout, const RecordSet *set, double share) {
   int lean = 0;
   shape_clocks(ctx, q, G, K, layout, set, share, &lean);
@@ -459,23 +462,29 @@ int choose_layout(const ish_ctx *ctx, int rows, int G, int K, int mode, int ends
 // 31 columns per thread at the pace of the longest record's one group.  The
 // padded query counts towards the fast regime's bounds, so a shape for the set is
 // taken only where it keeps the query and the set's longest record inside them.
+// The autotuner's choice stands for the shape with the highest rate; it was timed
+// on records of like lengths, so a set's few or uneven ones still count.
 void pick_shape(ish_ctx *ctx, const Query &q, int *G, int *K, int *layout, const RecordSet *set, double share) {
   const int mode = q.algo == ISH_ALGO_LOCAL ? SW : SG;
   auto it = ctx->tuned.find(tune_key(mode, q.rows, q.Q));
-  if (!ctx->force_G && !ctx->force_K && ctx->force_layout < 0 && it != ctx->tuned.end()) {
+  const bool tuned = !ctx->force_G && !ctx->force_K && ctx->force_layout < 0 && it != ctx->tuned.end();
+  if (tuned) {
     *G = it->second.G;
     *K = it->second.K;
     *layout = it->second.layout >= 0 ? it->second.layout : shape_layout(ctx, q, *G, *K);
-    return;
+  } else {
+    choose_shape(ctx, q, nullptr, 1, G, K);
+    *layout = shape_layout(ctx, q, *G, *K);
   }
-  choose_shape(ctx, q, nullptr, 1, G, K);
-  *layout = shape_layout(ctx, q, *G, *K);
   if (!set || !*G) return;
   int g = 0, k = 0;
   choose_shape(ctx, q, set, share, &g, &k);
   const int l = shape_layout(ctx, q, g, k);
-  // (closer than that the model does not tell shapes apart)
-  if (!g || shape_clocks(ctx, q, g, k, l, set, share) > 0.97 * shape_clocks(ctx, q, *G, *K, *layout, set, share)) return;
+  // (closer than that the model does not tell shapes apart, or knows less than the
+  // autotuner)
+  if (!g || shape_clocks(ctx, q, g, k, l, set, share) >
+                (tuned ? 0.9 : 0.97) * shape_clocks(ctx, q, *G, *K, *layout, set, share))
+    return;
   const Regime r = regime(q, g * k);
   if (!r.fast || set->max_len > r.max_safe_len || !wave_fits(q, g, k, l)) return;
   *G = g;

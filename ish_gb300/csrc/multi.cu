@@ -527,12 +527,12 @@ int ish_gpu_autotune(ish_ctx *ctx, int32_t set_id, const int32_t *query_ids, uin
         int k = (q.Q + 1 + g - 1) / g;
         if (k > 32) k = (k + 1) & ~1;
         if (!wave_k_available(k)) continue;
-        const double m = (double)g * (k + 8) * (k > 48 ? 1.25 : 1.0);
-        best_model = std::min(best_model, m);
         // the layout rule's pick, and the 16/32-bit alternative to it (the
         // 32-bit profile saves an ALU instruction per column but can cost
         // occupancy)
         const int pick = choose_layout(ctx, q.rows, g, k, mode, q.ends);
+        const double m = shape_rate(ctx, q, g, k, pick);
+        best_model = std::min(best_model, m);
         cands.push_back({g, k, pick, m});
         const int other = pick == PROF_S32 ? PROF_S16 : (pick == PROF_S16 ? PROF_S32 : -1);
         if (other >= 0 && wave_fits(q, g, k, other)) cands.push_back({g, k, other, m});
