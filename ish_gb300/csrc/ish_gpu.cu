@@ -1099,6 +1099,7 @@ int launch_wave_range(ish_ctx *ctx, Query &q, RecordSet &rs, uint32_t first, uin
   const int threads = (int)std::min<uint32_t>(most, 32 * ceil_div(warps, ctx->num_sms));
   const uint32_t grid = std::min<uint32_t>(ctx->num_sms, ceil_div(warps, threads / 32));
   const size_t smem = wave_smem(prof_area, threads, K, mode);
+  CU(ctx->counter.ensure(64));
   WaveParams p;
   wave_params(q, *L, rs, out, ctx->error.as<int>(), &p);
   p.first = first;

@@ -253,6 +253,7 @@ cudaError_t cudaMemcpy(void *to, const void *from, size_t bytes, cudaMemcpyKind)
 }
 cudaError_t cudaMemset(void *p, int v, size_t bytes) { return memset(p, v, bytes), cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t bytes, cudaStream_t) {
+  if (!p) return cudaErrorInvalidValue;
   touch("memset", p, bytes);
   return cudaMemset(p, v, bytes);
 }
