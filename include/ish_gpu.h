@@ -84,9 +84,11 @@ extern "C" {
 #define ISH_OPT_WAVE_GROUP 5  /* force threads per record pair (0 = autotuned) */
 #define ISH_OPT_WAVE_K 6      /* force query columns per thread (0 = autotuned) */
 #define ISH_OPT_PROFILE_LAYOUT 7 /* force the profile layout: -1 auto, 0 16-bit, 1 pair, 2 32-bit */
-#define ISH_OPT_WAVE_BLOCKS 8 /* cap wavefront blocks per SM (0 = as many as fit) */
+#define ISH_OPT_WAVE_BLOCKS 8 /* cap an SM's threads: single launches at n x 256 (K <= 32 columns per thread) or
+                               * n x 128, batched ones at n blocks (0 = as many as fit) */
 #define ISH_OPT_WINDOWS 10    /* 1 (default): window long records when they would bound the pass; 0: never */
-#define ISH_OPT_WAVE_LEAN 9   /* 34 <= K <= 48: -1 measured default, 0 128x3 blocks, 1 128x2 (more registers) */
+#define ISH_OPT_WAVE_LEAN 9   /* 25 <= K <= 48: -1 measured default, 0 the build with more threads per SM (512 up to
+                               * K = 32, 384 above), 1 the one with more registers (384, 256) */
 #define ISH_OPT_SERVE_STEP_CELLS 13 /* serving: cells a step aims at per query (default 1.25e11); a query takes
                                     * cells/that steps, 1..chunks; 0: every query takes `chunks` steps */
 /* Fault injection for testing a caller's error paths (no counterpart in the
@@ -98,8 +100,7 @@ extern "C" {
  * to run out.  ISH_OPT_FAULT_ALLOC: n >= 0 makes the (n+1)-th device allocation
  * the library attempts from now on fail as if device memory were exhausted
  * (ISH_ENOMEM, where nothing kept between calls can be given back instead); it
- * applies to every context of the process and disarms after
- * firing; -1 disarms it.  Neither changes results when left at its default. */
+ * applies to every context of the process and disarms after firing; -1 disarms it.  Neither changes results when left at its default. */
 #define ISH_OPT_STEP_BUDGET 11
 #define ISH_OPT_FAULT_ALLOC 12
 
