@@ -757,15 +757,15 @@ int exact_prepare(ish_ctx *ctx, Query &q, uint32_t count, ExactRes &res) {
       if (ps.mode == SG || ps.reg_seg) {
         auto v = striped_profile<int16_t>(q, ps.W, ps.mode == SW, bias, ps.reg_seg);
         CU(prof.ensure(v.size() * 2));
-        CU(cudaMemcpy(prof.p, v.data(), v.size() * 2, cudaMemcpyHostToDevice));
+        CU(upload(prof.p, v.data(), v.size() * 2));
       } else if (!ps.word) {
         auto v = striped_profile<uint8_t>(q, ps.W, true, bias, 0);
         CU(prof.ensure(v.size()));
-        CU(cudaMemcpy(prof.p, v.data(), v.size(), cudaMemcpyHostToDevice));
+        CU(upload(prof.p, v.data(), v.size()));
       } else {
         auto v = striped_profile<uint16_t>(q, ps.W, true, bias, 0);
         CU(prof.ensure(v.size() * 2));
-        CU(cudaMemcpy(prof.p, v.data(), v.size() * 2, cudaMemcpyHostToDevice));
+        CU(upload(prof.p, v.data(), v.size() * 2));
       }
     }
     CU(res.scratch.ensure(ps.blocks * (ps.threads / ps.W) * ps.tile_bytes + 16));

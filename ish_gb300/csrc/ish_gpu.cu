@@ -559,7 +559,7 @@ int build_wave_layout(ish_ctx *ctx, Query &q, int G, int K, int layout, WaveLayo
     L.prof_bytes += 256;
   }
   CU(L.prof.ensure(L.prof_bytes));
-  CU(cudaMemcpy(L.prof.p, host.data(), L.prof_bytes, cudaMemcpyHostToDevice));
+  CU(upload(L.prof.p, host.data(), L.prof_bytes));
   auto res = q.layouts.emplace(key, std::move(L));
   *out = &res.first->second;
   return ISH_OK;
@@ -576,8 +576,8 @@ int build_plain(ish_ctx *ctx, Query &q) {
     for (int col = 0; col < q.Q; ++col) hin[col] = (int16_t)(-q.open - q.ext * col);
   CU(q.plain_prof.ensure(prof.size() * 2));
   CU(q.plain_hinit.ensure(hin.size() * 2));
-  CU(cudaMemcpy(q.plain_prof.p, prof.data(), prof.size() * 2, cudaMemcpyHostToDevice));
-  CU(cudaMemcpy(q.plain_hinit.p, hin.data(), hin.size() * 2, cudaMemcpyHostToDevice));
+  CU(upload(q.plain_prof.p, prof.data(), prof.size() * 2));
+  CU(upload(q.plain_hinit.p, hin.data(), hin.size() * 2));
   q.plain_ready = true;
   return ISH_OK;
 }
@@ -616,7 +616,7 @@ int device_encoding(ish_ctx *ctx, int kind, const uint8_t **out) {
     uint8_t t[4 * 256];
     for (int k = 0; k < 4; ++k) encoding_table(k, t + 256 * k);
     CU(ctx->enc_tables.ensure(sizeof t));
-    CU(cudaMemcpy(ctx->enc_tables.p, t, sizeof t, cudaMemcpyHostToDevice));
+    CU(upload(ctx->enc_tables.p, t, sizeof t));
   }
   *out = ctx->enc_tables.as<uint8_t>() + 256 * kind;
   return ISH_OK;

@@ -251,8 +251,8 @@ int build_plan(ish_ctx *ctx, const int32_t *qids, uint32_t nq, int32_t set_id, R
     P.n_counters += c.ntiles;
     CU(c.params.ensure(params.size() * sizeof(WaveParams)));
     CU(c.tiles.ensure(std::max<size_t>(1, tiles.size()) * sizeof(BatchTile)));
-    CU(cudaMemcpy(c.params.p, params.data(), params.size() * sizeof(WaveParams), cudaMemcpyHostToDevice));
-    if (!tiles.empty()) CU(cudaMemcpy(c.tiles.p, tiles.data(), tiles.size() * sizeof(BatchTile), cudaMemcpyHostToDevice));
+    CU(upload(c.params.p, params.data(), params.size() * sizeof(WaveParams)));
+    if (!tiles.empty()) CU(upload(c.tiles.p, tiles.data(), tiles.size() * sizeof(BatchTile)));
   }
   CU(P.counters.ensure((size_t)std::max<uint32_t>(1, P.n_counters) * 4 + 16));
   if (want & W_COMPACT) {

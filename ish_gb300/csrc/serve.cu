@@ -636,7 +636,7 @@ int ish_gpu_serve_start(ish_ctx *ctx, int32_t set_id, uint32_t max_active, uint6
   if ((e = S->step_tiles.ensure((size_t)max_active * sizeof(BatchTile))) != cudaSuccess) return bail(e);
   if ((e = S->step_counters.ensure((size_t)max_active * 4)) != cudaSuccess) return bail(e);
   if ((e = S->error.ensure(64)) != cudaSuccess) return bail(e);
-  if ((e = cudaMemset(S->error.p, 0, 64)) != cudaSuccess) return bail(e);
+  if ((e = cudaMemsetAsync(S->error.p, 0, 64, S->s)) != cudaSuccess) return bail(e);
   if ((e = cudaMallocHost((void **)&S->h_params, (size_t)max_active * sizeof(WaveParams))) != cudaSuccess)
     return bail(e);
   if ((e = cudaMallocHost((void **)&S->h_tiles, (size_t)max_active * sizeof(BatchTile))) != cudaSuccess)

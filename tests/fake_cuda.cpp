@@ -2,6 +2,9 @@
 // memory is host memory, streams run every call at once and the kernels listed
 // in launch() are written out here (the others do nothing).  It checks what a
 // device would not report:
+//   - what a blocking upload from pageable memory or a memset leaves on its way, in
+//     the order of the legacy stream alone, has been waited for when another stream
+//     launches a kernel;
 //   - the source of an asynchronous upload from pageable memory stays readable
 //     and unchanged until its stream has been waited for;
 //   - what the kernels written out here touch lies inside one allocation.
@@ -34,6 +37,7 @@ struct Upload {
 std::vector<Upload> uploads;  // not waited for yet
 std::string report, wave;             // wave: the last wavefront kernel launched
 std::vector<std::string> contents;  // of the asynchronous uploads from pageable memory
+bool on_its_way = false;  // a legacy-stream upload or memset that nothing has waited for
 bool refuse_func_attributes = false, refuse_other_threads = false;
 std::thread::id caller;  // where refuse_other_threads was set
 int copies_to_go = -1;  // asynchronous copies that still succeed before one is refused (-1: all)
@@ -213,6 +217,7 @@ cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *f) {
 }
 cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3, dim3, void **a, size_t, cudaStream_t) {
   std::lock_guard<std::recursive_mutex> lk(mu);
+  if (on_its_way) report += kernels[(const void *)k] + " launched while an upload was on its way\n";
   launch(kernels[(const void *)k], a);
   return cudaSuccess;
 }
@@ -247,15 +252,20 @@ cudaError_t cudaMemcpyAsync(void *to, const void *from, size_t bytes, cudaMemcpy
   memmove(to, from, bytes);
   return cudaSuccess;
 }
-cudaError_t cudaMemcpy(void *to, const void *from, size_t bytes, cudaMemcpyKind) {
+cudaError_t cudaMemcpy(void *to, const void *from, size_t bytes, cudaMemcpyKind kind) {
+  std::lock_guard<std::recursive_mutex> lk(mu);
   memmove(to, from, bytes);
+  on_its_way = kind == cudaMemcpyHostToDevice && !room(pinned, from);  // (earlier ones end before it begins)
   return cudaSuccess;
 }
-cudaError_t cudaMemset(void *p, int v, size_t bytes) { return memset(p, v, bytes), cudaSuccess; }
+cudaError_t cudaMemset(void *p, int v, size_t bytes) {
+  on_its_way = true;
+  return memset(p, v, bytes), cudaSuccess;
+}
 cudaError_t cudaMemsetAsync(void *p, int v, size_t bytes, cudaStream_t) {
   if (!p) return cudaErrorInvalidValue;
   touch("memset", p, bytes);
-  return cudaMemset(p, v, bytes);
+  return memset(p, v, bytes), cudaSuccess;
 }
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return handle(s); }
@@ -263,6 +273,7 @@ cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) {
   std::lock_guard<std::recursive_mutex> lk(mu);
+  if (!s || s == cudaStreamLegacy) on_its_way = false;
   waited(s);
   return cudaSuccess;
 }
@@ -281,10 +292,11 @@ cudaError_t cudaEventSynchronize(cudaEvent_t e) {
 }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { return *ms = 0, cudaSuccess; }
 
-cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaErrorInvalidValue; }
-cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *) { return cudaErrorInvalidValue; }
-cudaError_t cudaGraphInstantiate(cudaGraphExec_t *, cudaGraph_t, unsigned long long) { return cudaErrorInvalidValue; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaErrorInvalidValue; }
+// (a captured stream runs its calls at once, a graph launch runs nothing again)
+cudaError_t cudaStreamBeginCapture(cudaStream_t, cudaStreamCaptureMode) { return cudaSuccess; }
+cudaError_t cudaStreamEndCapture(cudaStream_t, cudaGraph_t *g) { return handle(g); }
+cudaError_t cudaGraphInstantiate(cudaGraphExec_t *g, cudaGraph_t, unsigned long long) { return handle(g); }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaGraphDestroy(cudaGraph_t) { return cudaSuccess; }
 cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 
