@@ -296,10 +296,10 @@ struct LoadTimer {
   } while (0)
 
 // cudaMemcpy from pageable memory, on the device when it returns.  By itself it may
-// return while the last bytes are on their way from the driver's staging buffer, in
-// the order of the legacy stream alone, for which the library's own streams do not
-// wait: a query's first launch has been seen reading the profile that its buffer
-// held before.
+// return while the last bytes are on their way from CUDA's staging buffer, in the
+// order of the legacy stream alone, for which the library's own streams do not wait:
+// a query's first launch has been seen reading the profile that its buffer held
+// before.
 inline cudaError_t upload(void *dst, const void *src, size_t bytes) {
   const cudaError_t e = cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice);
   return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e;

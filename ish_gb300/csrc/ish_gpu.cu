@@ -166,7 +166,7 @@ int matrix_alphabet_ok(uint32_t alphabet) { return alphabet >= 1 && alphabet <= 
 // registers that the builds with more warps are ahead or level: 0-6 % at K = 25..32
 // (K = 27 -3 %), 4-17 % at K = 34..48.  Local alignment keeps a row maximum and
 // more state, and its builds with more warps spill from K = 25 on but for 34 (24 to
-// 50 bytes read back at K = 25, 36 and 38, 60 to 240 elsewhere).  On proteins the
+// 52 bytes read back at K = 25..27, 36 and 38, 60 to 240 elsewhere).  On proteins the
 // lean build is ahead by 0-7 % at K = 27..32 and, where it has 8 warps against 12,
 // 10 % behind at K = 34..38, level at 42 and 3-12 % ahead from 44 (32 threads: 1.6
 // times at 46).  Pair profiles, with half the loads in flight, keep the 12 warps 3
@@ -397,8 +397,8 @@ static size_t slots_bytes(int layout, int alphabet, int slots, int K) {
 // threads or more never conflict; narrower groups of a quarter-warp read rows
 // of different codes that start at the same banks.  Their slices are repeated
 // up to eight per row, one set for each group of the quarter-warp, as long as
-// the profile stays at 44 KB (three blocks per SM of local alignment's widest
-// rows still fit beside it).  Measured on 300,000 proteins, semi-global: four
+// the profile stays at 44 KB (three blocks of a batched launch still fit an SM with
+// local alignment's widest rows beside it).  Measured on 300,000 proteins, semi-global: four
 // threads x 16 columns 4,155 -> 6,565 GCUPS, x 38 columns 4,661 -> 7,924.
 int profile_slots(int layout, int alphabet, int G, int K) {
   return G < 8 && slots_bytes(layout, alphabet, 8, K) <= 44 * 1024 ? 8 : G;
