@@ -7,6 +7,7 @@
 namespace ish {
 
 constexpr uint32_t NBUCKETS = 65536;     // length buckets of the record sort
+constexpr uint32_t LAST_BUCKET_LEN = 32768 + 32 * (NBUCKETS - 1 - 32768);  // lengths from here on share one
 constexpr uint32_t SCAN_TILE = 4096;     // values per block of k_scan64_block (1024 threads)
 constexpr uint32_t HIT_TILE = 8192;      // records per block of the hit compaction
 constexpr uint32_t SMEM_BUCKETS = 4096;  // length buckets counted in shared memory by k_lengths / k_scatter

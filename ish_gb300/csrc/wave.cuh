@@ -834,9 +834,11 @@ __global__ void __launch_bounds__(wave_sm_threads(K, LEAN), 1)
         sp.pair_stride = stride;
         sp.pair_phase = phase;
         // every group's steps are bounded by all pairs of the range at its
-        // longest length (records are sorted, the first is longest)
-        const uint64_t npairs = (tl.count + 1) / 2;
-        sp.max_steps = b.step_cap ? b.step_cap : npairs * ((uint64_t)qp->rec.len[tl.first] + 2 * 32 + 8) + 1024;
+        // longest length (records are sorted, the first is longest to within a
+        // bucket; the last bucket holds any length from its own on)
+        const uint64_t npairs = (tl.count + 1) / 2, first = qp->rec.len[tl.first];
+        const uint64_t most = first < LAST_BUCKET_LEN ? first : 0xffffffffu;
+        sp.max_steps = b.step_cap ? b.step_cap : npairs * (most + 2 * 32 + 8) + 1024;
       }
     }
     __syncthreads();
